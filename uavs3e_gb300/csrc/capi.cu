@@ -44,6 +44,43 @@ int ensure_init()
     return uavs3e_cuda_init(0);
 }
 
+// One memory pool per device for the calls' workspaces.  The device's default pool gives its memory
+// back at every synchronisation, so a call after one maps it anew (0.28 ms for 155 MB); this one
+// keeps up to WORK_POOL_KEEP bytes.  Allocations and frees follow the stream's order, so calls on
+// several streams or threads never share a block that is in use.
+int work_alloc(void **p, size_t bytes, cudaStream_t st)
+{
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    UC_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return set_status(UC_ERR_UNSUPPORTED, "workspace: device index");
+    cudaMemPool_t pool;
+    {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!pools[dev]) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof(props));
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            UC_CHECK(cudaMemPoolCreate(&pool, &props));
+            uint64_t keep = WORK_POOL_KEEP;
+            UC_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+            pools[dev] = pool;
+        }
+        pool = pools[dev];
+    }
+    UC_CHECK(cudaMallocFromPoolAsync(p, bytes, pool, st));
+    return UC_OK;
+}
+
+int work_free(void *p, cudaStream_t st)
+{
+    UC_CHECK(cudaFreeAsync(p, st));
+    return UC_OK;
+}
+
 // edge replication of a padded plane (com_img_padding with ext_size 0, one plane)
 __global__ void k_pad_plane(pel *p, int W, int H, int pad, int stride)
 {

@@ -42,6 +42,9 @@ __device__ __constant__ static const s8 kLumaTaps[4][8] = {
     { -1, 3, -7, 19, 57, -10, 4, -1 },
 };
 
+// shared-window address of a pointer to shared memory
+__device__ __forceinline__ u32 smem_addr(const void *p) { return (u32)__cvta_generic_to_shared(p); }
+
 __device__ __forceinline__ int clip255(int v) { return min(255, max(0, v)); }
 
 // sum over the four byte lanes of |a - b|, accumulated into c (PTX video instruction)

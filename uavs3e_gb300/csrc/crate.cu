@@ -6,15 +6,20 @@
 // (range and the channel's run, run_rdoq, level, last1, last2 models).  Results: the bits
 // counted, the range and the models after the block, bit-exact with the reference.
 //
-// The scan of each block runs over the warp's lanes; the coding is one chain per block (each bin
-// updates the model and range the next one reads), one lane per block, the models in registers /
-// local memory.  The model update is the rule the
-// reference tabulates in tbl_plps / tbl_plps_ext (src/entropy.c:41), computed.
+// Two launches with a grouping between them: a warp per block lists its levels in scan order
+// (k_cr_list), the blocks are ordered by the bins they will code (blocksort.cuh), and a lane per
+// block codes its chain (k_cr_code).  The chains bound the call: one lane's bins follow one another.
+// 60,000 blocks of the 23 shapes (5.6 M levels, 31 M bins, up to 5,300 bins a block) take 54 us to list
+// and 0.55 ms to code; one launch in which a warp listed 32 blocks in turn and then coded them side by
+// side, symbol after symbol, took 2.37 ms with 4 of 32 lanes active on average.  The model update is
+// the rule the reference tabulates in tbl_plps / tbl_plps_ext (src/entropy.c:41), computed.
+#include "blocksort.cuh"
 #include "common.cuh"
 #include "tables.h"
 #include "uavs3e_cuda_internal.h"
 #include "../../include/uavs3e_cuda.h"
 
+#include <algorithm>
 #include <mutex>
 #include <string.h>
 
@@ -32,168 +37,304 @@ struct CrParams {
     const s16 *levels;
     unsigned long long n_levels;
     CrOut *out;
+    u32 *fixed;                          // per block: bits that do not depend on the coder state, or CR_BAD
     const u16 *scan[7][7];
 };
 
 // the model after one bin: window state (bits 11-12: windows 3, 3, 4, 5), LPS probability (bits
 // 1-10), MPS (bit 0); an MPS shrinks the probability by p >> w + p >> (w + 2), an LPS grows it by
-// 197 / 95 / 46 (reflected about 1023 with the MPS flipped) and steps the state up
-__device__ __forceinline__ s16 cr_next(int model, bool mps)
+// 197 / 95 / 46 (reflected about 1023 with the MPS flipped) and steps the state up.  Both outcomes
+// are formed and selected: the chain waits on the select, not on a branch.
+__device__ __forceinline__ u32 cr_next(u32 model, bool mps)
 {
-    const int c = (model >> 11) & 3, w = c < 2 ? 3 : c + 2;
-    int p = (model >> 1) & 1023, m = model & 1;
-    if (mps) {
-        p -= (p >> w) + (p >> (w + 2));
-        return (s16)(((c == 0 ? 1 : c) << 11) | (p << 1) | m);
-    }
-    p += w == 3 ? 197 : (w == 4 ? 95 : 46);
-    if (p > 1023) { p = 2047 - p; m ^= 1; }
-    return (s16)((min(c + 1, 3) << 11) | (p << 1) | m);
+    const u32 c = (model >> 11) & 3, w = max(c + 2, 3u), p = (model >> 1) & 1023;
+    const u32 pm = p - (p >> w) - (p >> (w + 2));
+    const u32 m_next = (max(c, 1u) << 11) | (pm << 1) | (model & 1);
+    const u32 pl = p + __byte_perm(0x2E5FC5C5u, 0u, 0x4440 + c);     // 197, 197, 95, 46
+    const bool flip = pl > 1023;
+    const u32 l_next = (min(c + 1, 3u) << 11) | ((flip ? 2047 - pl : pl) << 1) | ((model & 1) ^ (flip ? 1u : 0u));
+    return mps ? m_next : l_next;
 }
 
-// counting-mode coding of one bin (lbac_encode_bin with no bitstream)
-__device__ __forceinline__ void cr_bin(u32 &range, u32 &bits, s16 &mdl, int bin)
+// counting-mode coding of one bin (lbac_encode_bin with no bitstream); the range after an LPS is
+// formed beside the one after an MPS and selected
+__device__ __forceinline__ void cr_code(u32 &range, u32 &bits, u32 lps, bool eq)
 {
-    const u32 lps = (u32)(mdl & 2047) >> 3;
     u32 mps = range - lps;
-    const int s = mps < 256;
+    const u32 s = mps < 256 ? 1u : 0u;
     mps |= 0x100;
-    if (bin == (mdl & 1)) {
-        bits += s;
-        range = mps;
-        mdl = cr_next(mdl, true);
-    } else {
-        const u32 l = (range << s) - mps;
-        const int sh = __clz(l) - 23;
-        range = l << sh;
-        bits += sh + s;
-        mdl = cr_next(mdl, false);
-    }
+    const u32 l = (range << s) - mps;                // at least 1: a model's LPS range is never 0
+    const u32 sh = (u32)__clz((int)l) - 23u;
+    range = eq ? mps : l << sh;
+    bits += s + (eq ? 0u : sh);
 }
 
-// truncated unary symbol: first bin ('1' for 0) on m0, then '0' per unit and the closing '1' on
-// m1, the closing bin omitted at the cap
-__device__ __forceinline__ void cr_unary(u32 &range, u32 &bits, s16 &m0, s16 &m1, int sym, int cap)
+// cr_next of every model and bin, in shared memory: next[2 model + bin].  The rule takes some 17
+// instructions, a look-up 3, and a chain runs 2 to 3 of them per bin.
+struct CrTable { u16 next[2 * 8192]; };
+
+__device__ __forceinline__ u32 cr_step(const CrTable &T, u32 mdl, u32 bin) { return T.next[2 * mdl + bin]; }
+
+// what the range coder needs of a bin: the model's LPS range (8 bits) and whether the bin is the MPS
+__device__ __forceinline__ u16 cr_code_of(u32 mdl, u32 bin)
 {
-    cr_bin(range, bits, m0, sym == 0);
-    for (int k = 1; k <= sym && k < cap; k++) cr_bin(range, bits, m1, k == sym);
+    return (u16)(((mdl >> 3) & 255) | (bin == (mdl & 1) ? 256u : 0u));
 }
 
-__device__ __forceinline__ u32 cr_egk(int v)
+// bits of the exp-Golomb escape of v >= -1 (order 0): sum of 2^k steps down to below 0
+__device__ __forceinline__ u32 cr_egk(int v) { return 2u * (31u - (u32)__clz(v + 2)) + 1u; }
+
+constexpr int CR_LIST_WARPS = 8;     // blocks per CTA of the listing
+constexpr int CR_LIST_UNROLL = 4;    // 32-position windows whose loads are in flight together
+constexpr u32 CR_BAD = 0xFFFFFFFFu;  // a request outside the domain, or fewer levels than num_sig
+
+// A listed level: its run of zeros (12 bits), min(level - 1, 7) (3), whether level - 1 >= 8 (1), the
+// last2 context of its position (4), whether it is the block's last scan position (1).
+__device__ __forceinline__ u32 cr_entry(int run, int sym, int pos, int n)
 {
-    int order = 1;
-    for (int s = v; s >= 0; order++) s -= 1 << order;
-    return (u32)((order << 1) - 1);
+    return (u32)run | (u32)min(sym, 7) << 12 | (sym >= 8 ? 1u << 15 : 0u) | (u32)(31 - __clz(pos + 1)) << 16 |
+           (pos == n - 1 ? 1u << 20 : 0u);
 }
 
-__device__ __forceinline__ bool cr_valid(const CrReq &q, unsigned long long n_levels)
+// Listing, a warp per block: checks the request and writes, in scan order, an entry for each of the
+// block's first num_sig non-zero levels to list[] at the block's own level offset (a ballot and a
+// prefix count per 32 positions); sums the bits the coder state has no part in (signs and escapes)
+// and the bins the block will code, which are its chain length for the grouping.
+__global__ void __launch_bounds__(32 * CR_LIST_WARPS) k_cr_list(const CrParams P, u32 *list_all, BlockOrder O)
 {
-    const int lw = q.log2w, lh = q.log2h, top = q.ch_type ? 5 : 6;
-    const unsigned long long nc = 1ull << (lw + lh);
-    bool ok = lw >= 2 && lw <= top && lh >= 2 && lh <= top && q.num_sig >= 1 && q.num_sig <= nc &&
-              q.range >= 256 && q.range <= 511 && (unsigned long long)q.coef_offset + nc <= n_levels;
-    const s16 *mdl = &q.ctx.run[0];
-    const int nchk = q.ch_type ? 52 : 54;             // chroma codes no last2 context past 9
-#pragma unroll
-    for (int k = 0; k < 54; k++)
-        ok = ok && (k >= nchk || (((mdl[k] >> 1) & 1023) >= 4 && mdl[k] >= 0 && mdl[k] < 8192));
-    return ok;
-}
-
-// Warp per 32 blocks.  First the warp takes its blocks one by one and lists, in scan order, the
-// positions and values of their first num_sig non-zero levels (a ballot and a prefix count per 32
-// positions) in list[] at the block's own level offset; then each lane codes its block's chain
-// from that list.  A run of zeros steps the run_rdoq model once per zero; the steps stop changing
-// the model once its probability is too small to move (p >> w == 0 after an MPS), so the walk ends
-// there.
-__global__ void __launch_bounds__(128) k_coef_rate(const CrParams P, u32 *list_all)
-{
-    __shared__ int s_cnt[4][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (blockIdx.x * 4 + warp) * 32;
-    if (r0 >= P.n) return;
-    for (int r = 0; r < 32 && r0 + r < P.n; r++) {
-        const CrReq q = P.reqs[r0 + r];
-        int cnt = 0;
-        if (cr_valid(q, P.n_levels)) {
-            const int n = 1 << (q.log2w + q.log2h);
-            const s16 *coef = P.levels + q.coef_offset;
-            const u16 *scan = P.scan[q.log2w][q.log2h];
-            u32 *list = list_all + q.coef_offset;
-            for (int base = 0; base < n && cnt < q.num_sig; base += 32) {
-                const int i = base + lane;
-                const int c = i < n ? coef[scan[i]] : 0;
-                const u32 m = __ballot_sync(0xffffffffu, c != 0);
-                const int at = cnt + __popc(m & ((1u << lane) - 1));
-                if (c != 0 && at < q.num_sig) list[at] = ((u32)i << 16) | (u16)(s16)c;
+    const int r = blockIdx.x * CR_LIST_WARPS + warp;
+    if (r >= P.n) return;
+    const u32 word = lane < 30 ? reinterpret_cast<const u32 *>(P.reqs + r)[lane] : 0u;
+    const u32 offset = __shfl_sync(0xffffffffu, word, 0), dims = __shfl_sync(0xffffffffu, word, 1);
+    const u32 sr = __shfl_sync(0xffffffffu, word, 2);
+    const int lw = dims & 255, lh = (dims >> 8) & 255, ch = (dims >> 16) & 255, top = ch ? 5 : 6;
+    const int num_sig = sr & 0xffff, range = sr >> 16;
+    bool ok = lw >= 2 && lw <= top && lh >= 2 && lh <= top;
+    const int n = ok ? 1 << (lw + lh) : 0;
+    ok = ok && num_sig >= 1 && num_sig <= n && range >= 256 && range <= 511 &&
+         (unsigned long long)offset + (unsigned long long)n <= P.n_levels;
+    // the models, two to a word from word 3 on: a live LPS probability and 13 bits (chroma codes no
+    // last2 context past 9: its last word is not looked at)
+    if (lane >= 3 && lane < (ch ? 29 : 30))
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int m = (int)(s16)(word >> (16 * k));
+            ok = ok && ((m >> 1) & 1023) >= 4 && m >= 0 && m < 8192;
+        }
+    ok = __all_sync(0xffffffffu, ok);
+    int cnt = 0;
+    u32 len = 0, fixed = 0;
+    if (ok) {
+        const s16 *coef = P.levels + offset;
+        const u16 *scan = P.scan[lw][lh];
+        u32 *list = list_all + offset;
+        int last = -1;                                // position of the last non-zero level before the window
+        for (int base = 0; base < n && cnt < num_sig; base += 32 * CR_LIST_UNROLL) {
+            int c[CR_LIST_UNROLL];
+#pragma unroll
+            for (int j = 0; j < CR_LIST_UNROLL; j++) {
+                const int i = base + 32 * j + lane;
+                c[j] = i < n ? coef[scan[i]] : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < CR_LIST_UNROLL; j++) {
+                const u32 m = __ballot_sync(0xffffffffu, c[j] != 0);
+                if (m == 0) continue;
+                const u32 below = m & ((1u << lane) - 1);
+                const int i = base + 32 * j + lane, at = cnt + __popc(below);
+                if (c[j] != 0 && at < num_sig) {
+                    const int prev = below ? base + 32 * j + 31 - __clz((int)below) : last;
+                    const int run = i - prev - 1, sym = abs(c[j]) - 1;
+                    list[at] = cr_entry(run, sym, i, n);
+                    len += 3 + min(run, 15) + min(sym, 7);
+                    fixed += 1 + (run >= 16 ? cr_egk(run - 17) : 0u) + (sym >= 8 ? cr_egk(sym - 9) : 0u);
+                }
                 cnt += __popc(m);
+                last = base + 32 * j + 31 - __clz((int)m);
             }
         }
-        if (lane == 0) s_cnt[warp][r] = min(cnt, 65535);
+        len = __reduce_add_sync(0xffffffffu, len);
+        fixed = __reduce_add_sync(0xffffffffu, fixed);
+        ok = cnt >= num_sig;
     }
-    __syncwarp();
-    const int i = r0 + lane;
-    if (i >= P.n) return;
-    const CrReq q = P.reqs[i];
-    CrOut o;
-    o.ctx = q.ctx;
-    o.pad = 0;
-    o.bits = ~0u;                     // outside the domain, or fewer levels than num_sig: state unchanged
-    o.range = q.range;
-    if (!cr_valid(q, P.n_levels) || s_cnt[warp][lane] < q.num_sig) {
-        P.out[i] = o;
-        return;
+    if (lane == 0) {
+        O.key[r] = bs_count(O.counts, ok ? len : 0u);
+        P.fixed[r] = ok ? fixed : CR_BAD;
     }
-    CoefCtx &c = o.ctx;
-    const u32 *list = list_all + q.coef_offset;
-    const int n = 1 << (q.log2w + q.log2h);
-    u32 range = q.range, bits = 0;
-    int t0 = 10, last = -1;
-    for (int k = 0; k < q.num_sig; k++) {
-        const u32 e = list[k];
-        const int pos = (int)(e >> 16), level = abs((int)(s16)(e & 0xFFFF));
-        const int run = pos - last - 1;
-        last = pos;
-        cr_unary(range, bits, c.run[t0], c.run[t0 + 1], min(run, 16), 16);
-        if (run >= 16) bits += cr_egk(run - 17);
-        c.run_rdoq[t0] = cr_next(c.run_rdoq[t0], (run == 0) == (c.run_rdoq[t0] & 1));
-        s16 m = c.run_rdoq[t0 + 1];
-        for (int z = 1; z < run; z++) {                // zeros: bin 0
-            const s16 nm = cr_next(m, (m & 1) == 0);
-            if (nm == m) break;                        // a fixed point: the remaining zeros keep it
-            m = nm;
+}
+
+// Coding, 32 chains of like length per CTA in the order of the grouping.  Neither the models nor the
+// order of the bins depend on the range, so the chain splits over the CTA's five warps, lane l of each
+// working on block l: warps 0 to 2 step the run, level and run_rdoq models, warp 3 the last models --
+// each but warp 2 writing a code per bin (the model's LPS range and whether the bin is the MPS) to its
+// place in the block's sequence of bins -- and warp 4 runs the range over the codes, one chunk behind.
+// All but warp 3 take one bin per iteration, whatever symbol of the block it belongs to, so lanes wait
+// for one another only at the end of a chunk.  What bounds a call is its longest chain, one dependent
+// instruction after the other: a lane that codes its block alone, symbol after symbol, has to loop
+// over the longest symbol of its warp each time.
+//
+// The 54 models of a lane's block sit in shared memory as [model][lane].
+constexpr int CR_CTAS = 3;            // CTAs of 74 KB that share an SM
+constexpr int CR_ROLES = 5;
+constexpr int CR_CODES = 256;         // most bins of a chunk
+constexpr int CR_LEVEL_CODES = 25;    // most bins of one level: run 16, level 8, last flag
+
+struct CrShared {
+    CrTable T;
+    u16 mdl[54][32];                  // run, run_rdoq, level (12 each), last1 (6), last2 (12)
+    u16 codes[2][CR_CODES + 4][32];
+    u32 ring[CR_ROLES - 1][BS_RING][32];
+    int n_codes[2][32];
+    int more[2];                      // another chunk follows
+    int group;
+};
+
+// where a lane stands in its block's list
+struct CrWalk {
+    BsWindow list;
+    u32 k, num_sig;
+    int t0;                           // context pair of the next level (2 min(previous level - 1, 5))
+    // the next level: its entry and context pair, and its place nc in the chunk, which moves past it
+    __device__ __forceinline__ u32 take(int &nc, int &at, int &t)
+    {
+        const u32 v = list.take(k++);
+        at = nc;
+        t = t0;
+        const int nl = (v >> 12) & 7;
+        nc += 3 + min((int)(v & 4095), 15) + nl - (int)(v >> 20);
+        t0 = min(nl, 5) << 1;
+        return v;
+    }
+};
+
+// the run (ROLE 0), level (1) or run_rdoq (2) models of a chunk's levels, one bin per iteration: a
+// truncated unary symbol is its first bin ('1' for 0) on the first model of the pair, then '0' per unit
+// and the closing '1' on the second, omitted at the cap (run 16, level 8; run_rdoq has none).  A long
+// run of zeros stops changing the run_rdoq model once its probability is too small to move, so its
+// walk skips to the closing bin there.
+template <int ROLE>
+__device__ __forceinline__ int cr_models(CrShared &S, CrWalk &W, u16 (*codes)[32], int lane)
+{
+    int nc = 0, at = 0, t = 0, z = 0, cnt = -1, target = 0;
+    for (;;) {
+        if (z > cnt) {                                 // the symbol is done
+            if (W.k >= W.num_sig || nc > CR_CODES - CR_LEVEL_CODES) break;
+            const u32 v = W.take(nc, at, t);
+            const int run = v & 4095, nr = min(run, 15), nl = (v >> 12) & 7;
+            target = ROLE == 1 ? nl + (int)((v >> 15) & 1) : run;
+            cnt = ROLE == 0 ? nr : ROLE == 1 ? nl : run;
+            at += ROLE == 1 ? 1 + nr : 0;
+            t += ROLE == 0 ? 0 : ROLE == 1 ? 24 : 12;
+            z = 0;
         }
-        if (run > 0) m = cr_next(m, (m & 1) == 1);     // the closing '1'
-        c.run_rdoq[t0 + 1] = m;
-        cr_unary(range, bits, c.level[t0], c.level[t0 + 1], min(level - 1, 8), 8);
-        if (level >= 9) bits += cr_egk(level - 10);
-        bits++;                                       // sign
-        if (pos == n - 1) break;
-        s16 &m1 = c.last1[t0 >> 1];
-        s16 &m2 = c.last2[31 - __clz(pos + 1)];
-        t0 = min(level - 1, 5) << 1;
-        const int p1 = (m1 & 2047) >> 1, p2 = (m2 & 2047) >> 1, c1 = m1 & 1, c2 = m2 & 1;
-        int cm, pl;
-        if (c1 == c2) { cm = c1; pl = (p1 + p2) >> 1; }
-        else if (p1 < p2) { cm = c1; pl = 1023 - ((p2 - p1) >> 1); }
-        else { cm = c2; pl = 1023 - ((p1 - p2) >> 1); }
-        const int flag = k == q.num_sig - 1;
-        u32 mps = range - ((u32)pl >> 2);
-        const int s = mps < 256;
-        mps |= 0x100;
-        if (flag == cm) { bits += s; range = mps; }
-        else {
-            const u32 l = (range << s) - mps;
-            const int sh = __clz(l) - 23;
-            range = l << sh;
-            bits += sh + s;
-        }
-        m1 = cr_next(m1, flag == c1);
-        m2 = cr_next(m2, flag == c2);
+        u16 &slot = S.mdl[t + (z > 0 ? 1 : 0)][lane];
+        const u32 m = slot, bin = z == target ? 1u : 0u;
+        const u32 nm = cr_step(S.T, m, bin);
+        if (ROLE != 2) codes[at + z][lane] = cr_code_of(m, bin);
+        slot = (u16)nm;
+        z = (ROLE == 2 && nm == m && z > 0 && z < target) ? target : z + 1;
     }
-    o.bits = bits;
-    o.range = (u16)range;
-    P.out[i] = o;
+    return nc;
+}
+
+// the last flags of a chunk's levels, each on the averaged pair of its two models
+__device__ __forceinline__ void cr_lasts(CrShared &S, CrWalk &W, u16 (*codes)[32], int lane)
+{
+    int nc = 0;
+    while (W.k < W.num_sig && nc <= CR_CODES - CR_LEVEL_CODES) {
+        int at, t;
+        const u32 v = W.take(nc, at, t);
+        if (v >> 20) break;                            // the last scan position has no flag
+        const int i1 = 36 + (t >> 1), i2 = 42 + (int)((v >> 16) & 15);
+        const u32 f1 = S.mdl[i1][lane], f2 = S.mdl[i2][lane];
+        const u32 p1 = (f1 & 2047) >> 1, p2 = (f2 & 2047) >> 1, c1 = f1 & 1, c2 = f2 & 1;
+        const bool first = p1 < p2;
+        const u32 cm = (c1 == c2 || first) ? c1 : c2;
+        const u32 pl = c1 == c2 ? (p1 + p2) >> 1 : 1023 - ((first ? p2 - p1 : p1 - p2) >> 1);
+        const u32 flag = W.k == W.num_sig ? 1u : 0u;
+        codes[nc - 1][lane] = (u16)((pl >> 2) | (flag == cm ? 256u : 0u));
+        S.mdl[i1][lane] = (u16)cr_step(S.T, f1, flag);
+        S.mdl[i2][lane] = (u16)cr_step(S.T, f2, flag);
+    }
+}
+
+__global__ void __launch_bounds__(32 * CR_ROLES) k_cr_code(const CrParams P, const u32 *list_all, const BlockOrder O)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CrShared &S = *reinterpret_cast<CrShared *>(smem_raw);
+    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < 2 * 8192; k += 32 * CR_ROLES)
+        S.T.next[k] = (u16)cr_next((u32)k >> 1, (k & 1) == ((k >> 1) & 1));
+    // a role's models: words [w0, w1) of the request's 27 and the same words of the result
+    const int w0 = role == 0 ? 0 : role == 1 ? 12 : role == 2 ? 6 : 18, w1 = role == 3 ? 27 : role == 4 ? 18 : w0 + 6;
+    // groups of 32 chains from the work counter, the longest chains first
+    for (;;) {
+        if (threadIdx.x == 0) S.group = (int)atomicAdd(O.counts + BS_WORK, 1u);
+        __syncthreads();
+        if (S.group * 32 >= P.n) return;
+        const int at = S.group * 32 + lane;
+        const bool mine = at < P.n;
+        const int i = mine ? O.perm[at] : 0;
+        const u32 *qw = reinterpret_cast<const u32 *>(P.reqs + i);
+        u32 *ow = reinterpret_cast<u32 *>(P.out + i);
+        const u32 fixed = mine ? P.fixed[i] : CR_BAD, sr = qw[2];
+        CrWalk W;
+        W.k = 0;
+        W.num_sig = fixed == CR_BAD ? 0u : sr & 0xffff;    // a bad request codes no level: its state stays
+        W.list.open(list_all + qw[0], role < 4 ? W.num_sig : 0u, smem_addr(&S.ring[role & 3][0][lane]));
+        W.t0 = 10;
+        for (int k = w0; k < w1; k++) {
+            const u32 x = qw[3 + k];
+            S.mdl[2 * k][lane] = (u16)x;
+            S.mdl[2 * k + 1][lane] = (u16)(x >> 16);
+        }
+        u32 range = sr >> 16, bits = fixed;
+        bool fill = true;
+        for (int s = 0;; s++) {
+            const int b = s & 1;
+            u16 (*codes)[32] = S.codes[b];
+            if (fill) {
+                if (role == 0) {
+                    const int nc = cr_models<0>(S, W, codes, lane);
+                    // up to a multiple of four codes: an MPS with LPS range 0 changes nothing
+#pragma unroll
+                    for (int j = 0; j < 3; j++) codes[nc + j][lane] = 256;
+                    S.n_codes[b][lane] = nc;
+                    const int more = __any_sync(0xffffffffu, W.k < W.num_sig);
+                    if (lane == 0) S.more[b] = more;
+                } else if (role == 1) {
+                    cr_models<1>(S, W, codes, lane);
+                } else if (role == 2) {
+                    cr_models<2>(S, W, codes, lane);
+                } else if (role == 3) {
+                    cr_lasts(S, W, codes, lane);
+                }
+            }
+            if (role == 4 && s > 0) {
+                codes = S.codes[b ^ 1];
+                const int nc = S.n_codes[b ^ 1][lane];
+                for (int j = 0; j < nc; j += 4) {
+                    u32 c[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) c[q] = codes[j + q][lane];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) cr_code(range, bits, c[q] & 255, c[q] >> 8);
+                }
+            }
+            __syncthreads();
+            if (!fill) break;
+            fill = S.more[b] != 0;
+        }
+        W.list.close();
+        if (mine) {
+            for (int k = w0; k < w1; k++) ow[2 + k] = (u32)S.mdl[2 * k][lane] | (u32)S.mdl[2 * k + 1][lane] << 16;
+            if (role == 4) {
+                ow[0] = bits;                          // CR_BAD = ~0 for a bad request
+                ow[1] = range;
+            }
+        }
+    }
 }
 
 int launch_coef_rate(const void *reqs, int n, const s16 *levels, unsigned long long n_levels, void *out,
@@ -210,12 +351,30 @@ int launch_coef_rate(const void *reqs, int n, const s16 *levels, unsigned long l
     P.reqs = (const CrReq *)reqs; P.n = n; P.levels = levels; P.n_levels = n_levels; P.out = (CrOut *)out;
     for (int a = 0; a < 7; a++)
         for (int b = 0; b < 7; b++) P.scan[a][b] = tab->scan[a][b];
-    u32 *list = nullptr;                              // one word per level, at the levels' offsets
-    UC_CHECK(cudaMallocAsync((void **)&list, (size_t)n_levels * sizeof(u32), st));
-    k_coef_rate<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(P, list);
-    UC_CHECK(cudaGetLastError());
-    UC_CHECK(cudaFreeAsync(list, st));
-    count_launch(1);
+    // one word per level (the lists, at the levels' offsets), the grouping's arrays, a word per block
+    const size_t b_list = ((size_t)n_levels * sizeof(u32) + 255) & ~(size_t)255, b_order = bs_bytes((size_t)n);
+    char *ws = nullptr;
+    int rc = work_alloc((void **)&ws, b_list + b_order + (size_t)n * sizeof(u32), st);
+    if (rc) return rc;
+    u32 *list = (u32 *)ws;
+    const BlockOrder O = bs_place(ws + b_list, (size_t)n);
+    P.fixed = (u32 *)(ws + b_list + b_order);
+    // persistent CTAs: each fills its model table once
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_cr_code, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CrShared));
+    if (e == cudaSuccess) e = cudaMemsetAsync(O.counts, 0, BS_CLEAR, st);
+    if (e == cudaSuccess) {
+        k_cr_list<<<(unsigned)((n + CR_LIST_WARPS - 1) / CR_LIST_WARPS), 32 * CR_LIST_WARPS, 0, st>>>(P, list, O);
+        k_bs_scatter<<<(unsigned)((n + BS_BUCKETS - 1) / BS_BUCKETS), BS_BUCKETS, 0, st>>>(O.key, O.counts, n, O.perm);
+        k_cr_code<<<(unsigned)std::min((n + 31) / 32, sms * CR_CTAS), 32 * CR_ROLES, sizeof(CrShared), st>>>(P, list, O);
+        e = cudaGetLastError();
+    }
+    rc = work_free(ws, st);
+    UC_CHECK(e);
+    if (rc) return rc;
+    count_launch(3);
     return UC_OK;
 }
 

@@ -3,13 +3,17 @@
 // the encoder derived from its entropy-coder state (rdoq_init_cu_est_bits, :139-156) -- the
 // levels and the count of coded coefficients bit-exact with the reference's call.
 //
-// One warp per 32 blocks.  First the warp takes its blocks one by one: zeroes the coefficients
-// past 32 columns / rows, runs quant_check, and lists in scan order the positions whose
-// first-pass level (quant_rdoq) is not zero (ballot + prefix count).  The decision pass is a
-// chain (each coded level selects the contexts of the next), so then every lane walks the chain
-// of one block over its listed positions: a run of z zero levels adds
+// Two launches with a grouping between them.  k_rdoq_list, a warp per block: zeroes the coefficients
+// past 32 columns / rows, runs quant_check, and lists in scan order the positions whose first-pass
+// level (quant_rdoq) is not zero.  The decision pass is a chain (each coded level selects the
+// contexts of the next), so k_rdoq_chain walks one block per lane over its listed positions, the
+// blocks ordered by their position counts (blocksort.cuh): a run of z zero levels adds
 // est_run[last_b_zero][0] + (z - 1) est_run[1][0] bits at once, as the reference's per-position
-// loop accumulates them.
+// loop accumulates them.  The listing is bound by memory latency (60 us for 60,000 blocks of the 23
+// shapes, 39 M coefficients), the chains by the dependent instructions of the longest block (0.30 ms
+// for 860 positions, about 190 instructions each).  One launch in which a warp listed its 32 blocks one
+// after the other and then walked them, whatever their lengths, took 1.10 ms.
+#include "blocksort.cuh"
 #include "common.cuh"
 #include "quant_tables.cuh"
 #include "tables.h"
@@ -22,7 +26,7 @@
 
 namespace uc {
 
-constexpr int RQ_WARPS = 4;
+constexpr int RQ_WARPS = 2;          // blocks per CTA of the listing: they differ in size, few wait for one another
 
 struct RdoqReq {
     u32 coef_offset; u8 log2w, log2h, qp, is_intra, ch_type, slice_type; u16 est; u32 pad; s64 lambda;
@@ -46,91 +50,156 @@ struct RdoqParams {
     s32 err_scale[80][6];     // tbl_rdoq_err_scale (rdoq_init_err_scale, src/quant.c:69-83), 8-bit
 };
 
-// rdoq_one_coef (src/quant.c:158-194)
-__device__ __forceinline__ u32 rq_coef(s64 uncoded, s64 *coded, u32 level_double, u32 abs_level, const s32 *est_run,
-                                       const s32 (*est_level)[2], int q_bits, s32 err_scale, s64 lambda, bool last_pos)
+// rate of a level (>= 1) beside the run's, rdoq_one_coef (src/quant.c:158-194): l0 / l1 = the costs of
+// the first and the further bins of the level symbol
+__device__ __forceinline__ s32 rq_level_rate(u32 level, int2 l0, int2 l1)
 {
-    u32 best = 0;
-    *coded = uncoded + (s64)est_run[0] * lambda;
-    for (int checks = 2; abs_level && checks; checks--, abs_level--) {
-        const s32 diff = (s32)(level_double - (abs_level << q_bits));
-        const s64 err = ((s64)diff * err_scale) >> 20;
-        s32 rate = 32768;
-        if (!last_pos) rate += est_run[1];
-        if (abs_level == 1) rate += est_level[0][1];
-        else if (abs_level < 9) rate += est_level[0][0] + est_level[1][0] * (s32)(abs_level - 2) + est_level[1][1];
-        else rate += est_level[0][0] + est_level[1][0] * 7 + (((31 - __clz((int)abs_level - 8)) << 1) + 1) * 32768;
-        const s64 cost = err * err + (s64)rate * lambda;
-        if (cost < *coded) { best = abs_level; *coded = cost; }
-    }
-    return best;
+    const s32 mid = l0.x + l1.x * (s32)(level - 2) + l1.y;
+    const s32 far = l0.x + l1.x * 7 + (((31 - __clz((int)level - 8)) << 1) + 1) * 32768;
+    return level == 1 ? l0.y : (level < 9 ? mid : far);
 }
 
-__global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq(const RdoqParams P)
+// block r's samples in shared memory while its positions are listed: rows below 32 (the coded part
+// of a 64-sample side), raster order
+constexpr int RQ_STAGE = 32 * 64;
+constexpr int RQ_UNROLL = 4;         // 32-position windows whose shared loads are in flight together
+
+// Listing, a warp per block: zeroes the coefficients past 32 columns / rows, runs quant_check and, for
+// a block that is coded, lists in scan order the positions whose first-pass level (quant_rdoq) is
+// not zero (a ballot and a prefix count per 32 positions), clears the block (the chain writes its
+// levels) and counts it into the grouping by its positions.  The block is read from memory once, by
+// 16-byte vectors where it starts on a 16-byte boundary.
+template <bool VEC>
+__device__ __forceinline__ void rq_list_block(const RdoqParams &P, const RdoqReq &q, int r, s16 *st, int lane,
+                                              const BlockOrder &O)
 {
-    __shared__ int s_cnt[RQ_WARPS][32];        // marked positions of each of the warp's blocks, -1: done
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = (blockIdx.x * RQ_WARPS + warp) * 32;
-    if (r0 >= P.n) return;
-    // phase 1, the warp over each of its 32 blocks in turn
-    for (int b = 0; b < 32; b++) {
-        const int r = r0 + b;
-        if (r >= P.n) break;
-        const RdoqReq q = P.reqs[r];
-        const int lw = q.log2w, lh = q.log2h, w = 1 << lw, h = 1 << lh;
-        // blocks outside the supported domain are left untouched, with num_nz = -1
-        if (lw < 2 || lw > 6 || lh < 2 || lh > 6 || q.qp > 79 || q.ch_type > 2 || q.est >= P.n_est ||
-            (unsigned long long)q.coef_offset + (unsigned long long)(w * h) > P.n_coefs) {
-            if (lane == 0) { P.num_nz[r] = -1; s_cnt[warp][b] = -1; }
-            continue;
+    const int lw = q.log2w, lh = q.log2h, w = 1 << lw, h = 1 << lh;
+    s16 *coef = P.coefs + q.coef_offset;
+    const int max_num = w * h, max_used = 1 << (lw + min(5, lh));
+    const int odd = (lw + lh) & 1, log2_size = (lw + lh) >> 1;
+    const int q_bits = 14 + (15 - 8 - log2_size);
+    const int q_value = odd ? ((int)kQScale[q.qp] * 181 + 64) >> 7 : (int)kQScale[q.qp];
+    const int offset = (q.slice_type == 1 ? 201 : 153) << (q_bits - 9);
+    const int nz_thr = ((((1 << q_bits) - offset) << 10) / q_value - 1) >> 10;
+    // rows below 32 into shared memory (columns past 32 as zeros, in memory too); quant_check
+    // (rdoq_quant_block) over these first max_used coefficients
+    bool above = false;
+    if (VEC) {
+        const int nv = max_used / 8;                  // 2 .. 256
+        for (int v0 = lane; v0 < nv; v0 += 32 * RQ_UNROLL) {
+            uint4 x[RQ_UNROLL];
+#pragma unroll
+            for (int j = 0; j < RQ_UNROLL; j++) {
+                const int v = v0 + 32 * j;
+                // w = 64: the vectors of a row's right half are not coded
+                x[j] = v < nv && !(w > 32 && ((8 * v) & 32)) ? reinterpret_cast<const uint4 *>(coef)[v] : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int j = 0; j < RQ_UNROLL; j++) {
+                const int v = v0 + 32 * j;
+                if (v >= nv) break;
+                if (w > 32 && ((8 * v) & 32)) reinterpret_cast<uint4 *>(coef)[v] = x[j];
+                reinterpret_cast<uint4 *>(st)[v] = x[j];
+                const u32 xs[4] = { x[j].x, x[j].y, x[j].z, x[j].w };
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int c0 = (int)(s16)xs[k], c1 = (int)xs[k] >> 16;
+                    above |= c0 > nz_thr || c0 < -nz_thr || c1 > nz_thr || c1 < -nz_thr;
+                }
+            }
         }
-        s16 *coef = P.coefs + q.coef_offset;
-        const int max_num = w * h, max_used = 1 << (lw + min(5, lh));
-        // quant_non_zero: coefficients past 32 columns / rows are zeroed
-        if (w > 32 || h > 32)
-            for (int p = lane; p < max_num; p += 32)
-                if ((p & (w - 1)) >= 32 || (p >> lw) >= 32) coef[p] = 0;
-        __syncwarp();
-        // rdoq_quant_block: quant_check over the first max_used coefficients (raster order)
-        const int odd = (lw + lh) & 1, log2_size = (lw + lh) >> 1;
-        const int q_bits = 14 + (15 - 8 - log2_size);
-        const int q_value = odd ? ((int)kQScale[q.qp] * 181 + 64) >> 7 : (int)kQScale[q.qp];
-        const int offset = (q.slice_type == 1 ? 201 : 153) << (q_bits - 9);
-        const int nz_thr = ((((1 << q_bits) - offset) << 10) / q_value - 1) >> 10;
-        bool above = false;
+        for (int v = max_used / 8 + lane; v < max_num / 8; v += 32)    // rows past 32
+            reinterpret_cast<uint4 *>(coef)[v] = make_uint4(0, 0, 0, 0);
+    } else {
         for (int p = lane; p < max_used; p += 32) {
-            const int c = coef[p];
+            int c = coef[p];
+            if ((p & (w - 1)) >= 32) coef[p] = (s16)(c = 0);
+            st[p] = (s16)c;
             above |= c > nz_thr || c < -nz_thr;
         }
-        if (!__any_sync(0xffffffffu, above)) {
-            if (lane == 0) { P.num_nz[r] = 0; s_cnt[warp][b] = -1; }
-            continue;
-        }
-        // scan order; the positions whose first-pass level (quant_rdoq) is not zero -- exactly
-        // those with |c| >= thr -- are listed in order as (position << 16 | coefficient)
-        const u16 *scan = P.scan[lw][lh];
-        const int thr = ((1 << (q_bits - 1)) - 1) / q_value + 1;
-        u32 *list = P.scratch + q.coef_offset;
-        int cnt = 0;
-        for (int base = 0; base < max_num; base += 32) {
-            const int i = base + lane;
-            const int c = i < max_num ? coef[scan[i]] : 0;
-            const bool mark = abs(c) >= thr;
-            const u32 m = __ballot_sync(0xffffffffu, mark);
-            if (mark) list[cnt + __popc(m & ((1u << lane) - 1))] = ((u32)i << 16) | (u16)c;
-            cnt += __popc(m);
-        }
-        __syncwarp();
-        for (int p = lane; p < max_num; p += 32) coef[p] = 0;   // levels are written over the block
-        if (lane == 0) s_cnt[warp][b] = cnt;
-        __syncwarp();
+        for (int p = max_used + lane; p < max_num; p += 32) coef[p] = 0;
+    }
+    if (!__any_sync(0xffffffffu, above)) {
+        if (lane == 0) { P.num_nz[r] = 0; O.key[r] = bs_count(O.counts, 0); }
+        return;
     }
     __syncwarp();
-    // phase 2: lane b walks the decision chain of block b
-    const int r = r0 + lane;
+    // scan order; the positions whose first-pass level (quant_rdoq) is not zero -- exactly those
+    // with |c| >= thr -- are listed in order as (position << 16 | coefficient).  The zig-zag visits
+    // the anti-diagonals one after the other, so everything past the last kept coefficient's position
+    // lies outside the kept 32 columns / rows.
+    const u16 *scan = P.scan[lw][lh];
+    const int n_scan = (int)P.scanpos[lw][lh][(min(h, 32) - 1) * w + min(w, 32) - 1] + 1;
+    const int thr = ((1 << (q_bits - 1)) - 1) / q_value + 1;
+    u32 *list = P.scratch + q.coef_offset;
+    int cnt = 0;
+    for (int base = 0; base < n_scan; base += 32 * RQ_UNROLL) {
+        int c[RQ_UNROLL];
+#pragma unroll
+        for (int j = 0; j < RQ_UNROLL; j++) {
+            const int i = base + 32 * j + lane, p = i < n_scan ? scan[i] : RQ_STAGE;
+            c[j] = p < max_used ? st[p] : 0;
+        }
+#pragma unroll
+        for (int j = 0; j < RQ_UNROLL; j++) {
+            const bool mark = abs(c[j]) >= thr;
+            const u32 m = __ballot_sync(0xffffffffu, mark);
+            if (mark) list[cnt + __popc(m & ((1u << lane) - 1))] = ((u32)(base + 32 * j + lane) << 16) | (u16)(s16)c[j];
+            cnt += __popc(m);
+        }
+    }
+    if (VEC)
+        for (int v = lane; v < max_used / 8; v += 32) reinterpret_cast<uint4 *>(coef)[v] = make_uint4(0, 0, 0, 0);
+    else
+        for (int p = lane; p < max_used; p += 32) coef[p] = 0;
+    if (lane == 0) { P.num_nz[r] = cnt; O.key[r] = bs_count(O.counts, cnt); }
+}
+
+__global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq_list(const RdoqParams P, BlockOrder O)
+{
+    __shared__ __align__(16) s16 s_stage[RQ_WARPS][RQ_STAGE];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = blockIdx.x * RQ_WARPS + warp;
     if (r >= P.n) return;
-    const int cnt = s_cnt[warp][lane];
-    if (cnt < 0) return;
+    const RdoqReq q = P.reqs[r];
+    const int lw = q.log2w, lh = q.log2h;
+    // blocks outside the supported domain are left untouched, with num_nz = -1
+    if (lw < 2 || lw > 6 || lh < 2 || lh > 6 || q.qp > 79 || q.ch_type > 2 || q.est >= P.n_est ||
+        (unsigned long long)q.coef_offset + (1ull << (lw + lh)) > P.n_coefs) {
+        if (lane == 0) { P.num_nz[r] = -1; O.key[r] = bs_count(O.counts, 0); }
+        return;
+    }
+    if ((((uintptr_t)(P.coefs + q.coef_offset)) & 15) == 0) rq_list_block<true>(P, q, r, s_stage[warp], lane, O);
+    else rq_list_block<false>(P, q, r, s_stage[warp], lane, O);
+}
+
+// N pairs of estimates: 8 or 16 bytes at once where the estimate sets start on 16 bytes (a set is a
+// multiple of 16 bytes long, a class's two run or level pairs start on 16)
+template <int N, bool VEC>
+__device__ __forceinline__ void rq_pairs(const s32 (*p)[2], int2 (&v)[N])
+{
+    if constexpr (VEC && N == 2) {
+        const int4 x = *reinterpret_cast<const int4 *>(p);
+        v[0] = make_int2(x.x, x.y);
+        v[1] = make_int2(x.z, x.w);
+    } else if constexpr (VEC) {
+        v[0] = *reinterpret_cast<const int2 *>(p);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = make_int2(p[k][0], p[k][1]);
+    }
+}
+
+// Decision chains, a block per lane, 32 blocks with about as many listed positions per warp in the
+// order of the grouping.  num_nz[r] holds the positions listed (0 or -1: the block is done).
+template <bool VEC>
+__global__ void __launch_bounds__(32) k_rdoq_chain(const RdoqParams P, const int *perm)
+{
+    const int at = blockIdx.x * 32 + threadIdx.x;
+    if (at >= P.n) return;
+    const int r = perm[at];
+    const int cnt = P.num_nz[r];
+    if (cnt <= 0) return;
     const RdoqReq q = P.reqs[r];
     const int lw = q.log2w, lh = q.log2h, ch = q.ch_type, max_num = 1 << (lw + lh);
     const int odd = (lw + lh) & 1, log2_size = (lw + lh) >> 1;
@@ -150,49 +219,94 @@ __global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq(const RdoqParams P)
     const s32 (*lst)[2] = E.lst[ch != 0][5];
     const s32 (*est_run)[2] = E.run + 10 + base, (*est_lvl)[2] = E.lvl + 10 + base;
     u32 last_b_zero = 0;
-    int end_pos = 0, last_checked = 0, tmp_nz = 0, num_nz = 0, zero_bins = 0, prev = -1;
+    int k_end = -1, k_last = -1, tmp_nz = 0, num_nz = 0, prev = -1;
+    // the list two entries ahead and the next entry's raster position one ahead: neither waits
+    u32 next = list[0], next2 = list[min(1, cnt - 1)];
+    int p_next = scan[next >> 16];
     for (int k = 0; k < cnt; k++) {
-        const u32 ent = list[k];
+        const u32 ent = next;
+        const int p = p_next;
+        next = next2;
+        p_next = scan[next >> 16];
+        next2 = list[min(k + 2, cnt - 1)];
         const int i = (int)(ent >> 16), c = (s16)(ent & 0xffffu);
-        const int z = i - prev - 1;                // zero levels since the previous listed position
+        // every estimate the position may need, loaded at once: which ones follow from the previous
+        // level only
+        const int lg = 31 - __clz(i + 1);
+        int2 rv[2], lv[2], ev[1];
+        rq_pairs<2, VEC>(est_run, rv);
+        rq_pairs<2, VEC>(est_lvl, lv);
+        rq_pairs<1, VEC>(lst + lg, ev);
+        const int2 r0 = rv[0], r1 = rv[1], l0 = lv[0], l1 = lv[1], end = ev[0];
+        // distortions: the scaled magnitude of the coefficient and of its difference from the two
+        // levels tried stays below 2^31 for every block size and QP (2^30 at |c| = 2^15: the scale
+        // undoes the quantiser's), so the squares are 32 x 32-bit products
+        const u32 ld = (u32)abs(c) * (u32)q_value;
+        const s32 e = (s32)(((s64)ld * err_scale) >> 20);
+        const s64 zerr = (s64)e * e;
+        const u32 lev_a = (ld + add) >> q_bits;            // >= 1: a listed position
+        const s32 d_a = (s32)(ld - (lev_a << q_bits)), d_b = d_a + (s32)(1u << q_bits);
+        const s32 e_a = (s32)(((s64)d_a * err_scale) >> 20), e_b = (s32)(((s64)d_b * err_scale) >> 20);
+        const int z = i - prev - 1;                        // zero levels since the previous listed position
+        prev = i;
         if (z > 0) {
-            zero_bins += est_run[last_b_zero][0] + (z - 1) * est_run[1][0];
+            curr_delta += (s64)((last_b_zero ? r1.x : r0.x) + (z - 1) * r1.x) * lambda;
             last_b_zero = 1;
         }
-        prev = i;
-        if (zero_bins) { curr_delta += (s64)zero_bins * lambda; zero_bins = 0; }
-        const u32 ld = (u32)abs(c) * (u32)q_value;
-        const s64 e = ((s64)ld * err_scale) >> 20;
-        const s64 zerr = e * e;
-        const u32 abs_level = (u32)(s16)(u32)(((u64)ld + add) >> q_bits);
-        s64 cc;
-        const u32 level = rq_coef(zerr, &cc, ld, abs_level, est_run[last_b_zero], est_lvl, q_bits, err_scale, lambda,
-                                  i == max_num - 1);
+        // rdoq_one_coef: no level, then the rounded level, then the one below it (if not 0), each kept
+        // when it costs strictly less
+        const int2 run = last_b_zero ? r1 : r0;
+        const s32 rate0 = 32768 + (i == max_num - 1 ? 0 : run.y);
+        s64 cc = zerr + (s64)run.x * lambda;
+        const s64 c_a = (s64)e_a * e_a + (s64)(rate0 + rq_level_rate(lev_a, l0, l1)) * lambda;
+        const s64 c_b = (s64)e_b * e_b + (s64)(rate0 + rq_level_rate(lev_a - 1, l0, l1)) * lambda;
+        u32 level = 0;
+        if (c_a < cc) { cc = c_a; level = lev_a; }
+        if (lev_a > 1 && c_b < cc) { cc = c_b; level = lev_a - 1; }
         curr_delta += cc - zerr;
+        last_b_zero = 1;
         if (level) {
-            last_checked = i;
-            coef[scan[i]] = (s16)(c < 0 ? -(int)level : (int)level);
-            const int lg = 31 - __clz(i + 1);
-            const s64 end_cost = curr_delta + (s64)lst[lg][1] * lambda;
-            curr_delta += (s64)lst[lg][0] * lambda;
+            const s64 end_cost = curr_delta + (s64)end.y * lambda;
+            curr_delta += (s64)end.x * lambda;
+            k_last = k;
+            coef[p] = (s16)(c < 0 ? -(int)level : (int)level);
             tmp_nz++;
-            if (end_cost < best_delta) { best_delta = end_cost; end_pos = i; num_nz += tmp_nz; tmp_nz = 0; }
+            if (end_cost < best_delta) { best_delta = end_cost; k_end = k; num_nz += tmp_nz; tmp_nz = 0; }
             last_b_zero = 0;
             const int cls = min((int)level - 1, 5);
             est_lvl = E.lvl + (cls << 1) + base;
             est_run = E.run + (cls << 1) + base;
             lst = E.lst[ch != 0][cls];
-        } else {
-            last_b_zero = 1;
         }
     }
     if (num_nz)
-        for (int k = 0; k < cnt; k++) {            // positions after the chosen last one, back to zero
-            const int i = (int)(list[k] >> 16);
-            if (i > end_pos && i <= last_checked) coef[scan[i]] = 0;
-        }
+        for (int k = k_end + 1; k <= k_last; k++)  // levels after the chosen last position, back to zero
+            coef[scan[list[k] >> 16]] = 0;
     P.num_nz[r] = num_nz;
 }
+
+// rdoq_init_err_scale (src/quant.c:69-83) for 8-bit: 2^(15 - tr_shift) / q_value in 20-bit fixed
+// point, computed once
+struct RqErrScale {
+    s32 v[80][6];
+    RqErrScale()
+    {
+        static const u16 qs[80] = {
+            16302, 15024, 13777, 12634, 11626, 10624, 9742, 8958, 8192, 7512, 6889, 6305, 5793, 5303, 4878, 4467,
+            4091, 3756, 3444, 3161, 2894, 2654, 2435, 2235, 2048, 1878, 1722, 1579, 1449, 1329, 1218, 1117,
+            1024, 939, 861, 790, 724, 664, 609, 558, 512, 470, 430, 395, 362, 332, 304, 279,
+            256, 235, 215, 197, 181, 166, 152, 140, 128, 116, 108, 99, 91, 83, 76, 69,
+            64, 59, 54, 49, 45, 41, 38, 35, 32, 30, 27, 25, 23, 21, 19, 18,
+        };
+        for (int qp = 0; qp < 80; qp++)
+            for (int i = 0; i < 6; i++) {
+                const int tr_shift = 15 - 8 - (i + 1);
+                double es = pow(2.0, 15 - tr_shift);
+                es = es / qs[qp] / 1;
+                v[qp][i] = (s32)(es * (double)(1 << 20));
+            }
+    }
+};
 
 int launch_rdoq(const void *reqs, int n, const void *ests, int n_est, s16 *coefs, unsigned long long n_coefs,
                 s32 *num_nz, cudaStream_t st)
@@ -210,41 +324,29 @@ int launch_rdoq(const void *reqs, int n, const void *ests, int n_est, s16 *coefs
     P.coefs = coefs; P.n_coefs = n_coefs; P.num_nz = num_nz;
     for (int a = 0; a < 7; a++)
         for (int b = 0; b < 7; b++) { P.scan[a][b] = tab->scan[a][b]; P.scanpos[a][b] = tab->scanpos[a][b]; }
-    // rdoq_init_err_scale for 8-bit: 2^(15 - tr_shift) / q_value in 20-bit fixed point
-    static const u16 qs[80] = {
-        16302, 15024, 13777, 12634, 11626, 10624, 9742, 8958, 8192, 7512, 6889, 6305, 5793, 5303, 4878, 4467,
-        4091, 3756, 3444, 3161, 2894, 2654, 2435, 2235, 2048, 1878, 1722, 1579, 1449, 1329, 1218, 1117,
-        1024, 939, 861, 790, 724, 664, 609, 558, 512, 470, 430, 395, 362, 332, 304, 279,
-        256, 235, 215, 197, 181, 166, 152, 140, 128, 116, 108, 99, 91, 83, 76, 69,
-        64, 59, 54, 49, 45, 41, 38, 35, 32, 30, 27, 25, 23, 21, 19, 18,
-    };
-    for (int qp = 0; qp < 80; qp++)
-        for (int i = 0; i < 6; i++) {
-            const int tr_shift = 15 - 8 - (i + 1);
-            double es = pow(2.0, 15 - tr_shift);
-            es = es / qs[qp] / 1;
-            P.err_scale[qp][i] = (s32)(es * (double)(1 << 20));
-        }
-    // the position lists: one word per coefficient, kept per device and grown on demand
-    {
-        static u32 *scratch[64] = { nullptr };
-        static unsigned long long cap[64] = { 0 };
-        static std::mutex mu;
-        std::lock_guard<std::mutex> lk(mu);
-        if (cap[dev] < n_coefs) {
-            if (scratch[dev]) UC_CHECK(cudaFree(scratch[dev]));
-            scratch[dev] = nullptr;
-            cap[dev] = 0;
-            UC_CHECK(cudaMalloc(&scratch[dev], n_coefs * sizeof(u32)));
-            cap[dev] = n_coefs;
-        }
-        P.scratch = scratch[dev];
-    }
+    static const RqErrScale kErr;
+    memcpy(P.err_scale, kErr.v, sizeof(P.err_scale));
+    // one word per coefficient (the position lists, at the coefficients' offsets) and the grouping's
+    // arrays
+    const size_t b_list = ((size_t)n_coefs * sizeof(u32) + 255) & ~(size_t)255;
+    char *ws = nullptr;
+    int rc = work_alloc((void **)&ws, b_list + bs_bytes((size_t)n), st);
+    if (rc) return rc;
+    P.scratch = (u32 *)ws;
+    const BlockOrder O = bs_place(ws + b_list, (size_t)n);
     prof_begin(PROF_RDOQ, st);
-    const int warps = (n + 31) / 32;
-    k_rdoq<<<(unsigned)((warps + RQ_WARPS - 1) / RQ_WARPS), 32 * RQ_WARPS, 0, st>>>(P);
-    UC_CHECK(cudaGetLastError());
-    count_launch(1);
+    cudaError_t e = cudaMemsetAsync(O.counts, 0, BS_CLEAR, st);
+    if (e == cudaSuccess) {
+        k_rdoq_list<<<(unsigned)((n + RQ_WARPS - 1) / RQ_WARPS), 32 * RQ_WARPS, 0, st>>>(P, O);
+        k_bs_scatter<<<(unsigned)((n + BS_BUCKETS - 1) / BS_BUCKETS), BS_BUCKETS, 0, st>>>(O.key, O.counts, n, O.perm);
+        if (((uintptr_t)ests & 15) == 0) k_rdoq_chain<true><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(P, O.perm);
+        else k_rdoq_chain<false><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(P, O.perm);
+        e = cudaGetLastError();
+    }
+    rc = work_free(ws, st);
+    UC_CHECK(e);
+    if (rc) return rc;
+    count_launch(3);
     prof_end(PROF_RDOQ, st);
     return UC_OK;
 }
