@@ -124,12 +124,15 @@ __device__ __forceinline__ void load_diff(int *d, const pel *o, int io, const pe
 // more on this GPU than the 64-bit multiply.
 __host__ __device__ __forceinline__ u64 had_scale_k(double sq) { return (u64)(2199023255552.0 / sq + 0.5); }
 
+// the double expression, out of line: it is rare and its division is long
+static __device__ __noinline__ u32 had_scale_double(int s, double sq) { return (u32)(int)((double)s / sq * 2.0); }
+
 __device__ __forceinline__ u32 had_scale(int s, double sq, u64 k)
 {
     const u64 prod = (u64)(u32)s * k;
     const u64 frac = prod & ((1ull << 40) - 1);
     if ((u32)s < (1u << 23) && frac >= (1ull << 24) && frac <= (1ull << 40) - (1ull << 24)) return (u32)(prod >> 40);
-    return (u32)(int)((double)s / sq * 2.0);
+    return had_scale_double(s, sq);
 }
 
 // Hadamard SATD of a tw x th tile (com_had_4x4/8x8/16x8/8x16/8x4/4x8, src/com_cost.c:176-710).
