@@ -7,11 +7,21 @@
 //
 // One warp per call.  The CU's org (or bi org) and the current prediction sit in shared memory;
 // the prediction (com_mc_blk_affine_luma, src/com_mc.c:202-250) is rebuilt there after every
-// step, the lanes walk its samples for the SATD tiles and the equation sums, which reduce across
-// the warp in 64-bit integers.  The 4x4 solve runs over the warp's lanes in IEEE double with every
-// operation rounded on its own (no fused multiply-add), in the reference's order.
-#include "common.cuh"
+// step, the lanes walk its samples for the SATD tiles (packed rows, had.cuh) and, a column each, for the
+// equation sums, which reduce across the warp in 64-bit integers.  The 4x4 solve runs over the warp's
+// lanes in IEEE double with every operation rounded on its own (no fused multiply-add), in the
+// reference's order; its divisions run on the integer pipe (f64div.cuh).
+//
+// The 40,860 calls of a 1080p frame take 1.91 ms (6.3 steps a call), issue-bound (61 % of the slots): by
+// cycles the prediction is the largest part, then the solve and the sums.  With the divisions on the FP64
+// pipe (45 % busy), the sums as 14 64-bit products per sample, SATD samples read byte by byte and one
+// column per lane in the prediction it was 2.95 ms.  Solving 32 calls per warp in launches of their own,
+// between launches of one step of every call, took 1.87 ms at this size and twice the time of this kernel
+// below 5,000 calls.
 #include "affine.cuh"
+#include "common.cuh"
+#include "f64div.cuh"
+#include "had.cuh"
 #include "uavs3e_cuda_internal.h"
 #include "../../include/uavs3e_cuda.h"
 
@@ -20,7 +30,6 @@
 
 namespace uc {
 
-constexpr int AME_WARPS = 2;
 constexpr s32 CPMV_MIN = -131072, CPMV_MAX = 131071;
 
 struct AffMeReq {
@@ -65,98 +74,163 @@ __device__ __forceinline__ int ame_bits(const s32 *mv, const s32 *mvp, int num_r
 // com_mc_blk_affine_luma (src/com_mc.c:202-250) into dst (w x h, stride w): each sample takes the
 // MV of its SUB x SUB block (centre, or the control point for the two top corner blocks), rounded
 // to 1/16 and clipped to 18 bits, and is filtered from the integer plane (com_mc_blk_luma, hp).
-// A lane takes one column of one band of sub-blocks (aff_luma_column).
-template <int SUB>
-__device__ void ame_pred_t(const AffMeParams &P, const pel *plane, int x, int y, int w, int h, int lw, const s32 *mv,
-                           pel *dst, int lane)
-{
-    const s32 dhx = ((mv[2] - mv[0]) * 128) >> lw, dhy = ((mv[3] - mv[1]) * 128) >> lw;
-    const s32 dvx = -dhy, dvy = dhx;
-    const int tasks = w * (h / SUB);
-    for (int t = lane; t < tasks; t += 32) {
-        const int c = t & (w - 1), by = (t >> lw) * SUB, bx = c & ~(SUB - 1);
-        int px = bx + SUB / 2, py = by + SUB / 2;
-        if (bx == 0 && by == 0) { px = 0; py = 0; }
-        else if (bx + SUB == w && by == 0) { px = w; py = 0; }
-        const s32 mx = min(max(aff_round7(mv[0] * 128 + dhx * px + dvx * py), CPMV_MIN), CPMV_MAX);
-        const s32 my = min(max(aff_round7(mv[1] * 128 + dhy * px + dvy * py), CPMV_MIN), CPMV_MAX);
-        const int qx = ((x + bx) << 4) + mx, qy = ((y + by) << 4) + my;
-        int v[SUB];
-        aff_luma_column<SUB>(plane, P.i_ref, P.W, P.H, qx, qy, c - bx, v);
-#pragma unroll
-        for (int o = 0; o < SUB; o++) dst[(by + o) * w + c] = (pel)v[o];
-    }
-}
-
+// A lane takes two columns of a band of 4 rows, or 8 where the sub-blocks are 8x8 and that leaves every
+// lane a task, four rows of both at a time (aff_luma_pair).  One copy of the filter for both sizes: with
+// unrolled variants the step kernel waited for instructions a third of its time.
 __device__ __noinline__ void ame_pred(const AffMeParams &P, const pel *plane, int x, int y, int w, int h, int lw,
                                       const s32 *mv, int sub, pel *dst, int lane)
 {
-    if (sub == 8) ame_pred_t<8>(P, plane, x, y, w, h, lw, mv, dst, lane);
-    else ame_pred_t<4>(P, plane, x, y, w, h, lw, mv, dst, lane);
+    const s32 dhx = ((mv[2] - mv[0]) * 128) >> lw, dhy = ((mv[3] - mv[1]) * 128) >> lw;
+    const s32 dvx = -dhy, dvy = dhx;
+    const int lr = sub == 8 && w * h >= 512 ? 3 : 2;       // log2 of a task's rows
+    const int tasks = (w * h) >> (1 + lr);
+#pragma unroll 1
+    for (int t = lane; t < tasks; t += 32) {
+        const int c = (2 * t) & (w - 1), row = ((2 * t) >> lw) << lr, bx = c & -sub, by = row & -sub;
+        int px = bx + (sub >> 1), py = by + (sub >> 1);
+        if (bx == 0 && by == 0) { px = 0; py = 0; }
+        else if (bx + sub == w && by == 0) { px = w; py = 0; }
+        const s32 mx = min(max(aff_round7(mv[0] * 128 + dhx * px + dvx * py), CPMV_MIN), CPMV_MAX);
+        const s32 my = min(max(aff_round7(mv[1] * 128 + dhy * px + dvy * py), CPMV_MIN), CPMV_MAX);
+        const int qx = ((x + bx) << 4) + mx, qy = ((y + by) << 4) + my;
+        pel *d = dst + row * w + c;
+        aff_luma_pair(plane, P.i_ref, P.W, P.H, qx, qy, c - bx, row - by, 1 << (lr - 2), [&](int o, int v0, int v1) {
+            *reinterpret_cast<u16 *>(d + o * w) = (u16)(v0 | v1 << 8);
+        });
+    }
 }
 
-// com_had (src/com_cost.c:712-812) of the w x h block o - p (both stride w) with TW x TH tiles.
-// 2:1 tiles: each pass's group sums move to one lane per tile, and the double normalisation runs
-// once for all (at most 16) tiles of the block instead of once per pass.
-template <int TW, int TH>
-__device__ u32 ame_had_tiles(const pel *o, const pel *p, int w, int h, int lane, double sq32, double sq128, u64 k32,
-                             u64 k128)
+// com_had (src/com_cost.c:712-812) of the 2^lw x 2^lh block o - p (both in shared memory, dense rows):
+// 8x8 tiles of square blocks, 16x8 / 8x16 of the others, 8 lanes to a tile (had.cuh)
+__device__ __noinline__ u32 ame_had(const pel *o, const pel *p, int lw, int lh, int lane, const AffMeParams &P)
 {
-    constexpr int G = 32 / TH;                      // tiles per pass
-    const int ntx = w / TW, ntiles = ntx * (h / TH), total = ntiles * TH;
+    const HadSigns G = had_signs(lane);
+    const bool wide = lw > lh, pair = lw != lh;
+    const int lx = wide ? 4 : 3, ly = pair && !wide ? 4 : 3, lntx = lw - lx;
+    const int po = wide ? 8 : 8 << lw;                 // the second half of a 2:1 tile
+    const int total = 8 << (lntx + lh - ly);           // rows of all tiles: a multiple of 32
     u32 acc = 0;
-    int held = 0;
-    for (int base = 0, pass = 0; base < total; base += 32, pass++) {
-        const int t = base + lane;
-        const bool active = t < total;
-        const int tt = active ? t : 0, tile = tt / TH, row = tt - tile * TH;
-        const int off = ((tile / ntx) * TH + row) * w + (tile % ntx) * TW;
-        const int s = had_tile_sum<TW, TH>(o + off, p + off, active, lane);
-        if (TW == TH) {
-            if (active && row == 0) acc += had_tile_norm<TW, TH>(s, sq32, sq128, k32, k128);
+#pragma unroll 1
+    for (int t = lane; t < total; t += 32) {
+        const int row = t & 7, tile = t >> 3;
+        const int at = (((tile >> lntx) << ly) + row) * (1 << lw) + ((tile & ((1 << lntx) - 1)) << lx);
+        const uint2 ov = *reinterpret_cast<const uint2 *>(o + at), pv = *reinterpret_cast<const uint2 *>(p + at);
+        int q[4], s;
+        had_diff8(ov.x, ov.y, pv.x, pv.y, q);
+        if (pair) {
+            const uint2 ow = *reinterpret_cast<const uint2 *>(o + at + po), pw = *reinterpret_cast<const uint2 *>(p + at + po);
+            int e[4], d[4];
+            had_diff8(ow.x, ow.y, pw.x, pw.y, e);
+#pragma unroll
+            for (int i = 0; i < 4; i++) { d[i] = q[i] - e[i]; q[i] += e[i]; }
+            s = had8_lane(d, G);
+            s += had8_lane(q, G);
         } else {
-            const int got = __shfl_sync(0xffffffffu, s, ((lane - pass * G) * TH) & 31);
-            if (lane >= pass * G && lane < pass * G + G) held = got;
+            s = had8_lane(q, G);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        s += __shfl_xor_sync(0xffffffffu, s, 4);
+        if (row == 0) acc += pair ? had_scale(2 * s, P.sq128, P.k128) : (u32)((2 * s + 2) >> 2);
+    }
+    return __reduce_add_sync(0xffffffffu, acc);
+}
+
+// The sums of one gradient step (affine_sobel_flt_hor / _ver and affine_coef_computer,
+// src/com_util.c:2966-3045): per sample (j, k) the Sobel gradients gx, gy of the prediction at the
+// nearest interior position, the four model columns c0 = gx, c1 = k gx + j gy, c2 = gy, c3 = j gx - k gy
+// and the residual r; e[0..9] = the sums of the products c_i c_j (i <= j), e[10..13] of c_i r, written
+// to dst by the lanes that hold them.
+//
+// A lane walks a column (for 16 columns, half of one), so k is a factor of its sums and only gx gx,
+// gx gy, gy gy (each also times j and j^2) and gx r, gy r (also times j) are summed per sample; a row
+// costs three new samples.  All but the j^2 sums stay below 2^31: |gx|, |gy| <= 1020 and the sum of j
+// over 64 rows is 2016.
+__device__ __noinline__ void ame_equations(const pel *o, const pel *p, int lw, int lh, int lane, s64 *dst)
+{
+    const int w = 1 << lw, h = 1 << lh;
+    s64 e[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) e[i] = 0;
+    const int halves = w < 32 ? 2 : 1, rows = h / halves, j0 = halves == 2 ? (lane >> 4) * rows : 0;
+#pragma unroll 1
+    for (int k = lane & (w - 1); k < w; k += 32) {
+        const int kk = min(max(k, 1), w - 2);
+        const pel *pc = p + kk;
+        s32 xx = 0, xy = 0, yy = 0, jxx = 0, jxy = 0, jyy = 0, xr = 0, yr = 0, jxr = 0, jyr = 0;
+        s64 jjxx = 0, jjxy = 0, jjyy = 0;
+        // rows of the window around the gradient's row: horizontal difference d and smoothing s
+        int jj = min(max(j0, 1), h - 2);
+        const auto load = [&](int row, int &d, int &s) {
+            const pel *q = pc + (row << lw);
+            const int l = q[-1], c = q[0], r = q[1];
+            d = r - l;
+            s = l + 2 * c + r;
+        };
+        int d0, d1, d2, s0, s1, s2;
+        load(jj - 1, d0, s0);
+        load(jj, d1, s1);
+        load(jj + 1, d2, s2);
+#pragma unroll 1
+        for (int j = j0; j < j0 + rows; j++) {
+            const int gx = d0 + 2 * d1 + d2, gy = s2 - s0;
+            const int r = (int)o[(j << lw) + k] - (int)p[(j << lw) + k];
+            const int a = gx * gx, b = gx * gy, c = gy * gy, g = j * r;
+            const int ja = j * a, jb = j * b, jc = j * c;
+            xx += a; xy += b; yy += c;
+            jxx += ja; jxy += jb; jyy += jc;
+            jjxx += (s64)ja * j; jjxy += (s64)jb * j; jjyy += (s64)jc * j;
+            xr += gx * r; yr += gy * r;
+            jxr += gx * g; jyr += gy * g;
+            // the next sample's gradient row is the next one inside the block
+            if (j >= 1 && j < h - 2) {
+                d0 = d1; d1 = d2; s0 = s1; s1 = s2;
+                load(j + 2, d2, s2);
+            }
+        }
+        const s64 K = k, K2 = k * k;
+        e[0] += xx;
+        e[1] += K * xx + jxy;
+        e[2] += xy;
+        e[3] += jxx - K * xy;
+        e[4] += K2 * xx + 2 * K * jxy + jjyy;
+        e[5] += K * xy + jyy;
+        e[6] += K * jxx - K2 * xy + jjxy - K * jyy;
+        e[7] += yy;
+        e[8] += jxy - K * yy;
+        e[9] += jjxx - 2 * K * jxy + K2 * yy;
+        e[10] += xr;
+        e[11] += K * xr + jyr;
+        e[12] += yr;
+        e[13] += jxr - K * yr;
+    }
+    // the 16 sums over the warp: at each step a lane keeps the half of its sums that its bit selects
+    // and sends the other, so 16 exchanges leave sum (bit 4, 3, 2, 1 of the lane) on each lane pair
+#pragma unroll
+    for (int st = 0; st < 4; st++) {
+        const int m = 16 >> st, half = 8 >> st;
+        const bool up = lane & m;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const s64 keep = up ? e[i + half] : e[i], send = up ? e[i] : e[i + half];
+            e[i] = keep + __shfl_xor_sync(0xffffffffu, send, m);
         }
     }
-    if (TW != TH && lane < ntiles) acc = had_tile_norm<TW, TH>(held, sq32, sq128, k32, k128);
-#pragma unroll
-    for (int m = 16; m; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-    return acc;
+    e[0] += __shfl_xor_sync(0xffffffffu, e[0], 1);
+    const int idx = (lane >> 1) & 15;                  // bits 4, 3, 2, 1 of the lane, highest first
+    if (!(lane & 1) && idx < 14) dst[idx] = e[0];
 }
 
-__device__ __noinline__ u32 ame_had(const pel *o, const pel *p, int w, int h, int lane, const AffMeParams &P)
+// IEEE division on the integer pipe (f64div.cuh); zeros, infinities, NaNs, denormals and results outside
+// the normal range take the hardware's.  The elimination's divisions go this way, the back substitution's
+// four (one lane each) to the FP64 pipe: 10 issue slots against 90, and the pipe has room for them -- not
+// for all seven, with which it was busy 45 % of the search and its latency bound the solve.
+__device__ __noinline__ double ame_div_hw(double a, double b) { return __ddiv_rn(a, b); }
+__device__ __noinline__ double ame_div(double a, double b)
 {
-    if (w == h) return ame_had_tiles<8, 8>(o, p, w, h, lane, P.sq32, P.sq128, P.k32, P.k128);
-    if (w > h) return ame_had_tiles<16, 8>(o, p, w, h, lane, P.sq32, P.sq128, P.k32, P.k128);
-    return ame_had_tiles<8, 16>(o, p, w, h, lane, P.sq32, P.sq128, P.k32, P.k128);
-}
-
-// the sums of one gradient step (affine_sobel_flt_hor / _ver and affine_coef_computer,
-// src/com_util.c:2966-3045): per sample the Sobel gradients of the prediction at the nearest
-// interior position, the four model columns c0..c3 and the residual; e[0..9] = the products
-// c_i c_j (i <= j), e[10..13] = c_i * residual, summed over the block and the warp
-__device__ void ame_equations(const pel *o, const pel *p, int w, int h, int lw, int lane, s64 *e)
-{
-#pragma unroll
-    for (int i = 0; i < 14; i++) e[i] = 0;
-    for (int i = lane; i < w * h; i += 32) {
-        const int j = i >> lw, k = i & (w - 1);
-        const int jj = min(max(j, 1), h - 2), kk = min(max(k, 1), w - 2);
-        const pel *q = p + jj * w + kk;
-        const int gx = q[1 - w] - q[-1 - w] + 2 * (q[1] - q[-1]) + q[1 + w] - q[-1 + w];
-        const int gy = q[w - 1] - q[-w - 1] + 2 * (q[w] - q[-w]) + q[w + 1] - q[-w + 1];
-        const int r = (int)o[i] - (int)p[i];
-        const int c0 = gx, c1 = k * gx + j * gy, c2 = gy, c3 = j * gx - k * gy;
-        e[0] += (s64)c0 * c0; e[1] += (s64)c0 * c1; e[2] += (s64)c0 * c2; e[3] += (s64)c0 * c3;
-        e[4] += (s64)c1 * c1; e[5] += (s64)c1 * c2; e[6] += (s64)c1 * c3;
-        e[7] += (s64)c2 * c2; e[8] += (s64)c2 * c3; e[9] += (s64)c3 * c3;
-        e[10] += (s64)c0 * r; e[11] += (s64)c1 * r; e[12] += (s64)c2 * r; e[13] += (s64)c3 * r;
-    }
-#pragma unroll
-    for (int i = 0; i < 14; i++)
-#pragma unroll
-        for (int m = 16; m; m >>= 1) e[i] += __shfl_xor_sync(0xffffffffu, e[i], m);
+    uint64_t r;
+    if (f64_div_bits((uint64_t)__double_as_longlong(a), (uint64_t)__double_as_longlong(b), &r)) return __longlong_as_double((long long)r);
+    return ame_div_hw(a, b);
 }
 
 // (s16) of a double as x86-64 code converts it (the reference's platform): truncation to 32 bits
@@ -177,12 +251,26 @@ __device__ __forceinline__ unsigned long long ame_mag(double v)
     return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
 }
 
+// a component of the solution as a CPMV change at AMVR shift sh (src/inter.c:1412-1436): scaled, rounded
+// half away from zero (d >= 0: +0, -0 and positive values, not NaN) and rounded to the AMVR step
+__device__ __forceinline__ s16 ame_step_mv(double d, int sh)
+{
+    const long long db = __double_as_longlong(d);
+    const bool ge0 = db == (long long)0x8000000000000000ull ||
+                     (db >= 0 && (unsigned long long)db <= 0x7ff0000000000000ull);
+    const double half = ge0 ? 0.5 : -0.5;
+    if (sh == 0) return ame_to_s16(__dadd_rn(__dmul_rn(d, 16.0), half));
+    s16 q = ame_to_s16(__dadd_rn(__dmul_rn(d, 4.0), half));
+    q = (s16)(q << 2);
+    return (s16)(((q + (1 << (sh - 1))) >> sh) << sh);   // com_mv_rounding_s16
+}
+
 // solve_equal (src/inter.c:1280-1315) over the warp and the conversion of its solution to the four
 // CPMV changes (x0, y0, x1, y1) at AMVR shift sh.  Lane 5 r + k (< 25) holds element (r, k) of the
 // augmented matrix (rows 1..4, row 0 being the reference's swap buffer); in step i every element
 // (j > i, k >= i) of the elimination is one lane's a[j][k] - a[i][k] * a[j][i-1] / a[i][i-1], each
 // operation rounded on its own, so the values are the reference's; the back substitution runs on
-// lane 0 in the reference's order.  e[] = the equation sums (identical in every lane).
+// lane 0 in the reference's order.  e[] = the equation sums in shared memory.
 __device__ __noinline__ void ame_solve(const s64 *e, int w, int sh, int lane, s16 *mvd)
 {
     const bool mine = lane < 25;
@@ -191,15 +279,13 @@ __device__ __noinline__ void ame_solve(const s64 *e, int w, int sh, int lane, s1
     const int c = r - 1;
     const int lo = min(c, col), hi = max(c, col);
     const int idx = col == 4 ? 10 + c : (lo == 0 ? hi : (lo == 1 ? 3 + hi : (lo == 2 ? 5 + hi : 9)));
-    s64 val = 0;
-#pragma unroll
-    for (int i = 0; i < 14; i++) val = (i == idx) ? e[i] : val;
-    if (col == 4) val *= 8;
-    double v = (mine && r >= 1) ? __ll2double_rn(val) : 0.0;
+    double v = (mine && r >= 1) ? __ll2double_rn(col == 4 ? 8 * e[idx] : e[idx]) : 0.0;
+#pragma unroll 1
     for (int i = 1; i < 4; i++) {
         // fabs(cand) > best in integers: false when cand is NaN, and nothing exceeds a NaN best
         unsigned long long best = ame_mag(__shfl_sync(0xffffffffu, v, i * 5 + i - 1));
         int bi = i;
+#pragma unroll 1
         for (int j = i + 1; j < 5; j++) {
             const unsigned long long cand = ame_mag(__shfl_sync(0xffffffffu, v, j * 5 + i - 1));
             if (cand <= 0x7ff0000000000000ull && cand > best) { best = cand; bi = j; }
@@ -211,7 +297,7 @@ __device__ __noinline__ void ame_solve(const s64 *e, int w, int sh, int lane, s1
         const double aik = __shfl_sync(0xffffffffu, v, i * 5 + col);
         const double aji = __shfl_sync(0xffffffffu, v, r * 5 + i - 1);
         const double aii = __shfl_sync(0xffffffffu, v, i * 5 + i - 1);
-        if (mine && r > i && col >= i) v = __dsub_rn(v, __ddiv_rn(__dmul_rn(aik, aji), aii));
+        if (mine && r > i && col >= i) v = __dsub_rn(v, ame_div(__dmul_rn(aik, aji), aii));
     }
     double m[25];
 #pragma unroll
@@ -219,13 +305,13 @@ __device__ __noinline__ void ame_solve(const s64 *e, int w, int sh, int lane, s1
     double x[4] = { 0, 0, 0, 0 };
     if (lane == 0) {
 #define A(i, j) m[(i) * 5 + (j)]
-        x[3] = __ddiv_rn(A(4, 4), A(4, 3));
+        x[3] = ame_div_hw(A(4, 4), A(4, 3));
 #pragma unroll
         for (int i = 2; i >= 0; i--) {
             double t = 0;
 #pragma unroll
             for (int j = i + 1; j < 4; j++) t = __dadd_rn(t, __dmul_rn(A(i + 1, j), x[j]));
-            x[i] = __ddiv_rn(__dsub_rn(A(i + 1, 4), t), A(i + 1, i));
+            x[i] = ame_div_hw(__dsub_rn(A(i + 1, 4), t), A(i + 1, i));
         }
 #undef A
     }
@@ -237,19 +323,7 @@ __device__ __noinline__ void ame_solve(const s64 *e, int w, int sh, int lane, s1
         const double wd = (double)w;
         const double d = lane == 0 ? x0 : (lane == 1 ? x2 : (lane == 2 ? __dadd_rn(__dmul_rn(x1, wd), x0)
                                                                         : __dadd_rn(__dmul_rn(-x3, wd), x2)));
-        // d >= 0: +0, -0 and positive values, not NaN
-        const long long db = __double_as_longlong(d);
-        const bool ge0 = db == (long long)0x8000000000000000ull ||
-                         (db >= 0 && (unsigned long long)db <= 0x7ff0000000000000ull);
-        const double half = ge0 ? 0.5 : -0.5;
-        s16 q;
-        if (sh == 0) q = ame_to_s16(__dadd_rn(__dmul_rn(d, 16.0), half));
-        else {
-            q = ame_to_s16(__dadd_rn(__dmul_rn(d, 4.0), half));
-            q = (s16)(q << 2);
-            q = (s16)(((q + (1 << (sh - 1))) >> sh) << sh);   // com_mv_rounding_s16
-        }
-        o = (u32)(u16)q;
+        o = (u32)(u16)ame_step_mv(d, sh);
     }
     u32 packed[2];
     packed[0] = __shfl_sync(0xffffffffu, o, 0) | (__shfl_sync(0xffffffffu, o, 1) << 16);
@@ -266,126 +340,189 @@ __device__ __forceinline__ bool ame_cpmv_ok(const s32 (*m)[2])
            m[1][0] >= CPMV_MIN && m[1][0] <= CPMV_MAX && m[1][1] >= CPMV_MIN && m[1][1] <= CPMV_MAX;
 }
 
-__global__ void __launch_bounds__(32 * AME_WARPS, 20 / AME_WARPS) k_me_affine(const AffMeParams P)
+// calls outside the supported domain (CU inside the picture, sides 16..64, slots, AMVR index,
+// reference index, CPMVs within 18 bits) return cost ~0 with the start CPMVs
+__device__ __forceinline__ bool ame_valid(const AffMeParams &P, const AffMeReq &q)
 {
-    __shared__ __align__(16) pel s_org[AME_WARPS][64 * 64];
-    __shared__ __align__(16) pel s_pred[AME_WARPS][64 * 64];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * AME_WARPS + warp;
-    if (r >= P.n) return;
-    const AffMeReq q = P.reqs[r];
-    AffMeOut *out = P.out + r;
     const int w = q.w, h = q.h, bi = q.flags & UAVS3E_CUDA_AFFME_BI;
-    // calls outside the supported domain (CU inside the picture, sides 16..64, slots, AMVR index,
-    // reference index, CPMVs within 18 bits) return cost ~0 with the start CPMVs
-    if ((w != 16 && w != 32 && w != 64) || (h != 16 && h != 32 && h != 64) || q.x < 0 || q.y < 0 ||
-        q.x + w > P.W || q.y + h > P.H || q.ref_slot >= P.n_slots || (bi && q.other_slot >= P.n_slots) ||
-        q.mvr > 2 || q.refi < 0 || q.refi >= q.num_refp || !ame_cpmv_ok(q.mvp) ||
-        (!(q.flags & UAVS3E_CUDA_AFFME_UNI_START) && !ame_cpmv_ok(q.mv)) || (bi && !ame_cpmv_ok(q.other_mv))) {
-        if (lane == 0) {
-            for (int v = 0; v < 2; v++) { out->mv[v][0] = q.mv[v][0]; out->mv[v][1] = q.mv[v][1]; }
-            out->satd = 0;
-            out->bits = 0;
-            out->cost = ~0ull;
-        }
-        return;
-    }
-    pel *so = s_org[warp], *sp = s_pred[warp];
-    const int lw = 31 - __clz(w), n = w * h;
-    const pel *plane = P.planes[q.ref_slot];
+    return !((w != 16 && w != 32 && w != 64) || (h != 16 && h != 32 && h != 64) || q.x < 0 || q.y < 0 ||
+             q.x + w > P.W || q.y + h > P.H || q.ref_slot >= P.n_slots || (bi && q.other_slot >= P.n_slots) ||
+             q.mvr > 2 || q.refi < 0 || q.refi >= q.num_refp || !ame_cpmv_ok(q.mvp) ||
+             (!(q.flags & UAVS3E_CUDA_AFFME_UNI_START) && !ame_cpmv_ok(q.mv)) || (bi && !ame_cpmv_ok(q.other_mv)));
+}
+
+__device__ __forceinline__ void ame_write_invalid(const AffMeReq &q, AffMeOut *out)
+{
+    for (int v = 0; v < 2; v++) { out->mv[v][0] = q.mv[v][0]; out->mv[v][1] = q.mv[v][1]; }
+    out->satd = 0;
+    out->bits = 0;
+    out->cost = ~0ull;
+}
+
+__device__ __forceinline__ void ame_write_result(const AffMeReq &q, const s32 *mv, u64 best, int best_bits, AffMeOut *out)
+{
+    const u64 satd = best - ame_mv_cost(q.lambda_mv, best_bits);
+    for (int v = 0; v < 2; v++) { out->mv[v][0] = mv[2 * v]; out->mv[v][1] = mv[2 * v + 1]; }
+    out->satd = (u32)satd;
+    out->bits = best_bits;
+    out->cost = satd + ame_mv_cost(q.lambda_mv, best_bits);
+}
+
+// a call's search state: the CPMVs of the last step, the best ones with their cost and bits
+struct AmeState { s32 mvt[4], mv[4]; u64 best; s32 bits, pad; };
+
+// steps of a call at most
+__device__ __forceinline__ int ame_steps(const AffMeReq &q) { return (q.flags & UAVS3E_CUDA_AFFME_BI) ? 5 : 7; }
+
+__device__ __forceinline__ int ame_sub(const AffMeReq &q)
+{
+    return (q.flags & (UAVS3E_CUDA_AFFME_BI | UAVS3E_CUDA_AFFME_SUB8)) ? 8 : 4;
+}
+
+// the org block in so; for a bi call create_bi_org (src/inter.c:55) with the 8x8 prediction of the other
+// list, formed in sp
+__device__ __noinline__ void ame_org(const AffMeParams &P, const AffMeReq &q, pel *so, pel *sp, int lane)
+{
+    const int w = q.w, h = q.h, lw = 31 - __clz(w), n4 = (w * h) >> 2;
     const pel *org = P.org + (long long)q.y * P.i_org + q.x;
-    for (int i = lane; i < n; i += 32) so[i] = org[(i >> lw) * P.i_org + (i & (w - 1))];
-    if (bi) {                                      // create_bi_org (src/inter.c:55), 8x8 prediction
+    u32 *so4 = reinterpret_cast<u32 *>(so);
+#pragma unroll 1
+    for (int i = lane; i < n4; i += 32)
+        so4[i] = had_load4(org + (long long)(i >> (lw - 2)) * P.i_org + ((i << 2) & (w - 1)));
+    if (q.flags & UAVS3E_CUDA_AFFME_BI) {
         const s32 om[4] = { q.other_mv[0][0], q.other_mv[0][1], q.other_mv[1][0], q.other_mv[1][1] };
         ame_pred(P, P.planes[q.other_slot], q.x, q.y, w, h, lw, om, 8, sp, lane);
         __syncwarp();
-        for (int i = lane; i < n; i += 32) so[i] = (pel)min(255, max(0, 2 * (int)so[i] - (int)sp[i]));
+        const u32 *sp4 = reinterpret_cast<const u32 *>(sp);
+#pragma unroll 1
+        for (int i = lane; i < n4; i += 32) {
+            // 2 org - prediction, clipped, byte-wise: s + (s - p) where s >= p, else s - (p - s)
+            const u32 v = so4[i], pv = sp4[i];
+            so4[i] = __vsubus4(__vaddus4(v, __vsubus4(v, pv)), __vsubus4(pv, v));
+        }
     }
     __syncwarp();
-    const int sh = ame_shift(q.mvr), sub = (bi || (q.flags & UAVS3E_CUDA_AFFME_SUB8)) ? 8 : 4;
-    const int other = bi ? q.mot_bits_other : 0;
+}
+
+// the prediction at CPMVs mv into sp, and its com_had against so
+__device__ __forceinline__ u32 ame_cost(const AffMeParams &P, const AffMeReq &q, const s32 *mv, const pel *so, pel *sp, int lane)
+{
+    const int lw = 31 - __clz((int)q.w), lh = 31 - __clz((int)q.h);
+    __syncwarp();
+    ame_pred(P, P.planes[q.ref_slot], q.x, q.y, q.w, q.h, lw, mv, ame_sub(q), sp, lane);
+    __syncwarp();
+    return ame_had(so, sp, lw, lh, lane, P);
+}
+
+// the state before the first step, its prediction in sp: the start CPMVs (for an UNI_START call
+// analyze_affine_uni's choice) and their cost
+__device__ __forceinline__ void ame_start(const AffMeParams &P, const AffMeReq &q, const pel *so, pel *sp, int lane, AmeState &T)
+{
+    const int w = q.w, h = q.h, bi = q.flags & UAVS3E_CUDA_AFFME_BI, sh = ame_shift(q.mvr);
     const s32 mvp[4] = { q.mvp[0][0], q.mvp[0][1], q.mvp[1][0], q.mvp[1][1] };
     s32 mv[4] = { q.mv[0][0], q.mv[0][1], q.mv[1][0], q.mv[1][1] };
-    bool have_pred = false;
     u32 had = 0;
-    if (!bi && (q.flags & UAVS3E_CUDA_AFFME_UNI_START)) {
-        // analyze_affine_uni's start: the MVP, or the uni MV clipped (mv_clip, src/inter.c:1472) and
-        // scaled to 1/16 sample (rounded to whole samples at AMVR index 1), whichever costs less
-        ame_pred(P, plane, q.x, q.y, w, h, lw, mvp, sub, sp, lane);
-        __syncwarp();
-        const u64 c_mvp = (u64)ame_had(so, sp, w, h, lane, P) +
-                          ame_mv_cost(q.lambda_mv, ame_bits(mvp, mvp, q.num_refp, q.refi, sh));
-        const int x4 = q.x << 2, y4 = q.y << 2, w4 = w << 2, h4 = h << 2;
-        const int min_c = (-128 - 4) << 2, max_x = (P.W - 1 + 128 + 4) << 2, max_y = (P.H - 1 + 128 + 4) << 2;
-        s16 mx = (s16)q.mv[0][0], my = (s16)q.mv[0][1];
-        if (x4 + mx < min_c) mx = (s16)(min_c - x4);
-        if (y4 + my < min_c) my = (s16)(min_c - y4);
-        if (x4 + mx + w4 - 4 > max_x) mx = (s16)(max_x - x4 - w4 + 4);
-        if (y4 + my + h4 - 4 > max_y) my = (s16)(max_y - y4 - h4 + 4);
-        s32 tx = (s32)mx * 4, ty = (s32)my * 4;
-        if (q.mvr == 1) {
-            tx = tx >= 0 ? ((tx + 8) >> 4) << 4 : -(((-tx + 8) >> 4) << 4);
-            ty = ty >= 0 ? ((ty + 8) >> 4) << 4 : -(((-ty + 8) >> 4) << 4);
-        }
-        tx = min(max(tx, CPMV_MIN), CPMV_MAX);
-        ty = min(max(ty, CPMV_MIN), CPMV_MAX);
-        const s32 tmp[4] = { tx, ty, tx, ty };
-        __syncwarp();
-        ame_pred(P, plane, q.x, q.y, w, h, lw, tmp, sub, sp, lane);
-        __syncwarp();
-        const u32 had_tmp = ame_had(so, sp, w, h, lane, P);
-        const u64 c_tmp = (u64)had_tmp + ame_mv_cost(q.lambda_mv, ame_bits(tmp, mvp, q.num_refp, q.refi, sh));
-        if (c_tmp < c_mvp) {
-#pragma unroll
-            for (int v = 0; v < 4; v++) mv[v] = tmp[v];
-            have_pred = true;
-            had = had_tmp;
+    // candidates in order: for UNI_START the MVP (0), the uni MV (1) and, where the MVP won, its
+    // prediction again (2); else only the start CPMVs (2)
+    u64 c_mvp = 0;
+#pragma unroll 1
+    for (int k = (!bi && (q.flags & UAVS3E_CUDA_AFFME_UNI_START)) ? 0 : 2; k < 3; k++) {
+        s32 m[4];
+        if (k == 1) {
+            // the uni MV clipped (mv_clip, src/inter.c:1472) and scaled to 1/16 sample (rounded to
+            // whole samples at AMVR index 1)
+            const int x4 = q.x << 2, y4 = q.y << 2, w4 = w << 2, h4 = h << 2;
+            const int min_c = (-128 - 4) << 2, max_x = (P.W - 1 + 128 + 4) << 2, max_y = (P.H - 1 + 128 + 4) << 2;
+            s16 mx = (s16)q.mv[0][0], my = (s16)q.mv[0][1];
+            if (x4 + mx < min_c) mx = (s16)(min_c - x4);
+            if (y4 + my < min_c) my = (s16)(min_c - y4);
+            if (x4 + mx + w4 - 4 > max_x) mx = (s16)(max_x - x4 - w4 + 4);
+            if (y4 + my + h4 - 4 > max_y) my = (s16)(max_y - y4 - h4 + 4);
+            s32 tx = (s32)mx * 4, ty = (s32)my * 4;
+            if (q.mvr == 1) {
+                tx = tx >= 0 ? ((tx + 8) >> 4) << 4 : -(((-tx + 8) >> 4) << 4);
+                ty = ty >= 0 ? ((ty + 8) >> 4) << 4 : -(((-ty + 8) >> 4) << 4);
+            }
+            m[0] = m[2] = min(max(tx, CPMV_MIN), CPMV_MAX);
+            m[1] = m[3] = min(max(ty, CPMV_MIN), CPMV_MAX);
         } else {
 #pragma unroll
-            for (int v = 0; v < 4; v++) mv[v] = mvp[v];
+            for (int v = 0; v < 4; v++) m[v] = k == 0 ? mvp[v] : mv[v];
+        }
+        had = ame_cost(P, q, m, so, sp, lane);
+        const u64 c = (u64)had + ame_mv_cost(q.lambda_mv, ame_bits(m, mvp, q.num_refp, q.refi, sh));
+        if (k == 0) c_mvp = c;
+        if (k == 1) {
+            const bool uni = c < c_mvp;
+#pragma unroll
+            for (int v = 0; v < 4; v++) mv[v] = uni ? m[v] : mvp[v];
+            if (uni) break;
         }
     }
-    if (!have_pred) {
-        __syncwarp();
-        ame_pred(P, plane, q.x, q.y, w, h, lw, mv, sub, sp, lane);
-        __syncwarp();
-        had = ame_had(so, sp, w, h, lane, P);
+#pragma unroll
+    for (int v = 0; v < 4; v++) T.mv[v] = T.mvt[v] = mv[v];
+    T.bits = ame_bits(mv, mvp, q.num_refp, q.refi, sh) + (bi ? q.mot_bits_other : 0);
+    T.best = (u64)ame_mv_cost(q.lambda_mv, T.bits) + (had >> bi);
+}
+
+// the CPMVs after a step's change
+__device__ __forceinline__ void ame_move(const AffMeReq &q, const s16 *mvd, s32 *mvt)
+{
+    const int sh = ame_shift(q.mvr);
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+        s32 m = min(max(mvt[v] + (s32)mvd[v], CPMV_MIN), CPMV_MAX);
+        if (m == CPMV_MAX) m = m >> sh << sh;
+        mvt[v] = m;
     }
-    // affine_me_gradient
-    int best_bits = ame_bits(mv, mvp, q.num_refp, q.refi, sh) + other;
-    u64 best = (u64)ame_mv_cost(q.lambda_mv, best_bits) + (had >> bi);
-    s32 mvt[4] = { mv[0], mv[1], mv[2], mv[3] };
-    for (int iter = 0; iter < (bi ? 5 : 7); iter++) {
-        s64 e[14];
-        ame_equations(so, sp, w, h, lw, lane, e);
+}
+
+// the cost of the moved CPMVs (their prediction in sp); the best is kept
+__device__ __forceinline__ void ame_try(const AffMeParams &P, const AffMeReq &q, const pel *so, pel *sp, int lane, AmeState &T)
+{
+    const int bi = q.flags & UAVS3E_CUDA_AFFME_BI;
+    const s32 mvp[4] = { q.mvp[0][0], q.mvp[0][1], q.mvp[1][0], q.mvp[1][1] };
+    const u32 had = ame_cost(P, q, T.mvt, so, sp, lane);
+    const int bits = ame_bits(T.mvt, mvp, q.num_refp, q.refi, ame_shift(q.mvr)) + (bi ? q.mot_bits_other : 0);
+    const u64 cost = (u64)ame_mv_cost(q.lambda_mv, bits) + (had >> bi);
+    if (cost < T.best) {
+        T.best = cost;
+        T.bits = bits;
+#pragma unroll
+        for (int v = 0; v < 4; v++) T.mv[v] = T.mvt[v];
+    }
+}
+
+// One warp per CTA: calls differ 16-fold in size, and a slot frees as soon as its call ends.  9 KB of
+// shared memory and 80 registers let 24 warps share an SM.
+__global__ void __launch_bounds__(32, 24) k_me_affine(const AffMeParams P)
+{
+    __shared__ __align__(16) pel s_org[64 * 64];
+    __shared__ __align__(16) pel s_pred[64 * 64];
+    __shared__ s64 s_eq[14];
+    const int lane = threadIdx.x, r = blockIdx.x;
+    const AffMeReq q = P.reqs[r];
+    AffMeOut *out = P.out + r;
+    if (!ame_valid(P, q)) {
+        if (lane == 0) ame_write_invalid(q, out);
+        return;
+    }
+    pel *so = s_org, *sp = s_pred;
+    AmeState T;
+    ame_org(P, q, so, sp, lane);
+    ame_start(P, q, so, sp, lane, T);
+    const int steps = ame_steps(q);
+#pragma unroll 1
+    for (int iter = 0; iter < steps; iter++) {
+        ame_equations(so, sp, 31 - __clz((int)q.w), 31 - __clz((int)q.h), lane, s_eq);
+        __syncwarp();
         s16 mvd[4];
-        ame_solve(e, w, sh, lane, mvd);
+        ame_solve(s_eq, q.w, ame_shift(q.mvr), lane, mvd);
         if (!mvd[0] && !mvd[1] && !mvd[2] && !mvd[3]) break;
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            s32 m = min(max(mvt[v] + (s32)mvd[v], CPMV_MIN), CPMV_MAX);
-            if (m == CPMV_MAX) m = m >> sh << sh;
-            mvt[v] = m;
-        }
-        __syncwarp();
-        ame_pred(P, plane, q.x, q.y, w, h, lw, mvt, sub, sp, lane);
-        __syncwarp();
-        const int bits = ame_bits(mvt, mvp, q.num_refp, q.refi, sh) + other;
-        const u64 cost = (u64)ame_mv_cost(q.lambda_mv, bits) + (ame_had(so, sp, w, h, lane, P) >> bi);
-        if (cost < best) {
-            best = cost;
-            best_bits = bits;
-#pragma unroll
-            for (int v = 0; v < 4; v++) mv[v] = mvt[v];
-        }
+        ame_move(q, mvd, T.mvt);
+        ame_try(P, q, so, sp, lane, T);
     }
-    if (lane == 0) {
-        const u64 satd = best - ame_mv_cost(q.lambda_mv, best_bits);
-        for (int v = 0; v < 2; v++) { out->mv[v][0] = mv[2 * v]; out->mv[v][1] = mv[2 * v + 1]; }
-        out->satd = (u32)satd;
-        out->bits = best_bits;
-        out->cost = satd + ame_mv_cost(q.lambda_mv, best_bits);
-    }
+    if (lane == 0) ame_write_result(q, T.mv, T.best, T.bits, out);
 }
 
 int launch_me_affine(int W, int H, const pel *org, int i_org, const pel *const *planes, int n_slots, int i_ref,
@@ -411,7 +548,7 @@ int launch_me_affine(int W, int H, const pel *org, int i_org, const pel *const *
     P.reqs = (const AffMeReq *)reqs;
     P.out = (AffMeOut *)out;
     prof_begin(PROF_AFFME, st);
-    k_me_affine<<<(unsigned)((n + AME_WARPS - 1) / AME_WARPS), 32 * AME_WARPS, 0, st>>>(P);
+    k_me_affine<<<(unsigned)n, 32, 0, st>>>(P);
     UC_CHECK(cudaGetLastError());
     count_launch(1);
     prof_end(PROF_AFFME, st);

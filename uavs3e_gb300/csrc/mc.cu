@@ -217,22 +217,30 @@ __global__ void __launch_bounds__(32 * AFF_WARPS) k_mc_affine(const McParams P, 
         if (q.slot[l] >= 0) { aff_subblock_mvs(q, l, sub, s_mv[warp][k], lane); ls[k++] = l; }
     __syncwarp();
     pel *o = P.out + q.out_offset;
-    // luma: 16-phase filters per sub-block MV, a lane per column of a band of sub-blocks
-    const int tasks = w * (h / sub);
+    // luma: 16-phase filters per sub-block MV, a lane per two columns of a band of 4 rows
+    const int lw = 31 - __clz(w), tasks = (w * h) >> 3;
+#pragma unroll 1
     for (int t = lane; t < tasks; t += 32) {
-        const int c = t % w, by = (t / w) * sub, bx = c & ~(sub - 1);
-        int acc[8];
+        const int c = (2 * t) & (w - 1), row = ((2 * t) >> lw) << 2, bx = c & -sub, by = row & -sub;
+        u32 acc[4];
+#pragma unroll 1
         for (int u = 0; u < k; u++) {
-            const s32 *m = s_mv[warp][u][c >> 2][by >> 2];
+            const s32 *m = s_mv[warp][u][c >> 2][row >> 2];
             const int qx = ((q.x + bx) << 4) + m[0], qy = ((q.y + by) << 4) + m[1];
-            const pel *plane = P.planes[q.slot[ls[u]] * 16];
-            int v[8] = { 0, 0, 0, 0, 0, 0, 0, 0 };
-            if (sub == 8) aff_luma_column<8>(plane, P.i_ref, P.W, P.H, qx, qy, c - bx, v);
-            else aff_luma_column<4>(plane, P.i_ref, P.W, P.H, qx, qy, c - bx, v);
-#pragma unroll
-            for (int i = 0; i < 8; i++) acc[i] = u ? (acc[i] + v[i] + 1) >> 1 : v[i];
+            const bool second = u;
+            aff_luma_pair(P.planes[q.slot[ls[u]] * 16], P.i_ref, P.W, P.H, qx, qy, c - bx, row - by, 1,
+                          [&](int i, int v0, int v1) {
+                              const u32 v = (u32)v0 | (u32)v1 << 16;
+                              // the rounded average in both halves: sums below 2^10
+                              acc[i] = second ? ((acc[i] + v + 0x10001u) >> 1) & 0x00FF00FFu : v;
+                          });
         }
-        for (int i = 0; i < sub; i++) o[(by + i) * w + c] = (pel)acc[i];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            pel *d = o + (row + i) * w + c;
+            d[0] = (pel)acc[i];
+            d[1] = (pel)(acc[i] >> 16);
+        }
     }
     o += w * h;
     // chroma: 4x4 blocks per 8x8 luma with the rounded mean of their four 4x4 MVs
