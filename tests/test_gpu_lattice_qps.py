@@ -1,0 +1,56 @@
+"""QP counts and mode lists of the intra lattice against the oracle: the QPs of a tile run in pairs, a
+job that a QP codes nothing of keeps the prediction's SSD, and a tile holds a bounded number of jobs."""
+import numpy as np
+import pytest
+
+from test_gpu_intra import oracle_lattice
+from uavs3e_gb300.synth import intra_frame
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("ssd", "coef_hash", "num_nz", "last_nz", "sum_abs")
+
+
+def _frames(W, H, seed, noise):
+    org = intra_frame(W, H, seed=seed)
+    rng = np.random.default_rng(seed)
+    rec = np.clip(org.astype(int) + rng.integers(-noise, noise + 1, org.shape), 0, 255).astype(np.uint8)
+    return org, rec
+
+
+@pytest.mark.parametrize("qps", [[37], [63, 0], [51, 22, 63], [30, 63, 4, 45]])
+@pytest.mark.parametrize("ipf", [0, 1])
+def test_lattice_qp_counts(gpu, oracle, qps, ipf):
+    # unsorted QPs, from all jobs coded to none, one to four of them
+    W, H = 128, 72
+    org, rec = _frames(W, H, len(qps) + 10 * ipf, 4)
+    cus = gpu.lattice_cus(W, H)
+    satd, q = gpu.intra_lattice(org, rec, cus, qps, ipf=ipf)
+    satd_o, q_o = oracle_lattice(oracle, org, rec, cus, ipf, qps)
+    assert np.array_equal(satd, satd_o)
+    for f in FIELDS:
+        assert np.array_equal(q[f], q_o[f]), f
+
+
+@pytest.mark.parametrize("n_modes,n_qp", [(1, 2), (4, 1), (17, 3), (20, 2), (32, 1)])
+def test_lattice_mode_list_sizes(gpu, oracle, n_modes, n_qp):
+    import torch
+    W, H, qps = 128, 72, np.array([24, 41, 34][:n_qp], np.int32)
+    org, rec = _frames(W, H, 40 + n_modes, 8)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    satd_o, q_o = oracle_lattice(oracle, org, rec, cus, 1, list(qps))
+    rng = np.random.default_rng(n_modes)
+    modes = np.stack([rng.permutation(33)[:n_modes] for _ in range(n)]).astype(np.uint8)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8), modes)]
+    d_satd = torch.zeros(n * 33, dtype=torch.int32, device="cuda")
+    d_q = torch.zeros(n * 33 * n_qp * gpu.LAT_Q.itemsize, dtype=torch.uint8, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_modes_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, d[3].data_ptr(), n_modes, 1, qps.ctypes.data,
+        n_qp, 1, d_satd.data_ptr(), d_q.data_ptr(), torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    at = (np.arange(n)[:, None] * 33 + modes).ravel()
+    assert np.array_equal(d_satd.cpu().numpy().view(np.uint32)[at], satd_o.ravel()[at])
+    got, want = d_q.cpu().numpy().view(gpu.LAT_Q).reshape(n * 33, n_qp)[at], q_o.reshape(n * 33, n_qp)[at]
+    for f in FIELDS:
+        assert np.array_equal(got[f], want[f]), f

@@ -22,6 +22,12 @@
 // partial butterflies) on the byte/halfword dot-product instructions: the forward row pass is
 // the CU's org part (computed once per CU) minus a dp4a product with the u8 prediction; the
 // column pass and both inverse passes are dp2a products of s16 pairs with s8 matrix rows.
+//
+// The stages are bound by instruction issue and by the waits at their barriers, not by memory (a 1080p
+// frame at four QPs moves 1.06 GB, 0.16 ms of its time).  Prediction by table, four samples a task, the
+// QPs in pairs, the inverse stages over the coded jobs only and the Hadamard rows packed two to a register
+// took a 1080p frame at four QPs from 28.7 to 27.5 ms, 416x240 at one QP with the IPF from 0.83 to 0.81,
+// and SATD of all modes + records of 8 at four QPs on 1272x716 from 6.57 to 5.81.
 #include "lattice_kernel.cuh"
 
 #include <mutex>
@@ -96,6 +102,14 @@ __global__ void __launch_bounds__(256) k_lat_scatter(const LatCu *cus, int n, in
     }
 }
 
+// the prediction table: a CTA per (class, mode)
+__global__ void __launch_bounds__(256) k_lat_table(u32 *tab)
+{
+    const int lw = blockIdx.x / 5 + 2, lh = blockIdx.x % 5 + 2, m = blockIdx.y, w = 1 << lw, h = 1 << lh;
+    for (int p = threadIdx.x; p < w * h; p += blockDim.x)
+        tab[lat_table_at(lw, lh) + m * w * h + p] = lat_table_entry(w, h, m, p & (w - 1), p >> lw);
+}
+
 // plans the queue of one launch: exclusive offsets of the classes' CUs in perm, the classes'
 // tile runs in launch order (only the classes in the mask), the cursors and the tile counter reset
 struct LatPlan { int tiles_per_cu[LAT_SHAPES], nchunk[LAT_SHAPES]; u32 mask; };
@@ -149,14 +163,13 @@ __global__ void __launch_bounds__(LAT_THREADS, 4) k_intra_lattice(const __grid_c
     }
 }
 
-size_t lattice_smem_bytes(int w, int h, int nm)
+int lattice_pred_table(u32 **tab)
 {
-    int lw = 0, lh = 0;
-    while ((1 << lw) < w) lw++;
-    while ((1 << lh) < h) lh++;
-    LatLayout L;
-    lat_layout(lw, lh, nm, LAT_BUDGET, L);
-    return (size_t)L.smem;
+    UC_CHECK(cudaMalloc(tab, LAT_TABLE_ENTRIES * sizeof(u32)));
+    k_lat_table<<<dim3(LAT_SHAPES, 33), 256>>>(*tab);
+    UC_CHECK(cudaGetLastError());
+    UC_CHECK(cudaStreamSynchronize(0));
+    return UC_OK;
 }
 
 // Autotuning of the tile layouts: per device and mode count, the first call with at least
@@ -191,7 +204,7 @@ static int lat_run(LatParams P, const LatCu *cus, int n_cus, int W, int H, const
     int smem = 0;
     for (int c = 0; c < LAT_SHAPES; c++) {
         LatLayout L;
-        lat_layout(c / 5 + 2, c % 5 + 2, P.n_modes, budgets[c], L);
+        lat_layout(c / 5 + 2, c % 5 + 2, P.n_modes, P.n_qp, budgets[c], L);
         Q.tiles_per_cu[c] = L.G; Q.nchunk[c] = L.nchunk;
         if ((mask >> c) & 1) smem = std::max(smem, L.smem);
         P.budget[c] = budgets[c];
@@ -222,7 +235,7 @@ static int lat_tune_class(int c, const LatParams &P, const LatCu *cus, int n_cus
     for (int k = 0; k < LAT_SHAPES; k++) bud[k] = budgets[k];
     for (int b : kLatBudgets) {
         LatLayout L;
-        lat_layout(c / 5 + 2, c % 5 + 2, P.n_modes, b, L);
+        lat_layout(c / 5 + 2, c % 5 + 2, P.n_modes, P.n_qp, b, L);
         if (L.smem > LAT_BUDGET || L.G < 1) continue;
         bool dup = false;
         for (int k = 0; k < seen; k++) dup |= seen_g[k] == L.G && seen_mc[k] == L.MC;
@@ -298,6 +311,7 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
         P.fold[l] = tab->fold[l];
         for (int m = 0; m < 7; m++) P.scanpos[l][m] = tab->scanpos[l][m];
     }
+    P.ipred = tab->ipred;
     P.counts = S.counters; P.cu_off = S.counters + 64; P.tile_off = S.counters + 96; P.perm = S.perm;
     P.next = S.counters + 127;
     // the classes' layouts: tuned on the first call with QPs per device and mode count (that call

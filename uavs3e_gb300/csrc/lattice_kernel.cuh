@@ -2,6 +2,7 @@
 // persistent kernel, the device work queue, the layout tuner and the C ABI are in lattice.cu.
 #pragma once
 #include "common.cuh"
+#include "had.cuh"
 #include "intra.cuh"
 #include "tables.h"
 #include "uavs3e_cuda_internal.h"
@@ -58,7 +59,7 @@ constexpr int LAT_BUDGET = 48 * 1024;   // default dynamic shared bytes per CTA 
 constexpr int LAT_MAX_QP = 4;
 constexpr int LAT_SMEM_MAX = 96 * 1024;   // dynamic shared memory admitted by the kernel attribute
 constexpr int LAT_MAX_G = 8;            // CUs per CTA
-constexpr int LAT_MAX_JOBS = 33 * LAT_MAX_G;
+constexpr int LAT_MAX_JOBS = 144;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
 constexpr int LAT_NB = 592;             // neighbour buffer per CU (INTRA_NEIB_SIZE + pad)
 constexpr int LAT_SHAPES = 25;          // log2 sides 2..6
 
@@ -76,16 +77,17 @@ struct LatLayout {
     int o_cu, cu_bytes;                 // per-CU blocks: org, neighbours, org row-pass sums
     int c_org, c_nb, c_torg;
     int o_job, job_bytes;               // per-job blocks: prediction, T, C, DQ^T, T2
-    int j_pred, j_t, j_c, j_dqt, j_t2;
+    int j_pred, j_t, j_c, j_dqt, j_t2;   // (j_dqt, j_t2: of the first QP of a pair; the second's T2 takes T's place)
+    int j_dqt_b;
     int G, MC, nchunk;                  // CUs per CTA, modes per CTA, mode chunks per CU
     int smem;
 };
 
 __host__ __device__ __forceinline__ int lat_up16(int v) { return (v + 15) & ~15; }
 
-// the layout of a CTA for (2^lw) x (2^lh) CUs and nm modes within `budget` bytes of dynamic
+// the layout of a CTA for (2^lw) x (2^lh) CUs, nm modes and n_qp QPs within `budget` bytes of dynamic
 // shared memory: how many CUs (or which chunk of one CU's modes) a CTA takes
-__host__ __device__ inline void lat_layout(int lw, int lh, int nm, int budget, LatLayout &L)
+__host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int budget, LatLayout &L)
 {
     L.lw = lw; L.lh = lh; L.w = 1 << lw; L.h = 1 << lh;
     L.kw = L.w < 32 ? L.w : 32; L.kh = L.h < 32 ? L.h : 32;
@@ -112,16 +114,19 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int budget, L
     L.cu_bytes = c;
     int j = 0;
     L.j_pred = j; j += lat_up16(L.h * L.ps);
-    L.j_t = j; j += lat_up16(L.kw * L.ts * 2);
+    const int b_t = lat_up16(L.kw * L.ts * 2), b_t2 = lat_up16(L.h * L.t2s * 2);
+    L.j_t = j; j += n_qp > 1 && b_t2 > b_t ? b_t2 : b_t;
     L.j_c = j; j += lat_up16(L.kh * L.cs * 2);
     L.j_dqt = j; j += lat_up16(L.kw * L.ds * 2);
-    L.j_t2 = j; j += lat_up16(L.h * L.t2s * 2);
+    L.j_dqt_b = j; if (n_qp > 1) j += lat_up16(L.kw * L.ds * 2);
+    L.j_t2 = j; j += b_t2;
     L.job_bytes = j;
     const int avail = budget - o;
     // several whole CUs when nm jobs of the shape fit, else one CU and a chunk of its modes
     int G = avail / (nm * L.job_bytes + L.cu_bytes);
     if (G >= 1) {
         L.G = G < LAT_MAX_G ? G : LAT_MAX_G;
+        if (L.G * nm > LAT_MAX_JOBS) L.G = LAT_MAX_JOBS / nm;
         L.MC = nm; L.nchunk = 1;
     } else {
         int J = (avail - L.cu_bytes) / L.job_bytes;
@@ -146,6 +151,7 @@ struct LatParams {
     u32 *satd_out; LatQ *q_out;
     const s8 *fold[7];        // folded DCT2 matrices per log2 size
     const u16 *scanpos[7][7]; // raster -> scan index per (log2 w, log2 h)
+    const u32 *ipred;         // the prediction table (lat_table_at)
     const u8 *modes;          // [CU][n_modes] modes to evaluate, or null for all 33 in order
     int n_modes;
     int budget[LAT_SHAPES];   // dynamic shared bytes of each shape class's layout (lat_layout)
@@ -164,9 +170,12 @@ struct LatShared {
     IpredBlock B[LAT_MAX_G];
     int cu[LAT_MAX_G];
     u8 mode[LAT_MAX_JOBS];
-    u32 satd[LAT_MAX_JOBS], flag[LAT_MAX_JOBS];
-    u32 nz[LAT_MAX_JOBS], sum[LAT_MAX_JOBS], hash[LAT_MAX_JOBS], ssd[LAT_MAX_JOBS];
-    int last[LAT_MAX_JOBS];
+    u32 satd[LAT_MAX_JOBS], ssd0[LAT_MAX_JOBS];   // ssd0: of the prediction, for QPs that code nothing
+    // byte 0: bit q = QP q codes the job; byte 1 + b: the k-th job that QP b of the pair codes
+    u32 flag[LAT_MAX_JOBS];
+    u32 nz[2][LAT_MAX_JOBS], sum[2][LAT_MAX_JOBS], hash[2][LAT_MAX_JOBS], ssd[2][LAT_MAX_JOBS];   // per QP of the pair
+    int last[2][LAT_MAX_JOBS];
+    int coded[2];   // jobs that each QP of the pair codes
     int tables;   // shape class whose matrices and scan table are in place (-1: none)
 };
 
@@ -265,63 +274,178 @@ constexpr int lat_th(int w, int h)
     return w == h ? (w == 4 ? 4 : 8) : w > h ? (h == 4 ? 4 : 8) : (w == 4 ? 8 : 16);
 }
 
-// SATD of every (job, tile) by groups of R lanes (R = 4 or 8, the transform size): lane k of a
-// group holds row k of the tile's difference (of both halves for the 16x8 / 8x16 / 8x4 / 4x8
-// tiles, which combine two R x R transforms), transforms it in registers, and the column
-// transform runs across the group's lanes with shuffles.  Same coefficients, sums and
-// normalisation as satd_tile.
-template <int TW, int TH>
+// sum of the squares of the four byte differences of a and b, plus c
+__device__ __forceinline__ u32 lat_sq4(u32 a, u32 b, u32 c)
+{
+    const u32 d = __vabsdiffu4(a, b);
+    return __dp4a(d, d, c);
+}
+
+// SATD of every (job, tile), a tile row per lane (had.cuh): R = 8 or 4 lanes to a tile, whose two
+// squares (16x8 / 8x16 / 8x4 / 4x8 tiles) a lane holds a row of each.  With SSD, the sum of squared
+// differences of the prediction, which every QP that codes no level of the job keeps, is added to
+// s_ssd0[j] too.
+template <int TW, int TH, bool SSD>
 __device__ __forceinline__ void lat_satd_tiles(int n_tiles, int lnt, int ntx, const u8 *cub, int cu_bytes, int c_org,
-                                               const u8 *jobb, int job_bytes, int j_pred, int ps, int MCv,
-                                               u32 *s_satd, double sq32, double sq128, u64 k32, u64 k128)
+                                               const u8 *jobb, int job_bytes, int j_pred, int ps, u32 mc_magic,
+                                               u32 *s_satd, u32 *s_ssd0, double sq32, double sq128, u64 k32,
+                                               u64 k128)
 {
     constexpr int R = (TW == 4 || TH == 4) ? 4 : 8;
     constexpr bool PAIR = TW != TH, SIDE = TW > TH;
     constexpr int GPW = 32 / R;                       // groups per warp
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = lane % R, grp = lane / R;
+    const HadSigns G = had_signs(lane);
     for (int base = warp * GPW; base < n_tiles; base += (LAT_THREADS / 32) * GPW) {
         const int ti = base + grp;
         const bool act = ti < n_tiles;
         const int tt = act ? ti : base;
         const int j = tt >> lnt, t = tt & ((1 << lnt) - 1);
         const int ox = (t % ntx) * TW, oy = (t / ntx) * TH;
-        const u8 *o = cub + (j / MCv) * cu_bytes + c_org + (oy + k) * ps + ox;
+        const u8 *o = cub + ((u32)j * mc_magic >> 16) * cu_bytes + c_org + (oy + k) * ps + ox;
         const u8 *p = jobb + j * job_bytes + j_pred + (oy + k) * ps + ox;
-        int a[R], b[R];
+        const int bo = SIDE ? R : R * ps;
+        int sum;
+        u32 sq = 0;
+        if constexpr (R == 8) {
+            const uint2 ov = *reinterpret_cast<const uint2 *>(o), pv = *reinterpret_cast<const uint2 *>(p);
+            int q[4];
+            had_diff8(ov.x, ov.y, pv.x, pv.y, q);
+            if (SSD) sq = lat_sq4(ov.y, pv.y, lat_sq4(ov.x, pv.x, 0u));
+            if constexpr (PAIR) {
+                const uint2 ow = *reinterpret_cast<const uint2 *>(o + bo), pw = *reinterpret_cast<const uint2 *>(p + bo);
+                int e[4], d[4];
+                had_diff8(ow.x, ow.y, pw.x, pw.y, e);
+                if (SSD) sq = lat_sq4(ow.y, pw.y, lat_sq4(ow.x, pw.x, sq));
 #pragma unroll
-        for (int c = 0; c < R; c++) a[c] = (int)o[c] - (int)p[c];
-        if (PAIR) {
-            const int bo = SIDE ? R : R * ps;
-#pragma unroll
-            for (int c = 0; c < R; c++) b[c] = (int)o[bo + c] - (int)p[bo + c];
-        }
-        wht<R>(a);
-        if (PAIR) wht<R>(b);
-#pragma unroll
-        for (int d = 1; d < R; d <<= 1) {
-#pragma unroll
-            for (int c = 0; c < R; c++) {
-                const int x = __shfl_xor_sync(0xFFFFFFFFu, a[c], d);
-                a[c] = (k & d) ? x - a[c] : a[c] + x;
-                if (PAIR) {
-                    const int y = __shfl_xor_sync(0xFFFFFFFFu, b[c], d);
-                    b[c] = (k & d) ? y - b[c] : b[c] + y;
-                }
+                for (int i = 0; i < 4; i++) { d[i] = q[i] - e[i]; q[i] += e[i]; }
+                sum = had8_lane(d, G) + had8_lane(q, G);
+            } else {
+                sum = had8_lane(q, G);
+            }
+        } else {
+            const u32 ov = *reinterpret_cast<const u32 *>(o), pv = *reinterpret_cast<const u32 *>(p);
+            const int q0 = (int)(__byte_perm(ov, 0u, 0x4240) - __byte_perm(pv, 0u, 0x4240));
+            const int q1 = (int)(__byte_perm(ov, 0u, 0x4341) - __byte_perm(pv, 0u, 0x4341));
+            if (SSD) sq = lat_sq4(ov, pv, 0u);
+            if constexpr (PAIR) {
+                const u32 ow = *reinterpret_cast<const u32 *>(o + bo), pw = *reinterpret_cast<const u32 *>(p + bo);
+                const int e0 = (int)(__byte_perm(ow, 0u, 0x4240) - __byte_perm(pw, 0u, 0x4240));
+                const int e1 = (int)(__byte_perm(ow, 0u, 0x4341) - __byte_perm(pw, 0u, 0x4341));
+                if (SSD) sq = lat_sq4(ow, pw, sq);
+                sum = had4_lane(q0 - e0, q1 - e1, G) + had4_lane(q0 + e0, q1 + e1, G);
+            } else {
+                sum = had4_lane(q0, q1, G);
             }
         }
-        int sum = 0;
 #pragma unroll
-        for (int c = 0; c < R; c++) sum += PAIR ? 2 * max(abs(a[c]), abs(b[c])) : abs(a[c]);
-#pragma unroll
-        for (int d = 1; d < R; d <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+        for (int d = 1; d < R; d <<= 1) {
+            sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+            if (SSD) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, d);
+        }
+        sum *= 2;
         if (act && k == 0) {
             u32 v;
             if (!PAIR) v = R == 8 ? (u32)((sum + 2) >> 2) : (u32)((sum + 1) >> 1);
             else v = R == 8 ? had_scale(sum, sq128, k128) : had_scale(sum, sq32, k32);
-            atomicAdd(&s_satd[j], v);
+            if (n_tiles >> lnt == n_tiles) {           // one tile per job
+                s_satd[j] = v;
+                if (SSD) s_ssd0[j] = sq;
+            } else {
+                atomicAdd(&s_satd[j], v);
+                if (SSD) atomicAdd(&s_ssd0[j], sq);
+            }
         }
     }
+}
+
+// Prediction table.  A sample of every mode but the plane and the bilinear one is the 4-tap filter of
+// f4tap on four reference samples s[base], s[base + d], s[base + 2 d], s[base + 3 d] (d = 1 or -1; or 0,
+// which copies s[base]: the horizontal, the vertical and, with the DC value kept at LAT_DC, the DC mode;
+// mode 32's 3-tap filter is the 4-tap one with offset 0).  base, d and the filter offset depend on the
+// shape, the mode and the sample only, so they are tabulated once per device: one path for 31 modes, where
+// the mode's own arithmetic took three times the instructions and, on blocks of less than a warp's
+// samples, a pass for each of the modes a warp holds.  An entry is base (16 bits, signed), d (8, signed),
+// offset (8); entries are [class][mode][raster sample].  The end-of-reference clamps of the angular modes
+// have no place in it: the lattice's neighbour arrays repeat their last sample past 2w / 2h.
+constexpr int LAT_DC = -280;                          // where a CU's neighbour array keeps its DC value
+
+// first entry of a class's table
+__host__ __device__ constexpr int lat_table_at(int lw, int lh) { return 33 * (((1 << lw) - 4) * 124 + (1 << lw) * ((1 << lh) - 4)); }
+constexpr int LAT_TABLE_ENTRIES = 33 * 124 * 124;
+
+static __device__ u32 lat_table_entry(int w, int h, int m, int i, int j)
+{
+    int base = 0, d = 0, off = 0;
+    if (m == 0) base = LAT_DC;
+    else if (m == 12) base = 1 + i;
+    else if (m == 24) base = -1 - j;
+    else if (m >= 3 && m <= 11) { base = ang_ctx(m, 0, j + 1, &off) + i; d = 1; }
+    else if (m >= 13 && m <= 23) {
+        const int yy = j - ang_ctx(m, 1, i + 1, &off);
+        if (yy <= -1) { base = i + 2 - ang_ctx(m, 0, j + 1, &off); d = -1; }
+        else { base = -yy - 2; d = 1; }
+    } else if (m >= 25 && m <= 31) { base = -j - ang_ctx(m, 1, i + 1, &off); d = -1; }
+    else if (m == 32) {
+        const int rs = min(h / 2 + w - 1, h), n = (j >> 1) + i;
+        base = n >= rs ? -1 - 2 * rs : (j & 1) ? -3 - 2 * n : -2 - 2 * n;
+        d = -1;
+    }
+    return (u32)(u16)(s16)base | (u32)(u8)(s8)d << 16 | (u32)off << 24;
+}
+
+// four prediction samples of mode m along the row from (x, y), as bytes (com_intra_pred with ipf)
+template <int W, int H>
+__device__ __forceinline__ u32 lat_pred4(const u32 *tab, const pel *s, const IpredBlock &B, int m, int ipf, int x, int y)
+{
+    constexpr int LW_ = W == 4 ? 2 : W == 8 ? 3 : W == 16 ? 4 : W == 32 ? 5 : 6, LH_ = H == 4 ? 2 : H == 8 ? 3 : H == 16 ? 4 : H == 32 ? 5 : 6;
+    int v[4];
+    const bool own = m == 1 || m == 2;                 // their values enter the IPF unclipped
+    if (!own) {
+        const uint4 e4 = __ldg(reinterpret_cast<const uint4 *>(tab + (m * H + y) * W + x));
+        const u32 e[4] = { e4.x, e4.y, e4.z, e4.w };
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const pel *p = s + (int)(s16)(e[k] & 0xFFFF);
+            const int d = (int)(s8)(u8)(e[k] >> 16), off = (int)(e[k] >> 24);
+            const int p0 = p[0], p1 = p[d], p2 = p[2 * d], p3 = p[3 * d];
+            v[k] = (32 * (p0 + 2 * p1 + p2) + off * (p2 + p3 - p0 - p1) + 64) >> 7;   // f4tap
+        }
+    } else if (m == 1) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = (B.pl_t + y * B.pl_c + (x + k) * B.pl_b) >> 5;
+    } else {
+        constexpr int lxy = LW_ + LH_ + 1, offs = 1 << (LW_ + LH_);
+        const int le = s[-y - 1], dx = B.bi_a - le;
+        int predx = (le << LW_) + (x + 1) * dx;
+#pragma unroll
+        for (int k = 0; k < 4; k++, predx += dx) {
+            const int up = s[x + k + 1], refup = (up << LH_) + (y + 1) * (B.bi_b - up);
+            v[k] = ((predx << LH_) + (refup << LW_) + (x + k) * y * B.bi_wt + offs) >> lxy;
+        }
+    }
+    if (ipf) {
+        const int le = s[-y - 1];
+        int ih = LW_ - 2, iv = LH_ - 2, vr = H < 10 ? H : 10, hr = W < 10 ? W : 10;
+        if (m >= 3 && m <= 18) vr = 0;
+        if (m > 18) hr = 0;
+        if (y < vr || x < hr) {
+            const int ct = y < vr ? kIpfParam[iv][y] : 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int cl = x + k < hr ? kIpfParam[ih][x + k] : 0;
+                if (y < vr || x + k < hr) v[k] = (cl * le + ct * s[1 + x + k] + (64 - cl - ct) * v[k] + 32) >> 6;
+            }
+        }
+    }
+    u32 o = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (own) v[k] = min(255, max(0, v[k]));
+        o |= ((u32)v[k] & 255u) << (8 * k);            // (an IPF value may leave 0..255: stored modulo 256)
+    }
+    return o;
 }
 
 // Optional per-stage clocks (built with UAVS3E_LAT_STAGE_CLOCKS, off in the library): thread 0
@@ -357,14 +481,13 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     IpredBlock *sB = S.B;
     int *s_cu = S.cu;
     u8 *s_mode = S.mode;
-    u32 *s_satd = S.satd, *s_flag = S.flag, *s_nz = S.nz, *s_sum = S.sum, *s_hash = S.hash, *s_ssd = S.ssd;
-    int *s_last = S.last;
+    u32 *s_satd = S.satd, *s_flag = S.flag;
 
     LatLayout L;
     LAT_STAGE_BEGIN();
     // compile-time shape: the indices and trip counts below are constants
-    lat_layout(LW, LH, P.n_modes, P.budget[(LW - 2) * 5 + (LH - 2)], L);
-    const int w = L.w, h = L.h, lw = L.lw, lh = L.lh, kw = L.kw, kh = L.kh, lkw = L.lkw, lkh = L.lkh;
+    lat_layout(LW, LH, P.n_modes, P.n_qp, P.budget[(LW - 2) * 5 + (LH - 2)], L);
+    const int w = L.w, h = L.h, lw = L.lw, lh = L.lh, kw = L.kw, kh = L.kh, lkw = L.lkw;
     const int N = w * h, lN = lw + lh;
     constexpr int W_ = 1 << LW, H_ = 1 << LH, KW_ = W_ < 32 ? W_ : 32, KH_ = H_ < 32 ? H_ : 32;
     constexpr int LKW_ = LW < 5 ? LW : 5, LKH_ = LH < 5 ? LH : 5;
@@ -390,6 +513,16 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     u32 *fw = (u32 *)(sm + L.o_fw), *fh = (u32 *)(sm + L.o_fh);
     u32 *fht = (u32 *)(sm + L.o_fht), *fwt = (u32 *)(sm + L.o_fwt);
     u8 *cub = sm + L.o_cu, *jobb = sm + L.o_job;
+
+    // job j -> (CU g, mode m): j = g * MCv + (m - m0)
+#define JG(j) ((int)(((u32)(j) * mc_magic) >> 16))
+#define JPRED(j) (jobb + (j) * L.job_bytes + L.j_pred)
+#define JT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t))
+#define JC(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_c))
+#define JDQT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_dqt))
+#define JDQTB(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_dqt_b))
+#define JT2(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t2))
+#define CORG(g) (cub + (g) * L.cu_bytes + L.c_org)
 
     // ---- matrices: rows packed 4 bytes to a word.  The inverse passes use the even/odd
     // symmetry of the folded DCT2 (row k of an N-point matrix satisfies F[k][N-1-n] =
@@ -421,7 +554,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     for (int j = tid; j < J; j += LAT_THREADS) {
         const int g = j / MCv, mi = m0 + (j - g * MCv);
         s_mode[j] = P.modes ? P.modes[(size_t)perm[cu0 + g] * P.n_modes + mi] : (u8)mi;
-        s_satd[j] = 0; s_flag[j] = 0; s_nz[j] = 0; s_sum[j] = 0; s_hash[j] = 0; s_ssd[j] = 0; s_last[j] = -1;
+        s_satd[j] = 0; s_flag[j] = 0; S.ssd0[j] = 0;
     }
     __syncthreads(); LAT_STAGE(0);
     if (tid == 0) S.tables = cls;   // every thread has read S.tables above
@@ -463,7 +596,9 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     if (tid < Gv) {
         const LatCu cu = P.cus[s_cu[tid]];
         const int avail = (cu.y > 0 ? 1 : 0) | (cu.x > 0 ? 2 : 0) | ((cu.x > 0 && cu.y > 0) ? 4 : 0);
-        ipred_block_setup(cub + tid * L.cu_bytes + L.c_nb + 288, w, h, avail, 8, sB[tid]);
+        pel *nbm = cub + tid * L.cu_bytes + L.c_nb + 288;
+        ipred_block_setup(nbm, w, h, avail, 8, sB[tid]);
+        nbm[LAT_DC] = (pel)sB[tid].dc;
     }
     // org part of the forward row pass: Torg[y][u] = sum_x Fw[u][x] org[y][x] (no transform
     // stage runs when no QP is asked: SATD records only)
@@ -478,21 +613,13 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     }
     __syncthreads(); LAT_STAGE(2);
 
-    // job j -> (CU g, mode m): j = g * MCv + (m - m0)
-#define JG(j) ((int)(((u32)(j) * mc_magic) >> 16))
-#define JPRED(j) (jobb + (j) * L.job_bytes + L.j_pred)
-#define JT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t))
-#define JC(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_c))
-#define JDQT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_dqt))
-#define JT2(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t2))
-#define CORG(g) (cub + (g) * L.cu_bytes + L.c_org)
-
-    // ---- prediction
-    for (int i = tid; i < (J << lN); i += LAT_THREADS) {
-        const int j = i >> lN, p = i & (N - 1);
-        const int g = JG(j), m = s_mode[j];
-        const int x = p & (w - 1), y = p >> lw;
-        JPRED(j)[y * L.ps + x] = (pel)ipred_sample<W_, H_>(cub + g * L.cu_bytes + L.c_nb + 288, sB[g], m, P.ipf, x, y);
+    // ---- prediction, four samples a task
+    for (int i = tid; i < (J << (lN - 2)); i += LAT_THREADS) {
+        const int j = i >> (lN - 2), p = i & ((N >> 2) - 1);
+        const int m = s_mode[j];
+        const int x = (p << 2) & (w - 1), y = p >> (lw - 2), g = JG(j);
+        *reinterpret_cast<u32 *>(JPRED(j) + y * L.ps + x) =
+            lat_pred4<W_, H_>(P.ipred + lat_table_at(LW, LH), cub + g * L.cu_bytes + L.c_nb + 288, sB[g], m, P.ipf, x, y);
     }
     __syncthreads(); LAT_STAGE(3);
 
@@ -500,8 +627,12 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     {
         constexpr int TW = lat_tw(1 << LW, 1 << LH), TH = lat_th(1 << LW, 1 << LH);
         constexpr int lnt = LW + LH - (TW == 16 ? 4 : TW == 8 ? 3 : 2) - (TH == 16 ? 4 : TH == 8 ? 3 : 2);
-        lat_satd_tiles<TW, TH>(J << lnt, lnt, (1 << LW) / TW, cub, L.cu_bytes, L.c_org, jobb, L.job_bytes, L.j_pred, L.ps,
-                               MCv, s_satd, P.sq32, P.sq128, P.k32, P.k128);
+        if (P.n_qp > 0)
+            lat_satd_tiles<TW, TH, true>(J << lnt, lnt, (1 << LW) / TW, cub, L.cu_bytes, L.c_org, jobb, L.job_bytes,
+                                         L.j_pred, L.ps, mc_magic, s_satd, S.ssd0, P.sq32, P.sq128, P.k32, P.k128);
+        else
+            lat_satd_tiles<TW, TH, false>(J << lnt, lnt, (1 << LW) / TW, cub, L.cu_bytes, L.c_org, jobb, L.job_bytes,
+                                          L.j_pred, L.ps, mc_magic, s_satd, S.ssd0, P.sq32, P.sq128, P.k32, P.k128);
     }
     {
         const int sh1 = lw - 2, rnd1 = sh1 > 0 ? 1 << (sh1 - 1) : 0;
@@ -574,19 +705,47 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     for (int j = tid; j < J; j += LAT_THREADS)
         P.satd_out[(size_t)s_cu[JG(j)] * 33 + s_mode[j]] = s_satd[j];
 
-    for (int q = 0; q < P.n_qp; q++) {
-        const int qp = P.qp[q];
-        const u32 q_value = (u32)(((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0));
-        const int thr = ((1 << (q_bits - 1)) - 1) / (int)q_value + 1;
-        const int dq_scale = (int)kDqScale[qp];
-        const int dq_shift = (int)kDqShift[qp] - (15 - 8 - log2_size) + 1;
-        const int dq_off = dq_shift == 0 ? 0 : 1 << (dq_shift - 1);
+    // two QPs at a time: they share the reads of the coefficients, and half the CTA barriers are left
+    for (int q0 = 0; q0 < P.n_qp; q0 += 2) {
+        const int nb = min(2, P.n_qp - q0);
+        u32 q_value[2];
+        int dq_scale[2], dq_shift[2];
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const int qp = P.qp[min(q0 + b, LAT_MAX_QP - 1)];
+            q_value[b] = (u32)(((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0));
+            dq_scale[b] = (int)kDqScale[qp];
+            dq_shift[b] = (int)kDqShift[qp] - (15 - 8 - log2_size) + 1;
+        }
+        // the lists of the jobs each QP codes: quant_check found a coefficient above its threshold, whose
+        // level is then not zero; the others keep the prediction's SSD and empty statistics
+        if (tid < 2) S.coded[tid] = 0;
+        for (int j = tid; j < nb * J; j += LAT_THREADS) {
+            const int b = j >= J ? 1 : 0, jj = j - b * J;
+            S.nz[b][jj] = 0; S.sum[b][jj] = 0; S.hash[b][jj] = 0; S.last[b][jj] = -1; S.ssd[b][jj] = 0;
+        }
+        __syncthreads();
+        for (int base = wbase; base < nb * J; base += LAT_THREADS) {
+            const int j = base + lane, b = j >= J ? 1 : 0, jj = j - b * J;
+            const bool coded = j < nb * J && ((s_flag[jj] >> (q0 + b)) & 1);
+            // a warp may hold jobs of both QPs: one ballot each
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const u32 m = __ballot_sync(0xFFFFFFFFu, coded && b == c);
+                int at = 0;
+                if (lane == 0 && m) at = atomicAdd(&S.coded[c], __popc(m));
+                at = __shfl_sync(0xFFFFFFFFu, at, 0);
+                if (coded && b == c) ((u8 *)s_flag)[4 * (at + __popc(m & ((1u << lane) - 1))) + 1 + c] = (u8)jj;
+            }
+        }
         // first-pass levels, statistics, dequantisation (stored transposed, DQ^T[u][v], each row
         // in even/odd order of v).  The
         // level (|c| q_value + 2^(q_bits-1)) >> q_bits is exact in 32 bits: |c| <= 2^15 and
-        // q_value < 2^15.
-        // A task is one coefficient row v of a job over RU columns (lanes take consecutive v):
-        // the statistics are summed in registers and reduced once per task.
+        // q_value < 2^15; it is 0 below the level threshold and, with q_value 0, for a QP that codes
+        // nothing of the job.  A task is one coefficient row v of a job over RU columns (lanes take
+        // consecutive v) at both QPs: the statistics are summed in registers and reduced once per task.
+        // The position weight of raster position p = v w + u is linear in p but for its lowest bit, and
+        // w and the first column are even: weight = row part + constant of the column.
         {
             constexpr int TPJ = KH_ * NUC, SEG = TPJ < 32 ? TPJ : 32;
             for (int base = wbase; base < J * TPJ; base += LAT_THREADS) {
@@ -594,68 +753,77 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
                 const bool act = i < J * TPJ;
                 const int ii = act ? i : base;
                 const int v = ii & (KH_ - 1), uc = (ii >> LKH_) % NUC, j = ii / TPJ;
-                const bool coded = act && (s_flag[j] >> q & 1);
-                u32 nz = 0, sa = 0, hs = 0;
-                int last = -1;
+                const u32 fl = act ? s_flag[j] >> q0 : 0u;
+                const u32 wrow = (u32)(v * w + uc * RU) * 0x9E3779B1u + 0x7F4A7C15u;
+                u32 cp[RU / 2];
+                const u32 *cw = reinterpret_cast<const u32 *>(JC(j) + v * L.cs + uc * RU);
 #pragma unroll
-                for (int r = 0; r < RU; r++) {
-                    // branch-free: a zero level adds nothing to the statistics and dequantises
-                    // to zero ((0 * scale + 2^(shift-1)) >> shift)
-                    const int u = uc * RU + r;
-                    const int c = coded ? (int)JC(j)[v * L.cs + u] : 0;
-                    const int a = c < 0 ? -c : c;
-                    const int l = a >= thr ? (int)(s16)(((u32)a * q_value + qadd) >> q_bits) : 0;
-                    const int lev = c < 0 ? -l : l;
-                    nz += lev != 0 ? 1u : 0u;
-                    sa += (u32)(lev < 0 ? -lev : lev);
-                    hs += (u32)lev * lat_pos_weight((u32)(v * w + u));
-                    if (lev) last = max(last, (int)s_scan[v * KW_ + u]);
-                    int d = (lev * dq_scale + dq_off) >> dq_shift;
-                    d = min(32767, max(-32768, d));
-                    const int dq = odd ? (d * 181 + 128) >> 8 : d;
-                    if (act) JDQT(j)[u * L.ds + lat_eo(v, KH_)] = (s16)dq;
-                }
-                if (__any_sync(0xFFFFFFFFu, nz != 0)) {
-                    nz = lat_seg_sum<SEG>(nz, lane);
-                    sa = lat_seg_sum<SEG>(sa, lane);
-                    hs = lat_seg_sum<SEG>(hs, lane);
-                    last = lat_seg_max<SEG>(last, lane);
+                for (int r = 0; r < RU / 2; r++) cp[r] = cw[r];
+#pragma unroll 1
+                for (int b = 0; b < nb; b++) {
+                    const u32 on = (fl >> b) & 1;
+                    if (!__any_sync(0xFFFFFFFFu, on)) continue;
+                    const u32 qv = on ? b ? q_value[1] : q_value[0] : 0u;
+                    const int scale = b ? dq_scale[1] : dq_scale[0], shift = b ? dq_shift[1] : dq_shift[0];
+                    s16 *dqt = (b ? JDQTB(j) : JDQT(j)) + uc * RU * L.ds + lat_eo(v, KH_);
+                    u32 mask = 0, sa = 0, hs = 0;
+#pragma unroll
+                    for (int r = 0; r < RU; r++) {
+                        const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
+                        const u32 l = ((u32)abs(c) * qv + qadd) >> q_bits;
+                        const int lev = c < 0 ? -(int)l : (int)l;
+                        mask += min(l, 1u) << r;
+                        sa += l;
+                        hs += (u32)lev * (wrow + ((u32)r * 0x9E3779B1u + (r & 1)));
+                        int d = (lev * scale + (1 << shift >> 1)) >> shift;
+                        d = min(32767, max(-32768, d));
+                        if (act) dqt[r * L.ds] = (s16)(odd ? (d * 181 + 128) >> 8 : d);
+                    }
+                    const u32 nz = lat_seg_sum<SEG>((u32)__popc(mask), lane);
+                    sa = lat_seg_sum<SEG>(sa, lane); hs = lat_seg_sum<SEG>(hs, lane);
+                    // along a row the scan index grows with the column
+                    const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + 31 - __clz((int)mask)] : -1;
+                    const int last = lat_seg_max<SEG>(own_last, lane);
                     if (act && (lane & (SEG - 1)) == 0 && nz) {
-                        atomicAdd(&s_nz[j], nz);
-                        atomicAdd(&s_sum[j], sa);
-                        atomicAdd(&s_hash[j], hs);
-                        atomicMax(&s_last[j], last);
+                        atomicAdd(&S.nz[b][j], nz);
+                        atomicAdd(&S.sum[b][j], sa);
+                        atomicAdd(&S.hash[b][j], hs);
+                        atomicMax(&S.last[b][j], last);
                     }
                 }
             }
         }
         __syncthreads(); LAT_STAGE(6);
-        // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5), only
-        // for jobs with coded levels; a task forms rows y and H-1-y from the even-v and odd-v
+        // the inverse passes run over the coded (job, QP) pairs only
+        const int n0 = S.coded[0], JC2 = n0 + S.coded[1];
+        // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5); a task forms
+        // rows y and H-1-y from the even-v and odd-v
         // sums over CU columns u (T2 rows are stored in even/odd order of u).  Tiles with few
         // jobs take CU/2 columns per task so that the CTA's threads still have a task each.
         auto inv_col = [&](auto cu_tag) {
             constexpr int CU = decltype(cu_tag)::value, NCU = KW_ / CU;
-            for (int i = tid; i < J * NCU * (H_ / 2); i += LAT_THREADS) {
-                const int y = i & (H_ / 2 - 1), uc = (i >> (LH - 1)) % NCU, j = i / ((H_ / 2) * NCU);
-                if (!s_nz[j]) continue;
+            for (int i = tid; i < JC2 * NCU * (H_ / 2); i += LAT_THREADS) {
+                const int y = i & (H_ / 2 - 1), uc = (i >> (LH - 1)) % NCU, k = i / ((H_ / 2) * NCU);
+                const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
+                const s16 *dqt = b ? JDQTB(j) : JDQT(j);
+                s16 *t2b = b ? JT(j) : JT2(j);
                 u32 f[KH_ / 4];
 #pragma unroll
-                for (int k = 0; k < KH_ / 4; k++) f[k] = fht[y * L.fht_ws + k];
+                for (int e = 0; e < KH_ / 4; e++) f[e] = fht[y * L.fht_ws + e];
 #pragma unroll 2   // two columns per step: a full unroll spills at the 64-register limit
                 for (int r = 0; r < CU; r++) {
                     const int u = uc * CU + r;
                     u32 dw[KH_ / 2];
-                    lat_row<KH_ / 2>(JDQT(j) + u * L.ds, dw);
+                    lat_row<KH_ / 2>(dqt + u * L.ds, dw);
                     int e = 0, o = 0;
                     lat_eo_sums<KH_>(dw, f, e, o);
-                    s16 *t2 = JT2(j) + lat_eo(u, KW_);
+                    s16 *t2 = t2b + lat_eo(u, KW_);
                     t2[y * L.t2s] = (s16)min(32767, max(-32768, (e + o + 16) >> 5));
                     t2[(H_ - 1 - y) * L.t2s] = (s16)min(32767, max(-32768, (e - o + 16) >> 5));
                 }
             }
         };
-        if (RU > 2 && J * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, (RU > 2 ? RU / 2 : RU)>{});
+        if (RU > 2 && JC2 * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, (RU > 2 ? RU / 2 : RU)>{});
         else inv_col(std::integral_constant<int, RU>{});
         __syncthreads(); LAT_STAGE(7);
         // inverse row pass, reconstruction, SSD: a task is the column pair x, W-1-x over CY
@@ -664,15 +832,16 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         auto inv_row = [&](auto cy_tag) {
             constexpr int CY = decltype(cy_tag)::value, NCY = H_ / CY;
             constexpr int TPJ = (W_ / 2) * NCY, SEG = TPJ < 32 ? TPJ : 32;
-            for (int base = wbase; base < J * TPJ; base += LAT_THREADS) {
+            for (int base = wbase; base < JC2 * TPJ; base += LAT_THREADS) {
                 const int i = base + lane;
-                const bool act = i < J * TPJ;
+                const bool act = i < JC2 * TPJ;
                 const int ii = act ? i : base;
-                const int x = ii & (W_ / 2 - 1), yc = (ii >> (LW - 1)) % NCY, j = ii / TPJ;
-                const bool coded = s_nz[j] != 0;
+                const int x = ii & (W_ / 2 - 1), yc = (ii >> (LW - 1)) % NCY, k = ii / TPJ;
+                const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
+                const s16 *t2b = b ? JT(j) : JT2(j);
                 u32 f[KW_ / 4];
 #pragma unroll
-                for (int k = 0; k < KW_ / 4; k++) f[k] = fwt[x * L.fwt_ws + k];
+                for (int e = 0; e < KW_ / 4; e++) f[e] = fwt[x * L.fwt_ws + e];
                 const pel *po = CORG(JG(j));
                 const pel *pp = JPRED(j);
                 u32 e = 0;
@@ -680,37 +849,35 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
                 for (int r = 0; r < CY; r++) {
                     const int y = yc * CY + r;
                     int rv0 = pp[y * L.ps + x], rv1 = pp[y * L.ps + W_ - 1 - x];
-                    if (coded) {
-                        u32 tw[KW_ / 2];
-                        lat_row<KW_ / 2>(JT2(j) + y * L.t2s, tw);
-                        int se = 0, so = 0;
-                        lat_eo_sums<KW_>(tw, f, se, so);
-                        const int res0 = min(255, max(-256, (se + so + 2048) >> 12));
-                        const int res1 = min(255, max(-256, (se - so + 2048) >> 12));
-                        rv0 = min(255, max(0, rv0 + res0));
-                        rv1 = min(255, max(0, rv1 + res1));
-                    }
+                    u32 tw[KW_ / 2];
+                    lat_row<KW_ / 2>(t2b + y * L.t2s, tw);
+                    int se = 0, so = 0;
+                    lat_eo_sums<KW_>(tw, f, se, so);
+                    const int res0 = min(255, max(-256, (se + so + 2048) >> 12));
+                    const int res1 = min(255, max(-256, (se - so + 2048) >> 12));
+                    rv0 = min(255, max(0, rv0 + res0));
+                    rv1 = min(255, max(0, rv1 + res1));
                     const int d0 = (int)po[y * L.ps + x] - rv0, d1 = (int)po[y * L.ps + W_ - 1 - x] - rv1;
                     e += (u32)(d0 * d0) + (u32)(d1 * d1);
                 }
                 if (!act) e = 0;
                 e = lat_seg_sum<SEG>(e, lane);
-                if (act && (lane & (SEG - 1)) == 0) atomicAdd(&s_ssd[j], e);
+                if (act && (lane & (SEG - 1)) == 0) atomicAdd(&S.ssd[b][j], e);
             }
         };
-        if (RY > 2 && J * (W_ / 2) * NYC < LAT_THREADS) inv_row(std::integral_constant<int, (RY > 2 ? RY / 2 : RY)>{});
+        if (RY > 2 && JC2 * (W_ / 2) * NYC < LAT_THREADS) inv_row(std::integral_constant<int, (RY > 2 ? RY / 2 : RY)>{});
         else inv_row(std::integral_constant<int, RY>{});
         __syncthreads(); LAT_STAGE(8);
-        for (int j = tid; j < J; j += LAT_THREADS) {
-            const int g = JG(j);
+        for (int i = tid; i < nb * J; i += LAT_THREADS) {
+            const int j = nb == 2 ? i >> 1 : i, b = nb == 2 ? i & 1 : 0, g = JG(j);
+            const bool coded = (s_flag[j] >> (q0 + b)) & 1;
             LatQ o;
-            o.ssd = s_ssd[j];
-            o.coef_hash = s_hash[j];
-            o.num_nz = (u16)s_nz[j];
-            o.last_nz = (s16)s_last[j];
-            o.sum_abs = s_sum[j];
-            P.q_out[((size_t)s_cu[g] * 33 + s_mode[j]) * P.n_qp + q] = o;
-            s_ssd[j] = 0; s_hash[j] = 0; s_nz[j] = 0; s_last[j] = -1; s_sum[j] = 0;
+            o.ssd = coded ? S.ssd[b][j] : S.ssd0[j];
+            o.coef_hash = S.hash[b][j];
+            o.num_nz = (u16)S.nz[b][j];
+            o.last_nz = (s16)S.last[b][j];
+            o.sum_abs = S.sum[b][j];
+            P.q_out[((size_t)s_cu[g] * 33 + s_mode[j]) * P.n_qp + q0 + b] = o;
         }
         __syncthreads(); LAT_STAGE(9);
     }
@@ -720,6 +887,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
 #undef JC
 #undef JDQT
 #undef JT2
+#undef JDQTB
 #undef CORG
 }
 
