@@ -54,3 +54,26 @@ def test_lattice_mode_list_sizes(gpu, oracle, n_modes, n_qp):
     got, want = d_q.cpu().numpy().view(gpu.LAT_Q).reshape(n * 33, n_qp)[at], q_o.reshape(n * 33, n_qp)[at]
     for f in FIELDS:
         assert np.array_equal(got[f], want[f]), f
+
+
+@pytest.mark.parametrize("n_modes", [33, 20, 5])
+def test_lattice_satd_only(gpu, oracle, n_modes):
+    # no QP: the tiles hold predictions alone, so more CUs or modes of one
+    import torch
+    W, H = 136, 72
+    org, rec = _frames(W, H, 60 + n_modes, 6)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    satd_o, _ = oracle_lattice(oracle, org, rec, cus, 0, [32])
+    rng = np.random.default_rng(n_modes)
+    modes = np.stack([rng.permutation(33)[:n_modes] if n_modes < 33 else np.arange(33) for _ in range(n)]).astype(np.uint8)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8), modes)]
+    d_satd = torch.full((n * 33,), -1, dtype=torch.int32, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_modes_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, d[3].data_ptr() if n_modes < 33 else None,
+        n_modes, 0, None, 0, 1, d_satd.data_ptr(), None, torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    want = np.full(n * 33, 0xFFFFFFFF, np.uint32)
+    at = (np.arange(n)[:, None] * 33 + modes).ravel()
+    want[at] = satd_o.ravel()[at]
+    assert np.array_equal(d_satd.cpu().numpy().view(np.uint32), want)

@@ -45,32 +45,22 @@ struct IpredBlock {
     int bi_a, bi_b, bi_wt;        // bilinear corner values and weight
 };
 
-__device__ __forceinline__ void ipred_block_setup(const pel *s, int w, int h, int avail, int bd, IpredBlock &B)
+// the constants from the sums over the neighbours: up and left (w and h samples), ch and cv (the plane
+// mode's weighted differences)
+__device__ __forceinline__ void ipred_block_finish(const pel *s, int w, int h, int avail, int bd, int up, int left, int ch,
+                                                   int cv, IpredBlock &B)
 {
     B.w = w; B.h = h; B.lw = ilog2d(w); B.lh = ilog2d(h); B.avail = avail; B.bd = bd;
     // DC
-    int dc = 0;
-    if (avail & 2) {
-        for (int i = 0; i < h; i++) dc += s[-i - 1];
-        if (avail & 1) {
-            for (int j = 0; j < w; j++) dc += s[j + 1];
-            dc = (dc + ((w + h) >> 1)) * (4096 / (w + h)) >> 12;
-        } else {
-            dc = (dc + (h >> 1)) >> B.lh;
-        }
-    } else if (avail & 1) {
-        for (int j = 0; j < w; j++) dc += s[j + 1];
-        dc = (dc + (w >> 1)) >> B.lw;
-    } else {
-        dc = 1 << (bd - 1);
-    }
+    int dc;
+    if ((avail & 3) == 3) dc = (up + left + ((w + h) >> 1)) * (4096 / (w + h)) >> 12;
+    else if (avail & 2) dc = (left + (h >> 1)) >> B.lh;
+    else if (avail & 1) dc = (up + (w >> 1)) >> B.lw;
+    else dc = 1 << (bd - 1);
     B.dc = dc;
     // plane
     const int mult[5] = { 13, 17, 5, 11, 23 }, shf[5] = { 7, 10, 11, 15, 19 };
     int w2 = w >> 1, h2 = h >> 1, iw = B.lw - 2, ih = B.lh - 2;
-    int ch = 0, cv = 0;
-    for (int x = 1; x <= w2; x++) ch += x * (s[w2 + x] - s[w2 - x]);
-    for (int y = 1; y <= h2; y++) cv += y * (s[-h2 - y] - s[-h2 + y]);
     int a = (s[-h] + s[w]) << 4;
     B.pl_b = ((ch << 5) * mult[iw] + (1 << (shf[iw] - 1))) >> shf[iw];
     B.pl_c = ((cv << 5) * mult[ih] + (1 << (shf[ih] - 1))) >> shf[ih];
@@ -82,6 +72,17 @@ __device__ __forceinline__ void ipred_block_setup(const pel *s, int w, int h, in
     int ba = s[w], bb = s[-h];
     int bc = (w == h) ? (ba + bb + 1) >> 1 : (((ba << B.lw) + (bb << B.lh)) * wc + (1 << (ish + 5))) >> (ish + 6);
     B.bi_a = ba; B.bi_b = bb; B.bi_wt = (bc << 1) - ba - bb;
+}
+
+__device__ __forceinline__ void ipred_block_setup(const pel *s, int w, int h, int avail, int bd, IpredBlock &B)
+{
+    const int w2 = w >> 1, h2 = h >> 1;
+    int up = 0, left = 0, ch = 0, cv = 0;
+    for (int i = 0; i < h; i++) left += s[-i - 1];
+    for (int j = 0; j < w; j++) up += s[j + 1];
+    for (int x = 1; x <= w2; x++) ch += x * (s[w2 + x] - s[w2 - x]);
+    for (int y = 1; y <= h2; y++) cv += y * (s[-h2 - y] - s[-h2 + y]);
+    ipred_block_finish(s, w, h, avail, bd, up, left, ch, cv, B);
 }
 
 __device__ __forceinline__ int ang_ctx(int mode, int xy, int d, int *off)

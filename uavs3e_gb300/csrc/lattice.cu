@@ -27,7 +27,10 @@
 // frame at four QPs moves 1.06 GB, 0.16 ms of its time).  Prediction by table, four samples a task, the
 // QPs in pairs, the inverse stages over the coded jobs only and the Hadamard rows packed two to a register
 // took a 1080p frame at four QPs from 28.7 to 27.5 ms, 416x240 at one QP with the IPF from 0.83 to 0.81,
-// and SATD of all modes + records of 8 at four QPs on 1272x716 from 6.57 to 5.81.
+// and SATD of all modes + records of 5 at four QPs on 1272x716 from 6.57 to 5.81.  A SATD-only tile holds
+// predictions alone, so a CU's samples are fetched for several times as many modes, and a tile begins
+// with two dependent global loads (its CU's position, then the samples) instead of six: 27.3, 0.79 and
+// 3.75 ms.
 #include "lattice_kernel.cuh"
 
 #include <mutex>
@@ -79,7 +82,7 @@ __global__ void __launch_bounds__(256) k_lat_count(const LatCu *cus, int n, int 
 // lists the CUs of each shape (order within a shape is irrelevant: outputs go by CU index):
 // a block reserves one range per shape, its threads fill it
 __global__ void __launch_bounds__(256) k_lat_scatter(const LatCu *cus, int n, int W, int H, const int *offsets,
-                                                     int *cursor, int *perm)
+                                                     int *cursor, LatPerm *perm)
 {
     __shared__ int s_cnt[32], s_base[32];
     if (threadIdx.x < 32) s_cnt[threadIdx.x] = 0;
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(256) k_lat_scatter(const LatCu *cus, int n, in
 #pragma unroll
     for (int k = 0; k < LAT_GROUP_K; k++) {
         const int i = (blockIdx.x * LAT_GROUP_K + k) * blockDim.x + threadIdx.x;
-        if (cls[k] >= 0) perm[s_base[cls[k]] + rank[k]] = i;
+        if (cls[k] >= 0) perm[s_base[cls[k]] + rank[k]] = { i, cus[i].x, cus[i].y };
     }
 }
 
@@ -110,48 +113,60 @@ __global__ void __launch_bounds__(256) k_lat_table(u32 *tab)
         tab[lat_table_at(lw, lh) + m * w * h + p] = lat_table_entry(w, h, m, p & (w - 1), p >> lw);
 }
 
+// the transform and scan tables of the classes, as the tiles hold them
+__global__ void __launch_bounds__(256) k_lat_image(const DevTables t, u8 *images)
+{
+    const int lw = blockIdx.x / 5 + 2, lh = blockIdx.x % 5 + 2;
+    lat_image_fill(t.fold[lw], t.fold[lh], t.scanpos[lw][lh], lw, lh, images + blockIdx.x * LAT_IMAGE_BYTES);
+}
+
 // plans the queue of one launch: exclusive offsets of the classes' CUs in perm, the classes'
 // tile runs in launch order (only the classes in the mask), the cursors and the tile counter reset
 struct LatPlan { int tiles_per_cu[LAT_SHAPES], nchunk[LAT_SHAPES]; u32 mask; };
 
-__global__ void k_lat_plan(int *counters, const LatPlan Q)
+__global__ void __launch_bounds__(32) k_lat_plan(int *counters, const LatPlan Q)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int *counts = counters, *cursor = counters + 32, *cu_off = counters + 64, *tile_off = counters + 96;
-    int o = 0;
-    for (int c = 0; c < LAT_SHAPES; c++) { cu_off[c] = o; o += counts[c]; cursor[c] = 0; }
-    int t = 0;
-    for (int r = 0; r < LAT_SHAPES; r++) {
-        const int c = lat_order(r);
-        tile_off[r] = t;
-        if ((Q.mask >> c) & 1) t += (counts[c] + Q.tiles_per_cu[c] - 1) / Q.tiles_per_cu[c] * Q.nchunk[c];
+    int *cursor = counters + 32, *cu_off = counters + 64, *tile_off = counters + 96;
+    const int r = threadIdx.x, c = r < LAT_SHAPES ? lat_order(r) : 0;   // lane r: class r of cu_off, class c of the queue
+    const int n = r < LAT_SHAPES ? counters[r] : 0, nc = __shfl_sync(0xFFFFFFFFu, n, c);
+    const int t = r < LAT_SHAPES && ((Q.mask >> c) & 1) ? (nc + Q.tiles_per_cu[c] - 1) / Q.tiles_per_cu[c] * Q.nchunk[c] : 0;
+    int sn = n, stl = t;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int an = __shfl_up_sync(0xFFFFFFFFu, sn, d), at = __shfl_up_sync(0xFFFFFFFFu, stl, d);
+        if (r >= d) { sn += an; stl += at; }
     }
-    tile_off[LAT_SHAPES] = t;
-    counters[127] = 0;      // the tile counter
+    if (r < LAT_SHAPES) { cu_off[r] = sn - n; cursor[r] = 0; }
+    if (r <= LAT_SHAPES) tile_off[r] = stl - t;
+    if (r == 0) counters[127] = 0;      // the tile counter
 }
 
 // the persistent lattice: tiles from the queue until it is empty.  Its static shared memory is
-// the tile's LatShared and one word: with a 48 KB layout, four CTAs then still fit an SM (the
-// queue's tile offsets are read from global memory, not copied to shared memory, for that)
+// at most 8 KB: with a 48 KB layout, four CTAs then fit an SM
 __global__ void __launch_bounds__(LAT_THREADS, 4) k_intra_lattice(const __grid_constant__ LatParams P)
 {
     extern __shared__ __align__(16) u8 sm[];
     __shared__ LatShared S;
-    __shared__ int s_t;
     const int tid = threadIdx.x;
-    const int total = __ldg(P.tile_off + LAT_SHAPES);
     if (tid == 0) S.tables = -1;
-    for (;;) {
-        if (tid == 0) s_t = atomicAdd(P.next, 1);
-        __syncthreads();
-        const int t = s_t;
-        __syncthreads();
+    if (tid <= LAT_SHAPES) S.tile_off[tid] = P.tile_off[tid];
+    if (tid < LAT_SHAPES) { S.cu_off[tid] = P.cu_off[tid]; S.counts[tid] = P.counts[tid]; }
+    // a tile's number is taken while the one before it runs, and its class searched from there on
+    const auto search = [&](int t, int r) {
+        while (r < LAT_SHAPES && t >= S.tile_off[r + 1]) r++;
+        return r;
+    };
+    __syncthreads();
+    if (tid == LAT_THREADS - 1) { S.next[0] = atomicAdd(P.next, 1); S.rank[0] = search(S.next[0], 0); }
+    __syncthreads();
+    const int total = S.tile_off[LAT_SHAPES];
+    for (int k = 0;; k ^= 1) {
+        const int t = S.next[k], r = S.rank[k];
         if (t >= total) break;
-        int r = 0;
-        while (t >= __ldg(P.tile_off + r + 1)) r++;
-        const int c = lat_order(r), lt = t - __ldg(P.tile_off + r);
-        const int *perm = P.perm + P.cu_off[c];
-        const int n = P.counts[c];
+        if (tid == LAT_THREADS - 1) S.next[k ^ 1] = atomicAdd(P.next, 1);
+        const int c = lat_order(r), lt = t - S.tile_off[r];
+        const LatPerm *perm = P.perm + S.cu_off[c];
+        const int n = S.counts[c];
         switch (c) {
 #define LAT_CASE(lw, lh) case ((lw) - 2) * 5 + ((lh) - 2): lat_tile<lw, lh>(P, perm, n, lt, sm, S); break;
 #define LAT_ROW(lw) LAT_CASE(lw, 2) LAT_CASE(lw, 3) LAT_CASE(lw, 4) LAT_CASE(lw, 5) LAT_CASE(lw, 6)
@@ -160,15 +175,25 @@ __global__ void __launch_bounds__(LAT_THREADS, 4) k_intra_lattice(const __grid_c
 #undef LAT_CASE
         default: break;
         }
+        if (tid == LAT_THREADS - 1) S.rank[k ^ 1] = search(S.next[k ^ 1], S.rank[k]);
+        __syncthreads();
     }
 }
 
-int lattice_pred_table(u32 **tab)
+int lattice_tables(DevTables &t)
 {
-    UC_CHECK(cudaMalloc(tab, LAT_TABLE_ENTRIES * sizeof(u32)));
-    k_lat_table<<<dim3(LAT_SHAPES, 33), 256>>>(*tab);
+    u32 *ipred = nullptr;
+    u8 *images = nullptr;
+    UC_CHECK(cudaMalloc(&ipred, LAT_TABLE_ENTRIES * sizeof(u32)));
+    UC_CHECK(cudaMalloc(&images, LAT_SHAPES * LAT_IMAGE_BYTES));
+    UC_CHECK(cudaMemset(images, 0, LAT_SHAPES * LAT_IMAGE_BYTES));
+    k_lat_table<<<dim3(LAT_SHAPES, 33), 256>>>(ipred);
     UC_CHECK(cudaGetLastError());
-    UC_CHECK(cudaStreamSynchronize(0));
+    k_lat_image<<<LAT_SHAPES, 256>>>(t, images);
+    UC_CHECK(cudaGetLastError());
+    UC_CHECK(cudaStreamSynchronize(0));   // other streams' calls read them too
+    t.lat_ipred = ipred;
+    t.lat_images = images;
     return UC_OK;
 }
 
@@ -188,7 +213,7 @@ static bool g_tune_on = true;
 
 // per device: the CU permutation and the queue's counters
 struct LatScratch {
-    int *perm = nullptr;
+    LatPerm *perm = nullptr;
     int *counters = nullptr;   // [0, 32) counts, [32, 64) cursors, [64, 96) CU offsets, [96, 122) tile
                                // offsets, [127] tile counter
     size_t cap = 0;
@@ -288,7 +313,7 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
     if (S.cap < (size_t)n_cus) {
         if (S.perm) UC_CHECK(cudaFree(S.perm));
         S.perm = nullptr;
-        UC_CHECK(cudaMalloc(&S.perm, (size_t)n_cus * sizeof(int)));
+        UC_CHECK(cudaMalloc(&S.perm, (size_t)n_cus * sizeof(LatPerm)));
         S.cap = (size_t)n_cus;
     }
     prof_begin(PROF_LATTICE, st);
@@ -301,17 +326,13 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
     memset(&P, 0, sizeof(P));
     P.org = org; P.i_org = i_org; P.rec = rec; P.i_rec = i_rec; P.W = W; P.H = H;
     P.org_words = ((uintptr_t)org % 4 == 0 && i_org % 4 == 0) ? 1 : 0;
-    P.cus = cus; P.ipf = ipf; P.n_qp = n_qp; P.is_intra = is_intra;
+    P.ipf = ipf; P.n_qp = n_qp; P.is_intra = is_intra;
     for (int i = 0; i < LAT_MAX_QP; i++) P.qp[i] = i < n_qp ? qps[i] : 0;
     P.satd_out = satd_out; P.q_out = q_out;
     P.modes = modes; P.n_modes = n_modes;
     P.sq32 = sqrt(32.0); P.sq128 = sqrt(128.0);
     P.k32 = had_scale_k(P.sq32); P.k128 = had_scale_k(P.sq128);
-    for (int l = 0; l < 7; l++) {
-        P.fold[l] = tab->fold[l];
-        for (int m = 0; m < 7; m++) P.scanpos[l][m] = tab->scanpos[l][m];
-    }
-    P.ipred = tab->ipred;
+    P.images = tab->lat_images; P.ipred = tab->lat_ipred;
     P.counts = S.counters; P.cu_off = S.counters + 64; P.tile_off = S.counters + 96; P.perm = S.perm;
     P.next = S.counters + 127;
     // the classes' layouts: tuned on the first call with QPs per device and mode count (that call
@@ -321,7 +342,7 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
     {
         LatTune &T = g_tune[dev];
         std::lock_guard<std::mutex> lk(T.mu);
-        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = T.budget[n_modes][c] ? T.budget[n_modes][c] : LAT_BUDGET;
+        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = n_qp > 0 && T.budget[n_modes][c] ? T.budget[n_modes][c] : LAT_BUDGET;
         if (g_tune_on && !T.done[n_modes] && n_qp > 0) {
             T.done[n_modes] = true;   // one pass: classes with too few CUs keep the default
             int counts[32];

@@ -54,12 +54,14 @@ __device__ __forceinline__ int dp2a_hi(u32 a, u32 b, int c)
 struct LatCu { s16 x, y; u8 w, h; u16 pad; };
 struct LatQ { u32 ssd; u32 coef_hash; u16 num_nz; s16 last_nz; u32 sum_abs; };
 
+struct alignas(8) LatPerm { int id; s16 x, y; };   // a CU of a class: its index and position
+
 constexpr int LAT_THREADS = 256;
 constexpr int LAT_BUDGET = 48 * 1024;   // default dynamic shared bytes per CTA (4 CTAs per SM with the static part)
 constexpr int LAT_MAX_QP = 4;
 constexpr int LAT_SMEM_MAX = 96 * 1024;   // dynamic shared memory admitted by the kernel attribute
 constexpr int LAT_MAX_G = 8;            // CUs per CTA
-constexpr int LAT_MAX_JOBS = 144;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
+constexpr int LAT_MAX_JOBS = 136;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
 constexpr int LAT_NB = 592;             // neighbour buffer per CU (INTRA_NEIB_SIZE + pad)
 constexpr int LAT_SHAPES = 25;          // log2 sides 2..6
 
@@ -102,24 +104,26 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     // matrix rows are read one per lane: strides of an odd number of words
     L.fw_ws = L.w / 4 + 1; L.fh_ws = L.h / 4 + 1; L.fht_ws = L.kh / 4 + 1; L.fwt_ws = L.kw / 4 + 1;
     int o = 0;
-    L.o_fw = o; o += lat_up16(L.kw * L.fw_ws * 4);
-    L.o_fh = o; o += lat_up16(L.kh * L.fh_ws * 4);
-    L.o_fht = o; o += lat_up16(L.h * L.fht_ws * 4);
-    L.o_fwt = o; o += lat_up16(L.w * L.fwt_ws * 4);
-    L.o_scan = o; o += lat_up16(L.kw * L.kh * 2);
+    // without a QP (SATD records only) a tile has neither tables nor transform buffers
+    const int tr = n_qp > 0 ? 1 : 0;
+    L.o_fw = o; o += tr * lat_up16(L.kw * L.fw_ws * 4);
+    L.o_fh = o; o += tr * lat_up16(L.kh * L.fh_ws * 4);
+    L.o_fht = o; o += tr * lat_up16(L.h / 2 * L.fht_ws * 4);
+    L.o_fwt = o; o += tr * lat_up16(L.w / 2 * L.fwt_ws * 4);
+    L.o_scan = o; o += tr * lat_up16(L.kw * L.kh * 2);
     int c = 0;
     L.c_org = c; c += lat_up16(L.h * L.ps);
     L.c_nb = c; c += lat_up16(LAT_NB);
-    L.c_torg = c; c += lat_up16(L.kw * L.h * 4);
+    L.c_torg = c; c += tr * lat_up16(L.kw * L.h * 4);
     L.cu_bytes = c;
     int j = 0;
     L.j_pred = j; j += lat_up16(L.h * L.ps);
     const int b_t = lat_up16(L.kw * L.ts * 2), b_t2 = lat_up16(L.h * L.t2s * 2);
-    L.j_t = j; j += n_qp > 1 && b_t2 > b_t ? b_t2 : b_t;
-    L.j_c = j; j += lat_up16(L.kh * L.cs * 2);
-    L.j_dqt = j; j += lat_up16(L.kw * L.ds * 2);
+    L.j_t = j; j += tr * (n_qp > 1 && b_t2 > b_t ? b_t2 : b_t);
+    L.j_c = j; j += tr * lat_up16(L.kh * L.cs * 2);
+    L.j_dqt = j; j += tr * lat_up16(L.kw * L.ds * 2);
     L.j_dqt_b = j; if (n_qp > 1) j += lat_up16(L.kw * L.ds * 2);
-    L.j_t2 = j; j += b_t2;
+    L.j_t2 = j; j += tr * b_t2;
     L.job_bytes = j;
     const int avail = budget - o;
     // several whole CUs when nm jobs of the shape fit, else one CU and a chunk of its modes
@@ -145,12 +149,10 @@ struct LatParams {
     int org_words;            // org and i_org are multiples of 4: org blocks are read by words
     const pel *rec; int i_rec;
     int W, H;
-    const LatCu *cus;
     int ipf, n_qp, is_intra;
     int qp[LAT_MAX_QP];
     u32 *satd_out; LatQ *q_out;
-    const s8 *fold[7];        // folded DCT2 matrices per log2 size
-    const u16 *scanpos[7][7]; // raster -> scan index per (log2 w, log2 h)
+    const u8 *images;         // [class][LAT_IMAGE_BYTES] transform and scan tables (lat_image_fill)
     const u32 *ipred;         // the prediction table (lat_table_at)
     const u8 *modes;          // [CU][n_modes] modes to evaluate, or null for all 33 in order
     int n_modes;
@@ -161,14 +163,14 @@ struct LatParams {
     const int *counts;        // [LAT_SHAPES] CUs per shape class
     const int *cu_off;        // [LAT_SHAPES] first entry of each class in perm
     const int *tile_off;      // [LAT_SHAPES + 1] first tile of the class of each launch rank; [25] = total
-    const int *perm;          // CU indices grouped by class
+    const LatPerm *perm;      // the CUs grouped by class
     int *next;                // the next tile to take
 };
 
 // per-CTA shared scalars of a tile (the static part of the tile's shared memory)
 struct LatShared {
     IpredBlock B[LAT_MAX_G];
-    int cu[LAT_MAX_G];
+    LatPerm cu[LAT_MAX_G];
     u8 mode[LAT_MAX_JOBS];
     u32 satd[LAT_MAX_JOBS], ssd0[LAT_MAX_JOBS];   // ssd0: of the prediction, for QPs that code nothing
     // byte 0: bit q = QP q codes the job; byte 1 + b: the k-th job that QP b of the pair codes
@@ -176,6 +178,8 @@ struct LatShared {
     u32 nz[2][LAT_MAX_JOBS], sum[2][LAT_MAX_JOBS], hash[2][LAT_MAX_JOBS], ssd[2][LAT_MAX_JOBS];   // per QP of the pair
     int last[2][LAT_MAX_JOBS];
     int coded[2];   // jobs that each QP of the pair codes
+    int tile_off[LAT_SHAPES + 1], cu_off[LAT_SHAPES], counts[LAT_SHAPES];   // of the queue (LatParams)
+    int next[2], rank[2];           // the tile after this one and its launch rank, by the tile's parity
     int tables;   // shape class whose matrices and scan table are in place (-1: none)
 };
 
@@ -286,7 +290,8 @@ __device__ __forceinline__ u32 lat_sq4(u32 a, u32 b, u32 c)
 // differences of the prediction, which every QP that codes no level of the job keeps, is added to
 // s_ssd0[j] too.
 template <int TW, int TH, bool SSD>
-__device__ __forceinline__ void lat_satd_tiles(int n_tiles, int lnt, int ntx, const u8 *cub, int cu_bytes, int c_org,
+__device__ __forceinline__ void lat_satd_tiles(int n_tiles, int lnt, int ntx,
+                                               const u8 *cub, int cu_bytes, int c_org,
                                                const u8 *jobb, int job_bytes, int j_pred, int ps, u32 mc_magic,
                                                u32 *s_satd, u32 *s_ssd0, double sq32, double sq128, u64 k32,
                                                u64 k128)
@@ -471,15 +476,43 @@ __device__ unsigned long long g_lat_stage_clk[LAT_SHAPES][LAT_STAGES];
 #define LAT_STAGE(k) do { } while (0)
 #endif
 
+__device__ __forceinline__ LatPerm lat_perm(const LatPerm *p)
+{
+    const int2 v = __ldg(reinterpret_cast<const int2 *>(p));
+    return { v.x, (s16)(v.y & 0xFFFF), (s16)(v.y >> 16) };
+}
+
+// entry i of a class's table image: fold_w / fold_h are the folded DCT2 matrices, scanpos the scan order
+constexpr int LAT_IMAGE_BYTES = 9 * 1024;   // the largest: 8704 (64x64)
+static __device__ void lat_image_fill(const s8 *fold_w, const s8 *fold_h, const u16 *scanpos, int lw, int lh, u8 *img)
+{
+    LatLayout L;
+    lat_layout(lw, lh, 1, 1, LAT_BUDGET, L);
+    const int w = L.w, h = L.h, kw = L.kw, kh = L.kh;
+    for (int i = threadIdx.x; i < kw * w; i += blockDim.x) {
+        const int u = i >> lw, x = i & (w - 1);
+        const u8 v = (u8)fold_w[u * w + x];
+        img[L.o_fw + u * L.fw_ws * 4 + x] = v;        // Fw[u][x]
+        if (x < (w >> 1)) img[L.o_fwt + x * L.fwt_ws * 4 + lat_eo(u, kw)] = v;
+    }
+    for (int i = threadIdx.x; i < kh * h; i += blockDim.x) {
+        const int v = i >> lh, y = i & (h - 1);
+        const u8 c = (u8)fold_h[v * h + y];
+        img[L.o_fh + v * L.fh_ws * 4 + y] = c;        // Fh[v][y]
+        if (y < (h >> 1)) img[L.o_fht + y * L.fht_ws * 4 + lat_eo(v, kh)] = c;
+    }
+    for (int i = threadIdx.x; i < kw * kh; i += blockDim.x)
+        ((u16 *)(img + L.o_scan))[i] = scanpos[(i >> L.lkw) * w + (i & (kw - 1))];
+}
+
 // One tile of shape class (LW, LH): a few whole CUs, or one CU and a chunk of its modes, as the
 // class's layout says.  Called by every thread of the CTA; the tile's data lives in `sm` (the
 // layout's dynamic shared memory) and `S`.
 template <int LW, int LH>
-__device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, int n_shape, int tile, u8 *sm,
+__device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm, int n_shape, int tile, u8 *sm,
                                          LatShared &S)
 {
     IpredBlock *sB = S.B;
-    int *s_cu = S.cu;
     u8 *s_mode = S.mode;
     u32 *s_satd = S.satd, *s_flag = S.flag;
 
@@ -487,7 +520,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     LAT_STAGE_BEGIN();
     // compile-time shape: the indices and trip counts below are constants
     lat_layout(LW, LH, P.n_modes, P.n_qp, P.budget[(LW - 2) * 5 + (LH - 2)], L);
-    const int w = L.w, h = L.h, lw = L.lw, lh = L.lh, kw = L.kw, kh = L.kh, lkw = L.lkw;
+    const int w = L.w, h = L.h, lw = L.lw, lh = L.lh, kw = L.kw, lkw = L.lkw;
     const int N = w * h, lN = lw + lh;
     constexpr int W_ = 1 << LW, H_ = 1 << LH, KW_ = W_ < 32 ? W_ : 32, KH_ = H_ < 32 ? H_ : 32;
     constexpr int LKW_ = LW < 5 ? LW : 5, LKH_ = LH < 5 ? LH : 5;
@@ -510,8 +543,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     // j * MCv < 2^16 (here j < 8 * 33 and MCv <= 33)
     const u32 mc_magic = (65536u + (u32)MCv - 1u) / (u32)MCv;
 
-    u32 *fw = (u32 *)(sm + L.o_fw), *fh = (u32 *)(sm + L.o_fh);
-    u32 *fht = (u32 *)(sm + L.o_fht), *fwt = (u32 *)(sm + L.o_fwt);
+    const u32 *fw = (const u32 *)(sm + L.o_fw), *fh = (const u32 *)(sm + L.o_fh);
+    const u32 *fht = (const u32 *)(sm + L.o_fht), *fwt = (const u32 *)(sm + L.o_fwt);
     u8 *cub = sm + L.o_cu, *jobb = sm + L.o_job;
 
     // job j -> (CU g, mode m): j = g * MCv + (m - m0)
@@ -530,42 +563,30 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     // n they keep column n with the even-k entries first and the odd-k entries after them
     // (Fw^T, Fh^T in even/odd order), and each sum over k splits into an even part E and an odd
     // part O with out[n] = E + O and out[N-1-n] = E - O.
-    // A CTA takes its tiles from the queue in class order, so consecutive tiles mostly share
-    // the class: the tables of the previous tile are kept (the layout of a class is fixed
-    // within a launch).
-    const int cls = (LW - 2) * 5 + (LH - 2);
-    const bool tables_in_place = S.tables == cls;
-    for (int i = tid; i < (tables_in_place ? 0 : kw * w); i += LAT_THREADS) {
-        const int u = i >> lw, x = i & (w - 1);
-        const u8 v = (u8)P.fold[LW][u * w + x];
-        ((u8 *)fw)[u * L.fw_ws * 4 + x] = v;        // Fw[u][x]
-        if (x < (w >> 1)) ((u8 *)fwt)[x * L.fwt_ws * 4 + lat_eo(u, kw)] = v;
+    // The class's tables come as an image of this part of shared memory, built once per device.  A CTA
+    // takes its tiles from the queue in class order, so consecutive tiles mostly share the class: the
+    // tables of the previous tile are kept (the layout of a class is fixed within a launch).
+    constexpr int cls = (LW - 2) * 5 + (LH - 2);
+    if (P.n_qp > 0 && S.tables != cls) {
+        const uint4 *img = reinterpret_cast<const uint4 *>(P.images + cls * LAT_IMAGE_BYTES);
+        for (int i = tid; i < L.o_cu / 16; i += LAT_THREADS) reinterpret_cast<uint4 *>(sm)[i] = __ldg(img + i);
     }
-    for (int i = tid; i < (tables_in_place ? 0 : kh * h); i += LAT_THREADS) {
-        const int v = i >> lh, y = i & (h - 1);
-        const u8 c = (u8)P.fold[LH][v * h + y];
-        ((u8 *)fh)[v * L.fh_ws * 4 + y] = c;        // Fh[v][y]
-        if (y < (h >> 1)) ((u8 *)fht)[y * L.fht_ws * 4 + lat_eo(v, kh)] = c;
-    }
-    u16 *s_scan = (u16 *)(sm + L.o_scan);
-    for (int i = tid; i < (tables_in_place ? 0 : kw * kh); i += LAT_THREADS)
-        s_scan[i] = P.scanpos[LW][LH][(i >> lkw) * w + (i & (kw - 1))];
-    if (tid < Gv) s_cu[tid] = perm[cu0 + tid];
+    const u16 *s_scan = (const u16 *)(sm + L.o_scan);
+    if (tid < Gv) S.cu[tid] = lat_perm(perm + cu0 + tid);
     for (int j = tid; j < J; j += LAT_THREADS) {
-        const int g = j / MCv, mi = m0 + (j - g * MCv);
-        s_mode[j] = P.modes ? P.modes[(size_t)perm[cu0 + g] * P.n_modes + mi] : (u8)mi;
+        const int g = JG(j), mi = m0 + (j - g * MCv);
+        s_mode[j] = P.modes ? P.modes[(size_t)lat_perm(perm + cu0 + g).id * P.n_modes + mi] : (u8)mi;
         s_satd[j] = 0; s_flag[j] = 0; S.ssd0[j] = 0;
     }
-    __syncthreads(); LAT_STAGE(0);
-    if (tid == 0) S.tables = cls;   // every thread has read S.tables above
+    LAT_STAGE(0);
 
     // ---- per CU: org block, neighbours (com_intra_get_nbr with every in-picture sample
-    // reconstructed)
+    // reconstructed).  Each thread reads its CU's position itself: no wait between that and the samples.
     // four samples per thread (CU x positions are multiples of 4): one word load where the
     // picture and its pitch are word-aligned
     for (int i = tid; i < Gv * (N >> 2); i += LAT_THREADS) {
         const int g = i >> (lN - 2), p = (i & ((N >> 2) - 1)) << 2;
-        const LatCu cu = P.cus[s_cu[g]];
+        const LatPerm cu = lat_perm(perm + cu0 + g);
         const pel *src = P.org + (long long)(cu.y + (p >> lw)) * P.i_org + cu.x + (p & (w - 1));
         u32 v;
         if (P.org_words) v = __ldg(reinterpret_cast<const u32 *>(src));
@@ -575,7 +596,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     const int range = max(w, h) * 4 + 4;
     for (int i = tid; i < Gv * range; i += LAT_THREADS) {
         const int g = i / range, k = i - g * range;
-        const LatCu cu = P.cus[s_cu[g]];
+        const LatPerm cu = lat_perm(perm + cu0 + g);
         const int x = cu.x, y = cu.y;
         const int avail = (y > 0 ? 1 : 0) | (x > 0 ? 2 : 0);
         const int up_cnt = (y > 0) ? min(w >> 2, max(0, (P.W - (x + w)) >> 2)) : 0;
@@ -593,12 +614,30 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         }
     }
     __syncthreads(); LAT_STAGE(1);
-    if (tid < Gv) {
-        const LatCu cu = P.cus[s_cu[tid]];
+    if (tid == 0 && P.n_qp > 0) S.tables = cls;   // every thread has read S.tables above
+    if ((tid >> 5) < Gv) {
+        // a warp per CU: the sums that the DC and plane modes take from the neighbours
+        const int g = tid >> 5;
+        const LatPerm cu = S.cu[g];
         const int avail = (cu.y > 0 ? 1 : 0) | (cu.x > 0 ? 2 : 0) | ((cu.x > 0 && cu.y > 0) ? 4 : 0);
-        pel *nbm = cub + tid * L.cu_bytes + L.c_nb + 288;
-        ipred_block_setup(nbm, w, h, avail, 8, sB[tid]);
-        nbm[LAT_DC] = (pel)sB[tid].dc;
+        pel *nbm = cub + g * L.cu_bytes + L.c_nb + 288;
+        int up = 0, left = 0, ch = 0, cv = 0;
+#pragma unroll
+        for (int k = lane; k < w; k += 32) {
+            up += nbm[k + 1];
+            if (k < w / 2) ch += (k + 1) * (nbm[w / 2 + k + 1] - nbm[w / 2 - k - 1]);
+        }
+#pragma unroll
+        for (int k = lane; k < h; k += 32) {
+            left += nbm[-k - 1];
+            if (k < h / 2) cv += (k + 1) * (nbm[-h / 2 - k - 1] - nbm[-h / 2 + k + 1]);
+        }
+        up = __reduce_add_sync(0xFFFFFFFFu, up); left = __reduce_add_sync(0xFFFFFFFFu, left);
+        ch = __reduce_add_sync(0xFFFFFFFFu, ch); cv = __reduce_add_sync(0xFFFFFFFFu, cv);
+        if (lane == 0) {
+            ipred_block_finish(nbm, w, h, avail, 8, up, left, ch, cv, sB[g]);
+            nbm[LAT_DC] = (pel)sB[g].dc;
+        }
     }
     // org part of the forward row pass: Torg[y][u] = sum_x Fw[u][x] org[y][x] (no transform
     // stage runs when no QP is asked: SATD records only)
@@ -703,7 +742,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
     }
     __syncthreads(); LAT_STAGE(5);
     for (int j = tid; j < J; j += LAT_THREADS)
-        P.satd_out[(size_t)s_cu[JG(j)] * 33 + s_mode[j]] = s_satd[j];
+        P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
 
     // two QPs at a time: they share the reads of the coefficients, and half the CTA barriers are left
     for (int q0 = 0; q0 < P.n_qp; q0 += 2) {
@@ -719,7 +758,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         }
         // the lists of the jobs each QP codes: quant_check found a coefficient above its threshold, whose
         // level is then not zero; the others keep the prediction's SSD and empty statistics
-        if (tid < 2) S.coded[tid] = 0;
+        int *coded = S.coded;
+        if (tid < 2) coded[tid] = 0;
         for (int j = tid; j < nb * J; j += LAT_THREADS) {
             const int b = j >= J ? 1 : 0, jj = j - b * J;
             S.nz[b][jj] = 0; S.sum[b][jj] = 0; S.hash[b][jj] = 0; S.last[b][jj] = -1; S.ssd[b][jj] = 0;
@@ -727,15 +767,15 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         __syncthreads();
         for (int base = wbase; base < nb * J; base += LAT_THREADS) {
             const int j = base + lane, b = j >= J ? 1 : 0, jj = j - b * J;
-            const bool coded = j < nb * J && ((s_flag[jj] >> (q0 + b)) & 1);
+            const bool own = j < nb * J && ((s_flag[jj] >> (q0 + b)) & 1);
             // a warp may hold jobs of both QPs: one ballot each
 #pragma unroll
             for (int c = 0; c < 2; c++) {
-                const u32 m = __ballot_sync(0xFFFFFFFFu, coded && b == c);
+                const u32 m = __ballot_sync(0xFFFFFFFFu, own && b == c);
                 int at = 0;
-                if (lane == 0 && m) at = atomicAdd(&S.coded[c], __popc(m));
+                if (lane == 0 && m) at = atomicAdd(&coded[c], __popc(m));
                 at = __shfl_sync(0xFFFFFFFFu, at, 0);
-                if (coded && b == c) ((u8 *)s_flag)[4 * (at + __popc(m & ((1u << lane) - 1))) + 1 + c] = (u8)jj;
+                if (own && b == c) ((u8 *)s_flag)[4 * (at + __popc(m & ((1u << lane) - 1))) + 1 + c] = (u8)jj;
             }
         }
         // first-pass levels, statistics, dequantisation (stored transposed, DQ^T[u][v], each row
@@ -795,7 +835,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         }
         __syncthreads(); LAT_STAGE(6);
         // the inverse passes run over the coded (job, QP) pairs only
-        const int n0 = S.coded[0], JC2 = n0 + S.coded[1];
+        const int n0 = coded[0], JC2 = n0 + coded[1];
         // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5); a task forms
         // rows y and H-1-y from the even-v and odd-v
         // sums over CU columns u (T2 rows are stored in even/odd order of u).  Tiles with few
@@ -870,14 +910,14 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const int *perm, in
         __syncthreads(); LAT_STAGE(8);
         for (int i = tid; i < nb * J; i += LAT_THREADS) {
             const int j = nb == 2 ? i >> 1 : i, b = nb == 2 ? i & 1 : 0, g = JG(j);
-            const bool coded = (s_flag[j] >> (q0 + b)) & 1;
+            const bool own = (s_flag[j] >> (q0 + b)) & 1;
             LatQ o;
-            o.ssd = coded ? S.ssd[b][j] : S.ssd0[j];
+            o.ssd = own ? S.ssd[b][j] : S.ssd0[j];
             o.coef_hash = S.hash[b][j];
             o.num_nz = (u16)S.nz[b][j];
             o.last_nz = (s16)S.last[b][j];
             o.sum_abs = S.sum[b][j];
-            P.q_out[((size_t)s_cu[g] * 33 + s_mode[j]) * P.n_qp + q0 + b] = o;
+            P.q_out[((size_t)S.cu[g].id * 33 + s_mode[j]) * P.n_qp + q0 + b] = o;
         }
         __syncthreads(); LAT_STAGE(9);
     }

@@ -104,19 +104,17 @@ const DevTables *device_tables(int dev)
     if (g_tab_ok[dev]) return &g_tab[dev];
     const HostTables &h = host_tables();
     void *buf = nullptr;
-    u32 *ipred = nullptr;
-    if (lattice_pred_table(&ipred) != UC_OK) return nullptr;
     if (cudaMalloc(&buf, sizeof(HostTables)) != cudaSuccess) return nullptr;
     if (cudaMemcpy(buf, &h, sizeof(HostTables), cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
     const HostTables *d = (const HostTables *)buf;
     DevTables &t = g_tab[dev];
-    t.ipred = ipred;
     for (int L = 0; L <= 6; L++) {
         t.fold[L] = &d->fold[L][0];
         t.d87[0][L] = &d->d87[0][L][0];
         t.d87[1][L] = &d->d87[1][L][0];
         for (int M = 0; M <= 6; M++) { t.scanpos[L][M] = &d->scanpos[L][M][0]; t.scan[L][M] = &d->scan[L][M][0]; }
     }
+    if (lattice_tables(t) != UC_OK) return nullptr;
     g_tab_ok[dev] = true;
     return &t;
 }

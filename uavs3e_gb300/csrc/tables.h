@@ -19,10 +19,11 @@ struct DevTables {
     const s16 *d87[2][7];
     const u16 *scan[7][7];
     const u16 *scanpos[7][7];
-    const u32 *ipred;           // the lattice's prediction table
+    const u32 *lat_ipred;       // the lattice's prediction table and its tiles' table images
+    const u8 *lat_images;
 };
 
-int lattice_pred_table(u32 **tab);          // allocates and fills it on the current device
+int lattice_tables(DevTables &t);           // allocates and fills lat_ipred and lat_images on the current device
 const HostTables &host_tables();
 const DevTables *device_tables(int dev);   // uploads on first use; nullptr on failure
 
