@@ -61,7 +61,7 @@ constexpr int LAT_BUDGET = 48 * 1024;   // default dynamic shared bytes per CTA 
 constexpr int LAT_MAX_QP = 4;
 constexpr int LAT_SMEM_MAX = 96 * 1024;   // dynamic shared memory admitted by the kernel attribute
 constexpr int LAT_MAX_G = 8;            // CUs per CTA
-constexpr int LAT_MAX_JOBS = 136;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
+constexpr int LAT_MAX_JOBS = 132;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
 constexpr int LAT_NB = 592;             // neighbour buffer per CU (INTRA_NEIB_SIZE + pad)
 constexpr int LAT_SHAPES = 25;          // log2 sides 2..6
 
@@ -98,7 +98,7 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     // strides also keep the rows 8 lanes read at once on distinct banks
     L.ps = L.w <= 8 ? 16 : L.w <= 32 ? 48 : 80;
     L.ts = L.h >= 8 ? L.h + 8 : 8;
-    L.cs = L.kw + 2;
+    L.cs = L.kw >= 8 ? L.kw + 8 : 8;
     L.ds = L.kh >= 8 ? L.kh + 8 : 8;
     L.t2s = L.kw >= 8 ? L.kw + 8 : 8;
     // matrix rows are read one per lane: strides of an odd number of words
@@ -124,7 +124,9 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     L.j_dqt = j; j += tr * lat_up16(L.kw * L.ds * 2);
     L.j_dqt_b = j; if (n_qp > 1) j += lat_up16(L.kw * L.ds * 2);
     L.j_t2 = j; j += tr * b_t2;
-    L.job_bytes = j;
+    // an odd multiple of 16 bytes: where a warp holds several jobs, their rows lie on different banks
+    // (at a multiple of 128 the quantisation of 4x4 blocks took twice the time)
+    L.job_bytes = j | 16;
     const int avail = budget - o;
     // several whole CUs when nm jobs of the shape fit, else one CU and a chunk of its modes
     int G = avail / (nm * L.job_bytes + L.cu_bytes);
@@ -225,21 +227,64 @@ __device__ __forceinline__ void lat_row(const void *p, u32 (&r)[NW])
     }
 }
 
-// position of index k in a row of n entries stored in even/odd order (the even k first)
-__host__ __device__ __forceinline__ constexpr int lat_eo(int k, int n) { return (k & 1) ? (n >> 1) + (k >> 1) : (k >> 1); }
+// position of index k in a row of n entries stored for the even/odd sums: chunks of eight entries (or
+// the row of four), in each the even k first and the odd k after them
+__host__ __device__ __forceinline__ constexpr int lat_eo(int k, int n)
+{
+    return n == 4 ? (k & 1) * 2 + (k >> 1) : (k & ~7) + (k & 1) * 4 + ((k & 7) >> 1);
+}
 
-// the even part E and the odd part O of sum_k F[k] D[k] over N entries, D as s16 pairs and F as
-// bytes, both in even/odd order (D: N/2 words, F: N/4 words)
-template <int N>
-__device__ __forceinline__ void lat_eo_sums(const u32 (&d)[N / 2], const u32 (&f)[N / 4], int &e, int &o)
+// the even parts e[r] and the odd parts o[r] of sum_k F[k] D_r[k] over the first 8 nch of N entries of R rows
+// D_r (s16, `pitch` apart) and the row F (bytes at f), both in lat_eo order.  The loop over the chunks is
+// not unrolled: the code stays small, and rows that end in zeros cost what they hold.
+template <int N, int R>
+__device__ __forceinline__ void lat_eo_sums(const s16 *d, int pitch, const u32 *f, int nch, int (&e)[R], int (&o)[R])
 {
 #pragma unroll
-    for (int p = 0; p < N / 4; p++) {
-        constexpr int H = N / 2;
-        const int be = 2 * p, bo = H + 2 * p;   // byte of the pair's first entry in F
-        e = ((be >> 1) & 1) ? dp2a_hi(d[p], f[be >> 2], e) : dp2a_lo(d[p], f[be >> 2], e);
-        o = ((bo >> 1) & 1) ? dp2a_hi(d[N / 4 + p], f[bo >> 2], o) : dp2a_lo(d[N / 4 + p], f[bo >> 2], o);
+    for (int r = 0; r < R; r++) e[r] = o[r] = 0;
+    if constexpr (N == 4) {
+        const u32 fw = f[0];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const uint2 v = *reinterpret_cast<const uint2 *>(d + r * pitch);
+            e[r] = dp2a_lo(v.x, fw, 0); o[r] = dp2a_hi(v.y, fw, 0);
+        }
+    } else {
+#pragma unroll 1
+        for (int c = 0; c < nch; c++, d += 8, f += 2) {
+            const u32 fe = f[0], fo = f[1];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(d + r * pitch);
+                e[r] = dp2a_hi(v.y, fe, dp2a_lo(v.x, fe, e[r]));
+                o[r] = dp2a_hi(v.w, fo, dp2a_lo(v.z, fo, o[r]));
+            }
+        }
     }
+}
+
+// two values clipped to s16 and packed, lo in the low half
+__device__ __forceinline__ u32 lat_pack16(int lo, int hi)
+{
+    u32 d;
+    asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(d) : "r"(hi), "r"(lo));
+    return d;
+}
+// four values clipped to 0..255 and packed, a in the lowest byte
+__device__ __forceinline__ u32 lat_pack8(int a, int b, int c, int d)
+{
+    u32 t;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(d), "r"(c), "r"(0));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(b), "r"(a), "r"(t));
+    return t;
+}
+
+// stores NW words of a row (aligned to its size)
+template <int NW>
+__device__ __forceinline__ void lat_store(void *p, const u32 (&v)[NW])
+{
+    if constexpr (NW == 4) *reinterpret_cast<uint4 *>(p) = make_uint4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<uint2 *>(p) = make_uint2(v[0], v[1]);
 }
 
 // sum over aligned groups of SEG lanes (SEG a power of two <= 32)
@@ -677,21 +722,31 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         const int sh1 = lw - 2, rnd1 = sh1 > 0 ? 1 << (sh1 - 1) : 0;
         for (int i = tid; i < (P.n_qp > 0 ? J * NYC * KW_ : 0); i += LAT_THREADS) {
             const int u = i & (KW_ - 1), yc = (i >> LKW_) % NYC, j = i / (KW_ * NYC);
-            u32 f[W_ / 4];
+            const int *torg = (const int *)(cub + JG(j) * L.cu_bytes + L.c_torg) + yc * RY * KW_ + u;
+            const u8 *pr = JPRED(j) + yc * RY * L.ps;
+            constexpr int XW = W_ < 16 ? W_ / 4 : 4;     // words of a row at a time
+            int acc[RY];
 #pragma unroll
-            for (int k = 0; k < W_ / 4; k++) f[k] = fw[u * L.fw_ws + k];
-            const int *torg = (const int *)(cub + JG(j) * L.cu_bytes + L.c_torg);
-            s16 *T = JT(j);
+            for (int r = 0; r < RY; r++) acc[r] = 0;
+#pragma unroll 1
+            for (int x = 0; x < W_ / 4; x += XW) {
+                u32 f[XW];
 #pragma unroll
-            for (int r = 0; r < RY; r++) {
-                const int y = yc * RY + r;
-                u32 pw[W_ / 4];
-                lat_row<W_ / 4>(JPRED(j) + y * L.ps, pw);
-                int sacc = 0;
+                for (int k = 0; k < XW; k++) f[k] = fw[u * L.fw_ws + x + k];
 #pragma unroll
-                for (int k = 0; k < W_ / 4; k++) sacc = dp4a_us(pw[k], f[k], sacc);
-                T[u * L.ts + y] = (s16)((torg[y * KW_ + u] - sacc + rnd1) >> sh1);
+                for (int r = 0; r < RY; r++) {
+                    u32 pw[XW];
+                    lat_row<XW>(pr + r * L.ps + 4 * x, pw);
+#pragma unroll
+                    for (int k = 0; k < XW; k++) acc[r] = dp4a_us(pw[k], f[k], acc[r]);
+                }
             }
+            u32 tv[RY / 2];
+#pragma unroll
+            for (int r = 0; r < RY; r++) acc[r] = (torg[r * KW_] - acc[r] + rnd1) >> sh1;
+#pragma unroll
+            for (int r = 0; r < RY / 2; r++) tv[r] = __byte_perm((u32)acc[2 * r], (u32)acc[2 * r + 1], 0x5410);
+            lat_store<RY / 2>(JT(j) + u * L.ts + yc * RY, tv);
         }
     }
     __syncthreads(); LAT_STAGE(4);
@@ -715,28 +770,43 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         const int sh2 = lh + 5, rnd2 = 1 << (sh2 - 1);
         for (int i = tid; i < (P.n_qp > 0 ? J * NUC * KH_ : 0); i += LAT_THREADS) {
             const int v = i & (KH_ - 1), uc = (i >> LKH_) % NUC, j = i / (KH_ * NUC);
-            u32 f[H_ / 4];
+            const s16 *T = JT(j) + uc * RU * L.ts;
+            int acc[RU];
 #pragma unroll
-            for (int k = 0; k < H_ / 4; k++) f[k] = fh[v * L.fh_ws + k];
-            u32 fl = 0;
+            for (int r = 0; r < RU; r++) acc[r] = rnd2;
+            if constexpr (H_ == 4) {
+                const u32 f = fh[v * L.fh_ws];
+#pragma unroll
+                for (int r = 0; r < RU; r++) {
+                    const uint2 t = *reinterpret_cast<const uint2 *>(T + r * L.ts);
+                    acc[r] = dp2a_hi(t.y, f, dp2a_lo(t.x, f, acc[r]));
+                }
+            } else {
+#pragma unroll 1
+                for (int y = 0; y < H_; y += 8) {
+                    const u32 f0 = fh[v * L.fh_ws + y / 4], f1 = fh[v * L.fh_ws + y / 4 + 1];
+#pragma unroll
+                    for (int r = 0; r < RU; r++) {
+                        const uint4 t = *reinterpret_cast<const uint4 *>(T + r * L.ts + y);
+                        acc[r] = dp2a_hi(t.y, f0, dp2a_lo(t.x, f0, acc[r]));
+                        acc[r] = dp2a_hi(t.w, f1, dp2a_lo(t.z, f1, acc[r]));
+                    }
+                }
+            }
+            u32 cv[RU / 2];
+            int amax = 0;
 #pragma unroll
             for (int r = 0; r < RU; r++) {
-                const int u = uc * RU + r;
-                u32 tw[H_ / 2];
-                lat_row<H_ / 2>(JT(j) + u * L.ts, tw);
-                int acc = 0;
-#pragma unroll
-                for (int k = 0; k < H_ / 4; k++) {
-                    acc = dp2a_lo(tw[2 * k], f[k], acc);
-                    acc = dp2a_hi(tw[2 * k + 1], f[k], acc);
-                }
-                const int c = (acc + rnd2) >> sh2;
-                JC(j)[v * L.cs + u] = (s16)c;
-                const int a = c < 0 ? -(int)(s16)c : (int)(s16)c;
-#pragma unroll
-                for (int q = 0; q < LAT_MAX_QP; q++)
-                    if (q < P.n_qp && a > nz_thr[q]) fl |= 1u << q;
+                acc[r] = (int)(s16)(acc[r] >> sh2);
+                amax = max(amax, abs(acc[r]));
             }
+#pragma unroll
+            for (int r = 0; r < RU / 2; r++) cv[r] = __byte_perm((u32)acc[2 * r], (u32)acc[2 * r + 1], 0x5410);
+            lat_store<RU / 2>(JC(j) + v * L.cs + uc * RU, cv);
+            u32 fl = 0;
+#pragma unroll
+            for (int q = 0; q < LAT_MAX_QP; q++)
+                if (q < P.n_qp && amax > nz_thr[q]) fl |= 1u << q;
             if (fl) atomicOr(&s_flag[j], fl);
         }
     }
@@ -796,24 +866,27 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 const u32 fl = act ? s_flag[j] >> q0 : 0u;
                 const u32 wrow = (u32)(v * w + uc * RU) * 0x9E3779B1u + 0x7F4A7C15u;
                 u32 cp[RU / 2];
-                const u32 *cw = reinterpret_cast<const u32 *>(JC(j) + v * L.cs + uc * RU);
-#pragma unroll
-                for (int r = 0; r < RU / 2; r++) cp[r] = cw[r];
+                lat_row<RU / 2>(JC(j) + v * L.cs + uc * RU, cp);
 #pragma unroll 1
                 for (int b = 0; b < nb; b++) {
                     const u32 on = (fl >> b) & 1;
-                    if (!__any_sync(0xFFFFFFFFu, on)) continue;
                     const u32 qv = on ? b ? q_value[1] : q_value[0] : 0u;
-                    const int scale = b ? dq_scale[1] : dq_scale[0], shift = b ? dq_shift[1] : dq_shift[0];
-                    s16 *dqt = (b ? JDQTB(j) : JDQT(j)) + uc * RU * L.ds + lat_eo(v, KH_);
-                    u32 mask = 0, sa = 0, hs = 0;
+                    u32 lv[RU], mask = 0, sa = 0, hs = 0;
 #pragma unroll
                     for (int r = 0; r < RU; r++) {
                         const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
-                        const u32 l = ((u32)abs(c) * qv + qadd) >> q_bits;
-                        const int lev = c < 0 ? -(int)l : (int)l;
-                        mask += min(l, 1u) << r;
-                        sa += l;
+                        lv[r] = ((u32)abs(c) * qv + qadd) >> q_bits;
+                        sa += lv[r];
+                    }
+                    // rows and chunks of eight columns without a level are not stored: the inverse passes
+                    // do not read them (a chunk with a level is stored whole)
+                    if (!__any_sync(0xFFFFFFFFu, sa)) continue;
+                    const int scale = b ? dq_scale[1] : dq_scale[0], shift = b ? dq_shift[1] : dq_shift[0];
+                    s16 *dqt = (b ? JDQTB(j) : JDQT(j)) + uc * RU * L.ds + lat_eo(v, KH_);
+#pragma unroll
+                    for (int r = 0; r < RU; r++) {
+                        const int lev = ((r & 1 ? (int)cp[r >> 1] : (int)(cp[r >> 1] << 16)) < 0) ? -(int)lv[r] : (int)lv[r];
+                        mask += min(lv[r], 1u) << r;
                         hs += (u32)lev * (wrow + ((u32)r * 0x9E3779B1u + (r & 1)));
                         int d = (lev * scale + (1 << shift >> 1)) >> shift;
                         d = min(32767, max(-32768, d));
@@ -824,8 +897,20 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                     // along a row the scan index grows with the column
                     const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + 31 - __clz((int)mask)] : -1;
                     const int last = lat_seg_max<SEG>(own_last, lane);
+                    const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
                     if (act && (lane & (SEG - 1)) == 0 && nz) {
+                        // which chunks of columns and of rows hold levels (bits 16.. and 20..)
+                        u32 ch = 0;
+                        const u32 own = SEG == 32 ? rows : (rows >> lane) & ((1u << (SEG & 31)) - 1);
+#pragma unroll
+                        for (int k = 0; k < SEG / KH_; k++)
+                            if ((own >> (k * KH_ & 31)) & (KH_ == 32 ? 0xFFFFFFFFu : (1u << (KH_ & 31)) - 1)) ch |= 1u << (16 + (uc + k) % NUC);
+#pragma unroll
+                        for (int k = 0; k < SEG / 8; k++)
+                            if ((own >> (k * 8)) & 0xFFu) ch |= 1u << (20 + (KH_ < 8 ? 0 : k % (KH_ / 8 ? KH_ / 8 : 1)));
+                        if (KH_ < 8) ch |= 1u << 20;
                         atomicAdd(&S.nz[b][j], nz);
+                        atomicOr(&S.nz[b][j], ch);
                         atomicAdd(&S.sum[b][j], sa);
                         atomicAdd(&S.hash[b][j], hs);
                         atomicMax(&S.last[b][j], last);
@@ -837,38 +922,52 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         // the inverse passes run over the coded (job, QP) pairs only
         const int n0 = coded[0], JC2 = n0 + coded[1];
         // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5); a task forms
-        // rows y and H-1-y from the even-v and odd-v
-        // sums over CU columns u (T2 rows are stored in even/odd order of u).  Tiles with few
+        // rows y and H-1-y from the even-v and odd-v sums over CU columns u.  Chunks of columns past the
+        // last level's are left out, empty ones before it are zeros.  Tiles with few
         // jobs take CU/2 columns per task so that the CTA's threads still have a task each.
         auto inv_col = [&](auto cu_tag) {
             constexpr int CU = decltype(cu_tag)::value, NCU = KW_ / CU;
             for (int i = tid; i < JC2 * NCU * (H_ / 2); i += LAT_THREADS) {
                 const int y = i & (H_ / 2 - 1), uc = (i >> (LH - 1)) % NCU, k = i / ((H_ / 2) * NCU);
                 const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
-                const s16 *dqt = b ? JDQTB(j) : JDQT(j);
-                s16 *t2b = b ? JT(j) : JT2(j);
-                u32 f[KH_ / 4];
+                const u32 ch = S.nz[b][j] >> 16;
+                const int col = uc * CU >> 3;
+                if (KW_ > 8 && !((ch & 15) >> col)) continue;
+                int e[CU], o[CU];
+                const int nv = KW_ > 8 && !((ch >> col) & 1) ? 0 : KH_ > 8 ? 32 - __clz((int)((ch >> 4) & 15)) : 1;
+                if (KH_ == 4 && nv == 0) {
 #pragma unroll
-                for (int e = 0; e < KH_ / 4; e++) f[e] = fht[y * L.fht_ws + e];
-#pragma unroll 2   // two columns per step: a full unroll spills at the 64-register limit
-                for (int r = 0; r < CU; r++) {
-                    const int u = uc * CU + r;
-                    u32 dw[KH_ / 2];
-                    lat_row<KH_ / 2>(dqt + u * L.ds, dw);
-                    int e = 0, o = 0;
-                    lat_eo_sums<KH_>(dw, f, e, o);
-                    s16 *t2 = t2b + lat_eo(u, KW_);
-                    t2[y * L.t2s] = (s16)min(32767, max(-32768, (e + o + 16) >> 5));
-                    t2[(H_ - 1 - y) * L.t2s] = (s16)min(32767, max(-32768, (e - o + 16) >> 5));
+                    for (int r = 0; r < CU; r++) e[r] = o[r] = 0;
+                } else {
+                    lat_eo_sums<KH_, CU>((b ? JDQTB(j) : JDQT(j)) + uc * CU * L.ds, L.ds, fht + y * L.fht_ws, nv, e, o);
+                }
+                s16 *t2 = b ? JT(j) : JT2(j);
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+                    int t[CU];
+#pragma unroll
+                    for (int r = 0; r < CU; r++) t[r] = (half ? e[r] - o[r] + 16 : e[r] + o[r] + 16) >> 5;
+                    s16 *row = t2 + (half ? H_ - 1 - y : y) * L.t2s;
+                    if constexpr (CU == 8) {
+                        const u32 v[4] = { lat_pack16(t[0], t[2]), lat_pack16(t[4], t[6]), lat_pack16(t[1], t[3]), lat_pack16(t[5], t[7]) };
+                        lat_store<4>(row + uc * 8, v);
+                    } else if constexpr (KW_ == 4) {
+                        const u32 v[2] = { lat_pack16(t[0], t[2]), lat_pack16(t[1], t[3]) };
+                        lat_store<2>(row, v);
+                    } else {
+                        u32 *p = reinterpret_cast<u32 *>(row + (uc >> 1) * 8) + (uc & 1);
+                        p[0] = lat_pack16(t[0], t[2]); p[2] = lat_pack16(t[1], t[3]);
+                    }
                 }
             }
         };
-        if (RU > 2 && JC2 * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, (RU > 2 ? RU / 2 : RU)>{});
+        if (RU == 8 && JC2 * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, 4>{});
         else inv_col(std::integral_constant<int, RU>{});
         __syncthreads(); LAT_STAGE(7);
         // inverse row pass, reconstruction, SSD: a task is the column pair x, W-1-x over CY
         // rows (the even-u and odd-u sums of the T2 row give both); CY = RY / 2 for tiles with
-        // few jobs
+        // few jobs.  The clip of the residual to -256..255 is left out: the clip of the reconstruction
+        // gives the same sample without it.
         auto inv_row = [&](auto cy_tag) {
             constexpr int CY = decltype(cy_tag)::value, NCY = H_ / CY;
             constexpr int TPJ = (W_ / 2) * NCY, SEG = TPJ < 32 ? TPJ : 32;
@@ -878,27 +977,19 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 const int ii = act ? i : base;
                 const int x = ii & (W_ / 2 - 1), yc = (ii >> (LW - 1)) % NCY, k = ii / TPJ;
                 const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
-                const s16 *t2b = b ? JT(j) : JT2(j);
-                u32 f[KW_ / 4];
-#pragma unroll
-                for (int e = 0; e < KW_ / 4; e++) f[e] = fwt[x * L.fwt_ws + e];
-                const pel *po = CORG(JG(j));
-                const pel *pp = JPRED(j);
+                const int nu = KW_ > 8 ? 32 - __clz((int)((S.nz[b][j] >> 16) & 15)) : 1;
+                int se[CY], so[CY];
+                lat_eo_sums<KW_, CY>((b ? JT(j) : JT2(j)) + yc * CY * L.t2s, L.t2s, fwt + x * L.fwt_ws, nu, se, so);
+                const pel *po = CORG(JG(j)) + yc * CY * L.ps, *pp = JPRED(j) + yc * CY * L.ps;
                 u32 e = 0;
 #pragma unroll
-                for (int r = 0; r < CY; r++) {
-                    const int y = yc * CY + r;
-                    int rv0 = pp[y * L.ps + x], rv1 = pp[y * L.ps + W_ - 1 - x];
-                    u32 tw[KW_ / 2];
-                    lat_row<KW_ / 2>(t2b + y * L.t2s, tw);
-                    int se = 0, so = 0;
-                    lat_eo_sums<KW_>(tw, f, se, so);
-                    const int res0 = min(255, max(-256, (se + so + 2048) >> 12));
-                    const int res1 = min(255, max(-256, (se - so + 2048) >> 12));
-                    rv0 = min(255, max(0, rv0 + res0));
-                    rv1 = min(255, max(0, rv1 + res1));
-                    const int d0 = (int)po[y * L.ps + x] - rv0, d1 = (int)po[y * L.ps + W_ - 1 - x] - rv1;
-                    e += (u32)(d0 * d0) + (u32)(d1 * d1);
+                for (int r = 0; r < CY; r += 2) {
+                    const pel *p0 = pp + r * L.ps, *p1 = p0 + L.ps, *o0 = po + r * L.ps, *o1 = o0 + L.ps;
+                    const u32 rec = lat_pack8(p0[x] + ((se[r] + so[r] + 2048) >> 12), p0[W_ - 1 - x] + ((se[r] - so[r] + 2048) >> 12),
+                                              p1[x] + ((se[r + 1] + so[r + 1] + 2048) >> 12),
+                                              p1[W_ - 1 - x] + ((se[r + 1] - so[r + 1] + 2048) >> 12));
+                    const u32 org = (u32)o0[x] | (u32)o0[W_ - 1 - x] << 8 | (u32)o1[x] << 16 | (u32)o1[W_ - 1 - x] << 24;
+                    e = lat_sq4(org, rec, e);
                 }
                 if (!act) e = 0;
                 e = lat_seg_sum<SEG>(e, lane);
