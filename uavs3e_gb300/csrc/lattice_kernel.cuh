@@ -87,6 +87,10 @@ struct LatLayout {
 
 __host__ __device__ __forceinline__ int lat_up16(int v) { return (v + 15) & ~15; }
 
+// row stride for rows of n words (n = 2, 4, 8, 16) read 8 bytes per lane: n + 2 is twice an odd number but
+// for n = 2
+__host__ __device__ constexpr int lat_pair_stride(int n) { return n == 2 ? 6 : n + 2; }
+
 // the layout of a CTA for (2^lw) x (2^lh) CUs, nm modes and n_qp QPs within `budget` bytes of dynamic
 // shared memory: how many CUs (or which chunk of one CU's modes) a CTA takes
 __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int budget, LatLayout &L)
@@ -101,8 +105,12 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     L.cs = L.kw >= 8 ? L.kw + 8 : 8;
     L.ds = L.kh >= 8 ? L.kh + 8 : 8;
     L.t2s = L.kw >= 8 ? L.kw + 8 : 8;
-    // matrix rows are read one per lane: strides of an odd number of words
-    L.fw_ws = L.w / 4 + 1; L.fh_ws = L.h / 4 + 1; L.fht_ws = L.kh / 4 + 1; L.fwt_ws = L.kw / 4 + 1;
+    // matrix rows are read one per lane, a chunk in one load: 16 bytes of a forward row matrix, 8 of the
+    // others, at strides (in words) that keep those loads on distinct banks
+    L.fw_ws = L.w >= 32 ? L.w / 4 + 4 : L.w == 16 ? 12 : L.w == 8 ? 6 : 1;
+    L.fh_ws = L.h >= 8 ? lat_pair_stride(L.h / 4) : 1;
+    L.fht_ws = L.kh >= 8 ? lat_pair_stride(L.kh / 4) : 1;
+    L.fwt_ws = L.kw >= 8 ? lat_pair_stride(L.kw / 4) : 1;
     int o = 0;
     // without a QP (SATD records only) a tile has neither tables nor transform buffers
     const int tr = n_qp > 0 ? 1 : 0;
@@ -252,7 +260,8 @@ __device__ __forceinline__ void lat_eo_sums(const s16 *d, int pitch, const u32 *
     } else {
 #pragma unroll 1
         for (int c = 0; c < nch; c++, d += 8, f += 2) {
-            const u32 fe = f[0], fo = f[1];
+            const uint2 fv = *reinterpret_cast<const uint2 *>(f);
+            const u32 fe = fv.x, fo = fv.y;
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 const uint4 v = *reinterpret_cast<const uint4 *>(d + r * pitch);
@@ -528,7 +537,7 @@ __device__ __forceinline__ LatPerm lat_perm(const LatPerm *p)
 }
 
 // entry i of a class's table image: fold_w / fold_h are the folded DCT2 matrices, scanpos the scan order
-constexpr int LAT_IMAGE_BYTES = 9 * 1024;   // the largest: 8704 (64x64)
+constexpr int LAT_IMAGE_BYTES = 10 * 1024;   // the largest: 9472 (64x64)
 static __device__ void lat_image_fill(const s8 *fold_w, const s8 *fold_h, const u16 *scanpos, int lw, int lh, u8 *img)
 {
     LatLayout L;
@@ -731,8 +740,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
 #pragma unroll 1
             for (int x = 0; x < W_ / 4; x += XW) {
                 u32 f[XW];
-#pragma unroll
-                for (int k = 0; k < XW; k++) f[k] = fw[u * L.fw_ws + x + k];
+                lat_row<XW>(fw + u * L.fw_ws + x, f);
 #pragma unroll
                 for (int r = 0; r < RY; r++) {
                     u32 pw[XW];
@@ -784,7 +792,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
             } else {
 #pragma unroll 1
                 for (int y = 0; y < H_; y += 8) {
-                    const u32 f0 = fh[v * L.fh_ws + y / 4], f1 = fh[v * L.fh_ws + y / 4 + 1];
+                    const uint2 fv = *reinterpret_cast<const uint2 *>(fh + v * L.fh_ws + y / 4);
+                    const u32 f0 = fv.x, f1 = fv.y;
 #pragma unroll
                     for (int r = 0; r < RU; r++) {
                         const uint4 t = *reinterpret_cast<const uint4 *>(T + r * L.ts + y);
@@ -871,31 +880,57 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 for (int b = 0; b < nb; b++) {
                     const u32 on = (fl >> b) & 1;
                     const u32 qv = on ? b ? q_value[1] : q_value[0] : 0u;
-                    u32 lv[RU], mask = 0, sa = 0, hs = 0;
+                    // level of c: (|c| qv + 2^(q_bits - 1)) >> q_bits with c's sign, which is
+                    // (c qv + 2^(q_bits - 1) - (c < 0)) >> q_bits; two to a word (|c| <= 2^15, qv < 2^15 and
+                    // q_bits >= 15, so 16 bits hold one)
+                    int lv[RU];
+                    u32 lp[RU / 2], mask = 0;
 #pragma unroll
                     for (int r = 0; r < RU; r++) {
                         const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
-                        lv[r] = ((u32)abs(c) * qv + qadd) >> q_bits;
-                        sa += lv[r];
+                        lv[r] = (c * (int)qv + ((int)qadd + (c >> 31))) >> q_bits;
+                    }
+#pragma unroll
+                    for (int k = 0; k < RU / 2; k++) {
+                        lp[k] = __byte_perm((u32)lv[2 * k], (u32)lv[2 * k + 1], 0x5410);
+                        mask += __vminu2(lp[k], 0x00010001u) << k;   // bit k: column 2k, bit 16 + k: column 2k + 1
                     }
                     // rows and chunks of eight columns without a level are not stored: the inverse passes
                     // do not read them (a chunk with a level is stored whole)
-                    if (!__any_sync(0xFFFFFFFFu, sa)) continue;
+                    if (!__any_sync(0xFFFFFFFFu, mask != 0)) continue;
                     const int scale = b ? dq_scale[1] : dq_scale[0], shift = b ? dq_shift[1] : dq_shift[0];
                     s16 *dqt = (b ? JDQTB(j) : JDQT(j)) + uc * RU * L.ds + lat_eo(v, KH_);
+                    u32 sa = 0;
 #pragma unroll
-                    for (int r = 0; r < RU; r++) {
-                        const int lev = ((r & 1 ? (int)cp[r >> 1] : (int)(cp[r >> 1] << 16)) < 0) ? -(int)lv[r] : (int)lv[r];
-                        mask += min(lv[r], 1u) << r;
-                        hs += (u32)lev * (wrow + ((u32)r * 0x9E3779B1u + (r & 1)));
-                        int d = (lev * scale + (1 << shift >> 1)) >> shift;
-                        d = min(32767, max(-32768, d));
-                        if (act) dqt[r * L.ds] = (s16)(odd ? (d * 181 + 128) >> 8 : d);
+                    for (int r = 0; r < RU; r += 2) {
+                        sa += (u32)abs(lv[r]) + (u32)abs(lv[r + 1]);
+                        const int d0 = (lv[r] * scale + (1 << shift >> 1)) >> shift;
+                        const int d1 = (lv[r + 1] * scale + (1 << shift >> 1)) >> shift;
+                        u32 d = lat_pack16(d0, d1);
+                        if (odd) d = __byte_perm((u32)(((int)(s16)(d & 0xFFFF) * 181 + 128) >> 8), (u32)((((int)d >> 16) * 181 + 128) >> 8), 0x5410);
+                        if (act) {
+                            dqt[r * L.ds] = (s16)(d & 0xFFFF);
+                            dqt[(r + 1) * L.ds] = (s16)(d >> 16);
+                        }
                     }
-                    const u32 nz = lat_seg_sum<SEG>((u32)__popc(mask), lane);
-                    sa = lat_seg_sum<SEG>(sa, lane); hs = lat_seg_sum<SEG>(hs, lane);
+                    // sum of level x weight, the weight of column r being wrow + K r + (r & 1): from the
+                    // sums over the pairs k of s_k = lev[2k] + lev[2k+1], of k s_k, and of the odd columns
+                    int at = 0, ks = 0, odds = 0;
+#pragma unroll
+                    for (int k = RU / 2 - 1; k >= 0; k--) {
+                        at = dp2a_lo(lp[k], 0x0101u, at);
+                        if (k > 0) ks += at;
+                        odds = dp2a_lo(lp[k], 0x0100u, odds);
+                    }
+                    u32 hs = (u32)at * wrow + (u32)ks * (2u * 0x9E3779B1u) + (u32)odds * (0x9E3779B1u + 1u);
+                    // the count of levels rides above the sum of their magnitudes: of a segment's at most
+                    // 32 x 8 levels the sum is below 2^23
+                    const u32 both = lat_seg_sum<SEG>(sa | (u32)__popc(mask) << 23, lane);
+                    const u32 nz = both >> 23;
+                    sa = both & 0x7FFFFFu; hs = lat_seg_sum<SEG>(hs, lane);
                     // along a row the scan index grows with the column
-                    const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + 31 - __clz((int)mask)] : -1;
+                    const int he = 31 - __clz((int)(mask & 0xFFFFu)), ho = 31 - __clz((int)(mask >> 16));
+                    const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + max(2 * he, 2 * ho + 1)] : -1;
                     const int last = lat_seg_max<SEG>(own_last, lane);
                     const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
                     if (act && (lane & (SEG - 1)) == 0 && nz) {
@@ -964,31 +999,57 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         if (RU == 8 && JC2 * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, 4>{});
         else inv_col(std::integral_constant<int, RU>{});
         __syncthreads(); LAT_STAGE(7);
-        // inverse row pass, reconstruction, SSD: a task is the column pair x, W-1-x over CY
-        // rows (the even-u and odd-u sums of the T2 row give both); CY = RY / 2 for tiles with
+        // inverse row pass, reconstruction, SSD: a task is the columns x, x+1, W-2-x, W-1-x over CY
+        // rows (the even-u and odd-u sums of the T2 row give two of them); CY = 2 for tiles with
         // few jobs.  The clip of the residual to -256..255 is left out: the clip of the reconstruction
         // gives the same sample without it.
         auto inv_row = [&](auto cy_tag) {
             constexpr int CY = decltype(cy_tag)::value, NCY = H_ / CY;
-            constexpr int TPJ = (W_ / 2) * NCY, SEG = TPJ < 32 ? TPJ : 32;
+            constexpr int TPJ = (W_ / 4) * NCY, SEG = TPJ < 32 ? TPJ : 32;
             for (int base = wbase; base < JC2 * TPJ; base += LAT_THREADS) {
                 const int i = base + lane;
                 const bool act = i < JC2 * TPJ;
                 const int ii = act ? i : base;
-                const int x = ii & (W_ / 2 - 1), yc = (ii >> (LW - 1)) % NCY, k = ii / TPJ;
+                const int x = (ii & (W_ / 4 - 1)) * 2, yc = (ii >> (LW - 2)) % NCY, k = ii / TPJ;
                 const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
-                const int nu = KW_ > 8 ? 32 - __clz((int)((S.nz[b][j] >> 16) & 15)) : 1;
-                int se[CY], so[CY];
-                lat_eo_sums<KW_, CY>((b ? JT(j) : JT2(j)) + yc * CY * L.t2s, L.t2s, fwt + x * L.fwt_ws, nu, se, so);
+                const s16 *t2 = (b ? JT(j) : JT2(j)) + yc * CY * L.t2s;
+                const u32 *f = fwt + x * L.fwt_ws;
+                // e0, o0: column x (and W-1-x); e1, o1: column x+1 (and W-2-x)
+                int e0[CY], o0[CY], e1[CY], o1[CY];
+                if constexpr (KW_ == 4) {
+                    const u32 f0 = f[0], f1 = f[L.fwt_ws];
+#pragma unroll
+                    for (int r = 0; r < CY; r++) {
+                        const uint2 v = *reinterpret_cast<const uint2 *>(t2 + r * L.t2s);
+                        e0[r] = dp2a_lo(v.x, f0, 2048); o0[r] = dp2a_hi(v.y, f0, 0);
+                        e1[r] = dp2a_lo(v.x, f1, 2048); o1[r] = dp2a_hi(v.y, f1, 0);
+                    }
+                } else {
+#pragma unroll
+                    for (int r = 0; r < CY; r++) { e0[r] = e1[r] = 2048; o0[r] = o1[r] = 0; }
+                    const int nu = KW_ > 8 ? 32 - __clz((int)((S.nz[b][j] >> 16) & 15)) : 1;
+#pragma unroll 1
+                    for (int c = 0; c < nu; c++, t2 += 8, f += 2) {
+                        const uint2 f0 = *reinterpret_cast<const uint2 *>(f), f1 = *reinterpret_cast<const uint2 *>(f + L.fwt_ws);
+#pragma unroll
+                        for (int r = 0; r < CY; r++) {
+                            const uint4 v = *reinterpret_cast<const uint4 *>(t2 + r * L.t2s);
+                            e0[r] = dp2a_hi(v.y, f0.x, dp2a_lo(v.x, f0.x, e0[r]));
+                            o0[r] = dp2a_hi(v.w, f0.y, dp2a_lo(v.z, f0.y, o0[r]));
+                            e1[r] = dp2a_hi(v.y, f1.x, dp2a_lo(v.x, f1.x, e1[r]));
+                            o1[r] = dp2a_hi(v.w, f1.y, dp2a_lo(v.z, f1.y, o1[r]));
+                        }
+                    }
+                }
                 const pel *po = CORG(JG(j)) + yc * CY * L.ps, *pp = JPRED(j) + yc * CY * L.ps;
                 u32 e = 0;
 #pragma unroll
-                for (int r = 0; r < CY; r += 2) {
-                    const pel *p0 = pp + r * L.ps, *p1 = p0 + L.ps, *o0 = po + r * L.ps, *o1 = o0 + L.ps;
-                    const u32 rec = lat_pack8(p0[x] + ((se[r] + so[r] + 2048) >> 12), p0[W_ - 1 - x] + ((se[r] - so[r] + 2048) >> 12),
-                                              p1[x] + ((se[r + 1] + so[r + 1] + 2048) >> 12),
-                                              p1[W_ - 1 - x] + ((se[r + 1] - so[r + 1] + 2048) >> 12));
-                    const u32 org = (u32)o0[x] | (u32)o0[W_ - 1 - x] << 8 | (u32)o1[x] << 16 | (u32)o1[W_ - 1 - x] << 24;
+                for (int r = 0; r < CY; r++) {
+                    const auto pair = [](const pel *p) { return (u32)*reinterpret_cast<const u16 *>(p); };
+                    const u32 pl = pair(pp + r * L.ps + x), pr = pair(pp + r * L.ps + W_ - 2 - x);
+                    const u32 org = pair(po + r * L.ps + x) | pair(po + r * L.ps + W_ - 2 - x) << 16;
+                    const u32 rec = lat_pack8((int)(pl & 0xFF) + ((e0[r] + o0[r]) >> 12), (int)(pl >> 8) + ((e1[r] + o1[r]) >> 12),
+                                              (int)(pr & 0xFF) + ((e1[r] - o1[r]) >> 12), (int)(pr >> 8) + ((e0[r] - o0[r]) >> 12));
                     e = lat_sq4(org, rec, e);
                 }
                 if (!act) e = 0;
@@ -996,8 +1057,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 if (act && (lane & (SEG - 1)) == 0) atomicAdd(&S.ssd[b][j], e);
             }
         };
-        if (RY > 2 && JC2 * (W_ / 2) * NYC < LAT_THREADS) inv_row(std::integral_constant<int, (RY > 2 ? RY / 2 : RY)>{});
-        else inv_row(std::integral_constant<int, RY>{});
+        if (JC2 * (W_ / 4) * (H_ / 4) < LAT_THREADS) inv_row(std::integral_constant<int, 2>{});
+        else inv_row(std::integral_constant<int, 4>{});
         __syncthreads(); LAT_STAGE(8);
         for (int i = tid; i < nb * J; i += LAT_THREADS) {
             const int j = nb == 2 ? i >> 1 : i, b = nb == 2 ? i & 1 : 0, g = JG(j);
