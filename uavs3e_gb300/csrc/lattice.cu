@@ -25,14 +25,16 @@
 //
 // The stages are bound by instruction issue and by the waits at their barriers, not by memory (a 1080p
 // frame at four QPs moves 1.06 GB, 0.16 ms of its time).  Prediction by table, four samples a task, the
-// QPs in pairs, the inverse stages over the coded jobs only and the Hadamard rows packed two to a register
+// inverse stages over the coded jobs only, QPs in pairs and the Hadamard rows packed two to a register
 // took a 1080p frame at four QPs from 28.7 to 27.5 ms, 416x240 at one QP with the IPF from 0.83 to 0.81,
 // and SATD of all modes + records of 5 at four QPs on 1272x716 from 6.57 to 5.81.  A SATD-only tile holds
 // predictions alone, so a CU's samples are fetched for several times as many modes, and a tile begins
 // with two dependent global loads (its CU's position, then the samples) instead of six: 27.3, 0.79 and
 // 3.75 ms.  Products over chunks of eight entries in rolled loops (a third of the code, and the inverse
 // passes stop at the last chunk that holds a level), rows stored whole and saturating packs: 24.9, 0.71
-// and 3.58 ms.  Four columns a task in the inverse row pass and levels formed two to a word: 24.0, 0.71, 3.54.
+// and 3.58 ms.  Four columns a task in the inverse row pass
+// and levels formed two to a word: 24.0, 0.71, 3.54.  One QP at a time again, with the job's buffers sharing
+// bytes, so that a tile holds half as many jobs more: 22.4, 0.59, 3.49.
 #include "lattice_kernel.cuh"
 
 #include <mutex>
@@ -144,7 +146,7 @@ __global__ void __launch_bounds__(32) k_lat_plan(int *counters, const LatPlan Q)
 }
 
 // the persistent lattice: tiles from the queue until it is empty.  Its static shared memory is
-// at most 8 KB: with a 48 KB layout, four CTAs then fit an SM
+// at most 6 KB: with a 50 KB layout, four CTAs then fit an SM
 __global__ void __launch_bounds__(LAT_THREADS, 4) k_intra_lattice(const __grid_constant__ LatParams P)
 {
     extern __shared__ __align__(16) u8 sm[];
@@ -204,7 +206,7 @@ int lattice_tables(DevTables &t)
 // layout the candidate budgets give (every run writes the same records) and keeps the fastest.
 // All budgets are at most LAT_BUDGET, the launch's shared-memory size, so four CTAs share an SM.
 constexpr int LAT_TUNE_MIN_CUS = 512;
-static const int kLatBudgets[] = { 16 * 1024, 24 * 1024, 32 * 1024, 40 * 1024, 48 * 1024 };
+static const int kLatBudgets[] = { 16 * 1024, 24 * 1024, 32 * 1024, 40 * 1024, LAT_BUDGET };
 struct LatTune {
     std::mutex mu;
     int budget[34][LAT_SHAPES] = {};   // 0: the default LAT_BUDGET (not tuned)

@@ -57,7 +57,7 @@ struct LatQ { u32 ssd; u32 coef_hash; u16 num_nz; s16 last_nz; u32 sum_abs; };
 struct alignas(8) LatPerm { int id; s16 x, y; };   // a CU of a class: its index and position
 
 constexpr int LAT_THREADS = 256;
-constexpr int LAT_BUDGET = 48 * 1024;   // default dynamic shared bytes per CTA (4 CTAs per SM with the static part)
+constexpr int LAT_BUDGET = 50 * 1024;   // default dynamic shared bytes per CTA (4 CTAs per SM with the static part)
 constexpr int LAT_MAX_QP = 4;
 constexpr int LAT_SMEM_MAX = 96 * 1024;   // dynamic shared memory admitted by the kernel attribute
 constexpr int LAT_MAX_G = 8;            // CUs per CTA
@@ -79,8 +79,7 @@ struct LatLayout {
     int o_cu, cu_bytes;                 // per-CU blocks: org, neighbours, org row-pass sums
     int c_org, c_nb, c_torg;
     int o_job, job_bytes;               // per-job blocks: prediction, T, C, DQ^T, T2
-    int j_pred, j_t, j_c, j_dqt, j_t2;   // (j_dqt, j_t2: of the first QP of a pair; the second's T2 takes T's place)
-    int j_dqt_b;
+    int j_pred, j_t, j_c, j_dqt, j_t2;
     int G, MC, nchunk;                  // CUs per CTA, modes per CTA, mode chunks per CU
     int smem;
 };
@@ -127,11 +126,18 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     int j = 0;
     L.j_pred = j; j += lat_up16(L.h * L.ps);
     const int b_t = lat_up16(L.kw * L.ts * 2), b_t2 = lat_up16(L.h * L.t2s * 2);
-    L.j_t = j; j += tr * (n_qp > 1 && b_t2 > b_t ? b_t2 : b_t);
-    L.j_c = j; j += tr * lat_up16(L.kh * L.cs * 2);
-    L.j_dqt = j; j += tr * lat_up16(L.kw * L.ds * 2);
-    L.j_dqt_b = j; if (n_qp > 1) j += lat_up16(L.kw * L.ds * 2);
-    L.j_t2 = j; j += tr * b_t2;
+    // T is dead once C is formed, and C once the levels of the last QP are: T2 takes T's place, and with one
+    // QP DQT^T takes T's and T2 C's.  (Two QPs at a time, sharing the reads of C, took 24 % more bytes a
+    // job: 23.9 ms where one at a time takes 23.15, of a 1080p frame at four QPs.)
+    const int b_c = lat_up16(L.kh * L.cs * 2), b_dqt = lat_up16(L.kw * L.ds * 2);
+    if (n_qp > 1) {
+        L.j_t = L.j_t2 = j; j += b_t2 > b_t ? b_t2 : b_t;
+        L.j_c = j; j += b_c;
+        L.j_dqt = j; j += b_dqt;
+    } else {
+        L.j_t = L.j_dqt = j; j += tr * (b_dqt > b_t ? b_dqt : b_t);
+        L.j_c = L.j_t2 = j; j += tr * (b_t2 > b_c ? b_t2 : b_c);
+    }
     // an odd multiple of 16 bytes: where a warp holds several jobs, their rows lie on different banks
     // (at a multiple of 128 the quantisation of 4x4 blocks took twice the time)
     L.job_bytes = j | 16;
@@ -183,11 +189,13 @@ struct LatShared {
     LatPerm cu[LAT_MAX_G];
     u8 mode[LAT_MAX_JOBS];
     u32 satd[LAT_MAX_JOBS], ssd0[LAT_MAX_JOBS];   // ssd0: of the prediction, for QPs that code nothing
-    // byte 0: bit q = QP q codes the job; byte 1 + b: the k-th job that QP b of the pair codes
-    u32 flag[LAT_MAX_JOBS];
-    u32 nz[2][LAT_MAX_JOBS], sum[2][LAT_MAX_JOBS], hash[2][LAT_MAX_JOBS], ssd[2][LAT_MAX_JOBS];   // per QP of the pair
-    int last[2][LAT_MAX_JOBS];
-    int coded[2];   // jobs that each QP of the pair codes
+    u32 flag[LAT_MAX_JOBS];   // bit q: QP q codes the job
+    // of the QP at hand: the statistics, the SSD and the list of the jobs it codes.  nz also has bits
+    // 16 + k / 20 + k: chunk k of eight columns / rows holds a level
+    u32 nz[LAT_MAX_JOBS], sum[LAT_MAX_JOBS], hash[LAT_MAX_JOBS], ssd[LAT_MAX_JOBS];
+    int last[LAT_MAX_JOBS];
+    u8 list[LAT_MAX_JOBS];
+    int coded;      // jobs of the list
     int tile_off[LAT_SHAPES + 1], cu_off[LAT_SHAPES], counts[LAT_SHAPES];   // of the queue (LatParams)
     int next[2], rank[2];           // the tile after this one and its launch rank, by the tile's parity
     int tables;   // shape class whose matrices and scan table are in place (-1: none)
@@ -589,8 +597,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     const int grp = tile / L.nchunk, chunk = tile % L.nchunk;
     const int cu0 = grp * L.G;
     const int Gv = min(L.G, n_shape - cu0);
-    const int m0 = chunk * L.MC;
-    const int MCv = min(L.MC, P.n_modes - m0);
+    const int m0 = chunk * P.n_modes / L.nchunk;          // chunks differ by one mode at most
+    const int MCv = (chunk + 1) * P.n_modes / L.nchunk - m0;
     const int J = Gv * MCv;
     if (Gv <= 0 || MCv <= 0) return;
     // j / MCv as a multiply: with m = ceil(2^16 / MCv), (j m) >> 16 = j / MCv for every
@@ -607,7 +615,6 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
 #define JT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t))
 #define JC(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_c))
 #define JDQT(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_dqt))
-#define JDQTB(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_dqt_b))
 #define JT2(j) ((s16 *)(jobb + (j) * L.job_bytes + L.j_t2))
 #define CORG(g) (cub + (g) * L.cu_bytes + L.c_org)
 
@@ -823,46 +830,32 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     for (int j = tid; j < J; j += LAT_THREADS)
         P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
 
-    // two QPs at a time: they share the reads of the coefficients, and half the CTA barriers are left
-    for (int q0 = 0; q0 < P.n_qp; q0 += 2) {
-        const int nb = min(2, P.n_qp - q0);
-        u32 q_value[2];
-        int dq_scale[2], dq_shift[2];
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int qp = P.qp[min(q0 + b, LAT_MAX_QP - 1)];
-            q_value[b] = (u32)(((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0));
-            dq_scale[b] = (int)kDqScale[qp];
-            dq_shift[b] = (int)kDqShift[qp] - (15 - 8 - log2_size) + 1;
-        }
-        // the lists of the jobs each QP codes: quant_check found a coefficient above its threshold, whose
+    for (int q = 0; q < P.n_qp; q++) {
+        const int qp = P.qp[q];
+        const int q_value = ((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0);
+        const int dq_scale = (int)kDqScale[qp], dq_shift = (int)kDqShift[qp] - (15 - 8 - log2_size) + 1;
+        // the list of the jobs the QP codes: quant_check found a coefficient above its threshold, whose
         // level is then not zero; the others keep the prediction's SSD and empty statistics
-        int *coded = S.coded;
-        if (tid < 2) coded[tid] = 0;
-        for (int j = tid; j < nb * J; j += LAT_THREADS) {
-            const int b = j >= J ? 1 : 0, jj = j - b * J;
-            S.nz[b][jj] = 0; S.sum[b][jj] = 0; S.hash[b][jj] = 0; S.last[b][jj] = -1; S.ssd[b][jj] = 0;
+        if (tid == 0) S.coded = 0;
+        for (int j = tid; j < J; j += LAT_THREADS) {
+            S.nz[j] = 0; S.sum[j] = 0; S.hash[j] = 0; S.last[j] = -1; S.ssd[j] = 0;
         }
         __syncthreads();
-        for (int base = wbase; base < nb * J; base += LAT_THREADS) {
-            const int j = base + lane, b = j >= J ? 1 : 0, jj = j - b * J;
-            const bool own = j < nb * J && ((s_flag[jj] >> (q0 + b)) & 1);
-            // a warp may hold jobs of both QPs: one ballot each
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-                const u32 m = __ballot_sync(0xFFFFFFFFu, own && b == c);
-                int at = 0;
-                if (lane == 0 && m) at = atomicAdd(&coded[c], __popc(m));
-                at = __shfl_sync(0xFFFFFFFFu, at, 0);
-                if (own && b == c) ((u8 *)s_flag)[4 * (at + __popc(m & ((1u << lane) - 1))) + 1 + c] = (u8)jj;
-            }
+        for (int base = wbase; base < J; base += LAT_THREADS) {
+            const int j = base + lane;
+            const bool own = j < J && ((s_flag[j] >> q) & 1);
+            const u32 m = __ballot_sync(0xFFFFFFFFu, own);
+            int at = 0;
+            if (lane == 0 && m) at = atomicAdd(&S.coded, __popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (own) S.list[at + __popc(m & ((1u << lane) - 1))] = (u8)j;
         }
         // first-pass levels, statistics, dequantisation (stored transposed, DQ^T[u][v], each row
         // in even/odd order of v).  The
         // level (|c| q_value + 2^(q_bits-1)) >> q_bits is exact in 32 bits: |c| <= 2^15 and
         // q_value < 2^15; it is 0 below the level threshold and, with q_value 0, for a QP that codes
         // nothing of the job.  A task is one coefficient row v of a job over RU columns (lanes take
-        // consecutive v) at both QPs: the statistics are summed in registers and reduced once per task.
+        // consecutive v): the statistics are summed in registers and reduced once per task.
         // The position weight of raster position p = v w + u is linear in p but for its lowest bit, and
         // w and the first column are even: weight = row part + constant of the column.
         {
@@ -872,100 +865,96 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 const bool act = i < J * TPJ;
                 const int ii = act ? i : base;
                 const int v = ii & (KH_ - 1), uc = (ii >> LKH_) % NUC, j = ii / TPJ;
-                const u32 fl = act ? s_flag[j] >> q0 : 0u;
+                const u32 on = act ? (s_flag[j] >> q) & 1 : 0u;
+                if (!__any_sync(0xFFFFFFFFu, on)) continue;
                 const u32 wrow = (u32)(v * w + uc * RU) * 0x9E3779B1u + 0x7F4A7C15u;
+                const int qv = on ? q_value : 0;
                 u32 cp[RU / 2];
                 lat_row<RU / 2>(JC(j) + v * L.cs + uc * RU, cp);
-#pragma unroll 1
-                for (int b = 0; b < nb; b++) {
-                    const u32 on = (fl >> b) & 1;
-                    const u32 qv = on ? b ? q_value[1] : q_value[0] : 0u;
-                    // level of c: (|c| qv + 2^(q_bits - 1)) >> q_bits with c's sign, which is
-                    // (c qv + 2^(q_bits - 1) - (c < 0)) >> q_bits; two to a word (|c| <= 2^15, qv < 2^15 and
-                    // q_bits >= 15, so 16 bits hold one)
-                    int lv[RU];
-                    u32 lp[RU / 2], mask = 0;
+                // level of c: (|c| qv + 2^(q_bits - 1)) >> q_bits with c's sign, which is
+                // (c qv + 2^(q_bits - 1) - (c < 0)) >> q_bits; two to a word (|c| <= 2^15, qv < 2^15 and
+                // q_bits >= 15, so 16 bits hold one)
+                int lv[RU];
+                u32 lp[RU / 2], mask = 0;
 #pragma unroll
-                    for (int r = 0; r < RU; r++) {
-                        const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
-                        lv[r] = (c * (int)qv + ((int)qadd + (c >> 31))) >> q_bits;
+                for (int r = 0; r < RU; r++) {
+                    const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
+                    lv[r] = (c * qv + ((int)qadd + (c >> 31))) >> q_bits;
+                }
+#pragma unroll
+                for (int k = 0; k < RU / 2; k++) {
+                    lp[k] = __byte_perm((u32)lv[2 * k], (u32)lv[2 * k + 1], 0x5410);
+                    mask += __vminu2(lp[k], 0x00010001u) << k;   // bit k: column 2k, bit 16 + k: column 2k + 1
+                }
+                // rows and chunks of eight columns without a level are not stored: the inverse passes
+                // do not read them (a chunk with a level is stored whole)
+                if (!__any_sync(0xFFFFFFFFu, mask != 0)) continue;
+                s16 *dqt = JDQT(j) + uc * RU * L.ds + lat_eo(v, KH_);
+                u32 sa = 0;
+#pragma unroll
+                for (int r = 0; r < RU; r += 2) {
+                    sa += (u32)abs(lv[r]) + (u32)abs(lv[r + 1]);
+                    const int d0 = (lv[r] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
+                    const int d1 = (lv[r + 1] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
+                    u32 d = lat_pack16(d0, d1);
+                    if (odd) d = __byte_perm((u32)(((int)(s16)(d & 0xFFFF) * 181 + 128) >> 8), (u32)((((int)d >> 16) * 181 + 128) >> 8), 0x5410);
+                    if (act) {
+                        dqt[r * L.ds] = (s16)(d & 0xFFFF);
+                        dqt[(r + 1) * L.ds] = (s16)(d >> 16);
                     }
+                }
+                // sum of level x weight, the weight of column r being wrow + K r + (r & 1): from the
+                // sums over the pairs k of s_k = lev[2k] + lev[2k+1], of k s_k, and of the odd columns
+                int at = 0, ks = 0, odds = 0;
 #pragma unroll
-                    for (int k = 0; k < RU / 2; k++) {
-                        lp[k] = __byte_perm((u32)lv[2 * k], (u32)lv[2 * k + 1], 0x5410);
-                        mask += __vminu2(lp[k], 0x00010001u) << k;   // bit k: column 2k, bit 16 + k: column 2k + 1
-                    }
-                    // rows and chunks of eight columns without a level are not stored: the inverse passes
-                    // do not read them (a chunk with a level is stored whole)
-                    if (!__any_sync(0xFFFFFFFFu, mask != 0)) continue;
-                    const int scale = b ? dq_scale[1] : dq_scale[0], shift = b ? dq_shift[1] : dq_shift[0];
-                    s16 *dqt = (b ? JDQTB(j) : JDQT(j)) + uc * RU * L.ds + lat_eo(v, KH_);
-                    u32 sa = 0;
+                for (int k = RU / 2 - 1; k >= 0; k--) {
+                    at = dp2a_lo(lp[k], 0x0101u, at);
+                    if (k > 0) ks += at;
+                    odds = dp2a_lo(lp[k], 0x0100u, odds);
+                }
+                u32 hs = (u32)at * wrow + (u32)ks * (2u * 0x9E3779B1u) + (u32)odds * (0x9E3779B1u + 1u);
+                // the count of levels rides above the sum of their magnitudes: of a segment's at most
+                // 32 x 8 levels the sum is below 2^23
+                const u32 both = lat_seg_sum<SEG>(sa | (u32)__popc(mask) << 23, lane);
+                const u32 nz = both >> 23;
+                sa = both & 0x7FFFFFu; hs = lat_seg_sum<SEG>(hs, lane);
+                // along a row the scan index grows with the column
+                const int he = 31 - __clz((int)(mask & 0xFFFFu)), ho = 31 - __clz((int)(mask >> 16));
+                const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + max(2 * he, 2 * ho + 1)] : -1;
+                const int last = lat_seg_max<SEG>(own_last, lane);
+                const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
+                if (act && (lane & (SEG - 1)) == 0 && nz) {
+                    // which chunks of columns and of rows hold levels (bits 16.. and 20..)
+                    u32 ch = 0;
+                    const u32 own = SEG == 32 ? rows : (rows >> lane) & ((1u << (SEG & 31)) - 1);
 #pragma unroll
-                    for (int r = 0; r < RU; r += 2) {
-                        sa += (u32)abs(lv[r]) + (u32)abs(lv[r + 1]);
-                        const int d0 = (lv[r] * scale + (1 << shift >> 1)) >> shift;
-                        const int d1 = (lv[r + 1] * scale + (1 << shift >> 1)) >> shift;
-                        u32 d = lat_pack16(d0, d1);
-                        if (odd) d = __byte_perm((u32)(((int)(s16)(d & 0xFFFF) * 181 + 128) >> 8), (u32)((((int)d >> 16) * 181 + 128) >> 8), 0x5410);
-                        if (act) {
-                            dqt[r * L.ds] = (s16)(d & 0xFFFF);
-                            dqt[(r + 1) * L.ds] = (s16)(d >> 16);
-                        }
-                    }
-                    // sum of level x weight, the weight of column r being wrow + K r + (r & 1): from the
-                    // sums over the pairs k of s_k = lev[2k] + lev[2k+1], of k s_k, and of the odd columns
-                    int at = 0, ks = 0, odds = 0;
+                    for (int k = 0; k < SEG / KH_; k++)
+                        if ((own >> (k * KH_ & 31)) & (KH_ == 32 ? 0xFFFFFFFFu : (1u << (KH_ & 31)) - 1)) ch |= 1u << (16 + (uc + k) % NUC);
 #pragma unroll
-                    for (int k = RU / 2 - 1; k >= 0; k--) {
-                        at = dp2a_lo(lp[k], 0x0101u, at);
-                        if (k > 0) ks += at;
-                        odds = dp2a_lo(lp[k], 0x0100u, odds);
-                    }
-                    u32 hs = (u32)at * wrow + (u32)ks * (2u * 0x9E3779B1u) + (u32)odds * (0x9E3779B1u + 1u);
-                    // the count of levels rides above the sum of their magnitudes: of a segment's at most
-                    // 32 x 8 levels the sum is below 2^23
-                    const u32 both = lat_seg_sum<SEG>(sa | (u32)__popc(mask) << 23, lane);
-                    const u32 nz = both >> 23;
-                    sa = both & 0x7FFFFFu; hs = lat_seg_sum<SEG>(hs, lane);
-                    // along a row the scan index grows with the column
-                    const int he = 31 - __clz((int)(mask & 0xFFFFu)), ho = 31 - __clz((int)(mask >> 16));
-                    const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + max(2 * he, 2 * ho + 1)] : -1;
-                    const int last = lat_seg_max<SEG>(own_last, lane);
-                    const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
-                    if (act && (lane & (SEG - 1)) == 0 && nz) {
-                        // which chunks of columns and of rows hold levels (bits 16.. and 20..)
-                        u32 ch = 0;
-                        const u32 own = SEG == 32 ? rows : (rows >> lane) & ((1u << (SEG & 31)) - 1);
-#pragma unroll
-                        for (int k = 0; k < SEG / KH_; k++)
-                            if ((own >> (k * KH_ & 31)) & (KH_ == 32 ? 0xFFFFFFFFu : (1u << (KH_ & 31)) - 1)) ch |= 1u << (16 + (uc + k) % NUC);
-#pragma unroll
-                        for (int k = 0; k < SEG / 8; k++)
-                            if ((own >> (k * 8)) & 0xFFu) ch |= 1u << (20 + (KH_ < 8 ? 0 : k % (KH_ / 8 ? KH_ / 8 : 1)));
-                        if (KH_ < 8) ch |= 1u << 20;
-                        atomicAdd(&S.nz[b][j], nz);
-                        atomicOr(&S.nz[b][j], ch);
-                        atomicAdd(&S.sum[b][j], sa);
-                        atomicAdd(&S.hash[b][j], hs);
-                        atomicMax(&S.last[b][j], last);
-                    }
+                    for (int k = 0; k < SEG / 8; k++)
+                        if ((own >> (k * 8)) & 0xFFu) ch |= 1u << (20 + (KH_ < 8 ? 0 : k % (KH_ / 8 ? KH_ / 8 : 1)));
+                    if (KH_ < 8) ch |= 1u << 20;
+                    atomicAdd(&S.nz[j], nz);
+                    atomicOr(&S.nz[j], ch);
+                    atomicAdd(&S.sum[j], sa);
+                    atomicAdd(&S.hash[j], hs);
+                    atomicMax(&S.last[j], last);
                 }
             }
         }
         __syncthreads(); LAT_STAGE(6);
-        // the inverse passes run over the coded (job, QP) pairs only
-        const int n0 = coded[0], JC2 = n0 + coded[1];
+        // the inverse passes run over the coded jobs only
+        const int JC_ = S.coded;
         // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5); a task forms
         // rows y and H-1-y from the even-v and odd-v sums over CU columns u.  Chunks of columns past the
         // last level's are left out, empty ones before it are zeros.  Tiles with few
         // jobs take CU/2 columns per task so that the CTA's threads still have a task each.
         auto inv_col = [&](auto cu_tag) {
             constexpr int CU = decltype(cu_tag)::value, NCU = KW_ / CU;
-            for (int i = tid; i < JC2 * NCU * (H_ / 2); i += LAT_THREADS) {
+            for (int i = tid; i < JC_ * NCU * (H_ / 2); i += LAT_THREADS) {
                 const int y = i & (H_ / 2 - 1), uc = (i >> (LH - 1)) % NCU, k = i / ((H_ / 2) * NCU);
-                const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
-                const u32 ch = S.nz[b][j] >> 16;
+                const int j = S.list[k];
+                const u32 ch = S.nz[j] >> 16;
                 const int col = uc * CU >> 3;
                 if (KW_ > 8 && !((ch & 15) >> col)) continue;
                 int e[CU], o[CU];
@@ -974,9 +963,9 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
 #pragma unroll
                     for (int r = 0; r < CU; r++) e[r] = o[r] = 0;
                 } else {
-                    lat_eo_sums<KH_, CU>((b ? JDQTB(j) : JDQT(j)) + uc * CU * L.ds, L.ds, fht + y * L.fht_ws, nv, e, o);
+                    lat_eo_sums<KH_, CU>(JDQT(j) + uc * CU * L.ds, L.ds, fht + y * L.fht_ws, nv, e, o);
                 }
-                s16 *t2 = b ? JT(j) : JT2(j);
+                s16 *t2 = JT2(j);
 #pragma unroll
                 for (int half = 0; half < 2; half++) {
                     int t[CU];
@@ -996,7 +985,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 }
             }
         };
-        if (RU == 8 && JC2 * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, 4>{});
+        if (RU == 8 && JC_ * NUC * (H_ / 2) < LAT_THREADS) inv_col(std::integral_constant<int, 4>{});
         else inv_col(std::integral_constant<int, RU>{});
         __syncthreads(); LAT_STAGE(7);
         // inverse row pass, reconstruction, SSD: a task is the columns x, x+1, W-2-x, W-1-x over CY
@@ -1006,13 +995,13 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         auto inv_row = [&](auto cy_tag) {
             constexpr int CY = decltype(cy_tag)::value, NCY = H_ / CY;
             constexpr int TPJ = (W_ / 4) * NCY, SEG = TPJ < 32 ? TPJ : 32;
-            for (int base = wbase; base < JC2 * TPJ; base += LAT_THREADS) {
+            for (int base = wbase; base < JC_ * TPJ; base += LAT_THREADS) {
                 const int i = base + lane;
-                const bool act = i < JC2 * TPJ;
+                const bool act = i < JC_ * TPJ;
                 const int ii = act ? i : base;
                 const int x = (ii & (W_ / 4 - 1)) * 2, yc = (ii >> (LW - 2)) % NCY, k = ii / TPJ;
-                const int b = k >= n0 ? 1 : 0, j = ((const u8 *)s_flag)[4 * (k - b * n0) + 1 + b];
-                const s16 *t2 = (b ? JT(j) : JT2(j)) + yc * CY * L.t2s;
+                const int j = S.list[k];
+                const s16 *t2 = JT2(j) + yc * CY * L.t2s;
                 const u32 *f = fwt + x * L.fwt_ws;
                 // e0, o0: column x (and W-1-x); e1, o1: column x+1 (and W-2-x)
                 int e0[CY], o0[CY], e1[CY], o1[CY];
@@ -1027,7 +1016,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 } else {
 #pragma unroll
                     for (int r = 0; r < CY; r++) { e0[r] = e1[r] = 2048; o0[r] = o1[r] = 0; }
-                    const int nu = KW_ > 8 ? 32 - __clz((int)((S.nz[b][j] >> 16) & 15)) : 1;
+                    const int nu = KW_ > 8 ? 32 - __clz((int)((S.nz[j] >> 16) & 15)) : 1;
 #pragma unroll 1
                     for (int c = 0; c < nu; c++, t2 += 8, f += 2) {
                         const uint2 f0 = *reinterpret_cast<const uint2 *>(f), f1 = *reinterpret_cast<const uint2 *>(f + L.fwt_ws);
@@ -1054,22 +1043,20 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 }
                 if (!act) e = 0;
                 e = lat_seg_sum<SEG>(e, lane);
-                if (act && (lane & (SEG - 1)) == 0) atomicAdd(&S.ssd[b][j], e);
+                if (act && (lane & (SEG - 1)) == 0) atomicAdd(&S.ssd[j], e);
             }
         };
-        if (JC2 * (W_ / 4) * (H_ / 4) < LAT_THREADS) inv_row(std::integral_constant<int, 2>{});
+        if (JC_ * (W_ / 4) * (H_ / 4) < LAT_THREADS) inv_row(std::integral_constant<int, 2>{});
         else inv_row(std::integral_constant<int, 4>{});
         __syncthreads(); LAT_STAGE(8);
-        for (int i = tid; i < nb * J; i += LAT_THREADS) {
-            const int j = nb == 2 ? i >> 1 : i, b = nb == 2 ? i & 1 : 0, g = JG(j);
-            const bool own = (s_flag[j] >> (q0 + b)) & 1;
+        for (int j = tid; j < J; j += LAT_THREADS) {
             LatQ o;
-            o.ssd = own ? S.ssd[b][j] : S.ssd0[j];
-            o.coef_hash = S.hash[b][j];
-            o.num_nz = (u16)S.nz[b][j];
-            o.last_nz = (s16)S.last[b][j];
-            o.sum_abs = S.sum[b][j];
-            P.q_out[((size_t)S.cu[g].id * 33 + s_mode[j]) * P.n_qp + q0 + b] = o;
+            o.ssd = (s_flag[j] >> q) & 1 ? S.ssd[j] : S.ssd0[j];
+            o.coef_hash = S.hash[j];
+            o.num_nz = (u16)S.nz[j];
+            o.last_nz = (s16)S.last[j];
+            o.sum_abs = S.sum[j];
+            P.q_out[((size_t)S.cu[JG(j)].id * 33 + s_mode[j]) * P.n_qp + q] = o;
         }
         __syncthreads(); LAT_STAGE(9);
     }
@@ -1079,7 +1066,6 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
 #undef JC
 #undef JDQT
 #undef JT2
-#undef JDQTB
 #undef CORG
 }
 
