@@ -830,6 +830,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     for (int j = tid; j < J; j += LAT_THREADS)
         P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
 
+    // levels and magnitudes of a block of at most 256 coefficients go into one word, the count from bit 23
+    constexpr bool PACK = KW_ * KH_ <= 256, CHUNKS = KW_ > 8 || KH_ > 8;
     for (int q = 0; q < P.n_qp; q++) {
         const int qp = P.qp[q];
         const int q_value = ((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0);
@@ -925,6 +927,11 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
                 if (act && (lane & (SEG - 1)) == 0 && nz) {
                     // which chunks of columns and of rows hold levels (bits 16.. and 20..)
+                    atomicAdd(&S.sum[j], PACK ? both : sa);
+                    atomicAdd(&S.hash[j], hs);
+                    atomicMax(&S.last[j], last);
+                    if (!PACK) atomicAdd(&S.nz[j], nz);
+                    if (!CHUNKS) continue;
                     u32 ch = 0;
                     const u32 own = SEG == 32 ? rows : (rows >> lane) & ((1u << (SEG & 31)) - 1);
 #pragma unroll
@@ -934,11 +941,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                     for (int k = 0; k < SEG / 8; k++)
                         if ((own >> (k * 8)) & 0xFFu) ch |= 1u << (20 + (KH_ < 8 ? 0 : k % (KH_ / 8 ? KH_ / 8 : 1)));
                     if (KH_ < 8) ch |= 1u << 20;
-                    atomicAdd(&S.nz[j], nz);
                     atomicOr(&S.nz[j], ch);
-                    atomicAdd(&S.sum[j], sa);
-                    atomicAdd(&S.hash[j], hs);
-                    atomicMax(&S.last[j], last);
                 }
             }
         }
@@ -1053,9 +1056,9 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
             LatQ o;
             o.ssd = (s_flag[j] >> q) & 1 ? S.ssd[j] : S.ssd0[j];
             o.coef_hash = S.hash[j];
-            o.num_nz = (u16)S.nz[j];
+            o.num_nz = (u16)(PACK ? S.sum[j] >> 23 : S.nz[j] & 0xFFFFu);
             o.last_nz = (s16)S.last[j];
-            o.sum_abs = S.sum[j];
+            o.sum_abs = PACK ? S.sum[j] & 0x7FFFFFu : S.sum[j];
             P.q_out[((size_t)S.cu[JG(j)].id * 33 + s_mode[j]) * P.n_qp + q] = o;
         }
         __syncthreads(); LAT_STAGE(9);
