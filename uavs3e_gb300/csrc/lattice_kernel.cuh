@@ -12,14 +12,14 @@
 
 namespace uc {
 
-__device__ __constant__ static const u32 kDqScale[80] = {
+static const u32 hDqScale[80] = {
     32768, 36061, 38968, 42495, 46341, 50535, 55437, 60424, 32932, 35734, 38968, 42495, 46177, 50535, 55109, 59933,
     65535, 35734, 38968, 42577, 46341, 50617, 55027, 60097, 32809, 35734, 38968, 42454, 46382, 50576, 55109, 60056,
     65535, 35734, 38968, 42495, 46320, 50515, 55109, 60076, 65535, 35744, 38968, 42495, 46341, 50535, 55099, 60087,
     65535, 35734, 38973, 42500, 46341, 50535, 55109, 60097, 32771, 35734, 38965, 42497, 46341, 50535, 55109, 60099,
     32768, 36061, 38968, 42495, 46341, 50535, 55437, 60424, 32932, 35734, 38968, 42495, 46177, 50535, 55109, 59933,
 };
-__device__ __constant__ static const u8 kDqShift[80] = {
+static const u8 hDqShift[80] = {
     14, 14, 14, 14, 14, 14, 14, 14, 13, 13, 13, 13, 13, 13, 13, 13, 13, 12, 12, 12, 12, 12, 12, 12,
     11, 11, 11, 11, 11, 11, 11, 11, 11, 10, 10, 10, 10, 10, 10, 10, 10, 9, 9, 9, 9, 9, 9, 9,
     9, 8, 8, 8, 8, 8, 8, 8, 7, 7, 7, 7, 7, 7, 7, 7, 6, 6, 6, 6, 6, 6, 6, 6, 5, 5, 5, 5, 5, 5, 5, 5,
@@ -160,13 +160,31 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     L.smem = o;
 }
 
+// what a QP means for a CU size: the quantisation multiplier, the magnitude above which a coefficient makes
+// quant_check code the block, and the dequantisation.  Formed on the host: a division and four table reads
+// per QP, thread and tile otherwise.
+struct LatQp { int q_value, thr, dq_scale, dq_shift; };
+__host__ __device__ constexpr int lat_q_bits(int log2_size) { return 14 + (15 - 8 - log2_size); }
+
+inline LatQp lat_qp(int qp, int l_samples, int is_intra)
+{
+    const int odd = l_samples & 1, log2_size = l_samples >> 1, q_bits = lat_q_bits(log2_size);
+    const int offset = (is_intra ? 201 : 153) << (q_bits - 9);
+    LatQp o;
+    o.q_value = ((int)hQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0);
+    o.thr = ((((1 << q_bits) - offset) << 10) / o.q_value - 1) >> 10;
+    o.dq_scale = (int)hDqScale[qp];
+    o.dq_shift = (int)hDqShift[qp] - (15 - 8 - log2_size) + 1;
+    return o;
+}
+
 struct LatParams {
     const pel *org; int i_org;
     int org_words;            // org and i_org are multiples of 4: org blocks are read by words
     const pel *rec; int i_rec;
     int W, H;
-    int ipf, n_qp, is_intra;
-    int qp[LAT_MAX_QP];
+    int ipf, n_qp;
+    LatQp qp[9][LAT_MAX_QP];  // [log2 of the samples of a CU - 4][QP]
     u32 *satd_out; LatQ *q_out;
     const u8 *images;         // [class][LAT_IMAGE_BYTES] transform and scan tables (lat_image_fill)
     const u32 *ipred;         // the prediction table (lat_table_at)
@@ -768,20 +786,12 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
 
     // quantisation parameters per QP
     const int odd = lN & 1, log2_size = lN >> 1;
-    const int q_bits = 14 + (15 - 8 - log2_size);
-    const int offset = (P.is_intra ? 201 : 153) << (q_bits - 9);
+    const int q_bits = lat_q_bits(log2_size);
     const u32 qadd = 1u << (q_bits - 1);
 
     // ---- forward column pass C[v][u] = (sum_y Fh[v][y] T[u][y] + rnd2) >> sh2, and the
     // quant_check flags of every QP (bit q: some |C| above that QP's all-zero threshold)
     {
-        int nz_thr[LAT_MAX_QP];
-#pragma unroll
-        for (int q = 0; q < LAT_MAX_QP; q++) {
-            const int qp = P.qp[q];
-            const int q_value = ((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0);
-            nz_thr[q] = ((((1 << q_bits) - offset) << 10) / q_value - 1) >> 10;
-        }
         const int sh2 = lh + 5, rnd2 = 1 << (sh2 - 1);
         for (int i = tid; i < (P.n_qp > 0 ? J * NUC * KH_ : 0); i += LAT_THREADS) {
             const int v = i & (KH_ - 1), uc = (i >> LKH_) % NUC, j = i / (KH_ * NUC);
@@ -822,7 +832,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
             u32 fl = 0;
 #pragma unroll
             for (int q = 0; q < LAT_MAX_QP; q++)
-                if (q < P.n_qp && amax > nz_thr[q]) fl |= 1u << q;
+                if (q < P.n_qp && amax > P.qp[lN - 4][q].thr) fl |= 1u << q;
             if (fl) atomicOr(&s_flag[j], fl);
         }
     }
@@ -833,9 +843,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     // levels and magnitudes of a block of at most 256 coefficients go into one word, the count from bit 23
     constexpr bool PACK = KW_ * KH_ <= 256, CHUNKS = KW_ > 8 || KH_ > 8;
     for (int q = 0; q < P.n_qp; q++) {
-        const int qp = P.qp[q];
-        const int q_value = ((int)kQScale[qp] * (odd ? 181 : 1) + (odd ? 64 : 0)) >> (odd ? 7 : 0);
-        const int dq_scale = (int)kDqScale[qp], dq_shift = (int)kDqShift[qp] - (15 - 8 - log2_size) + 1;
+        const int q_value = P.qp[lN - 4][q].q_value, dq_scale = P.qp[lN - 4][q].dq_scale, dq_shift = P.qp[lN - 4][q].dq_shift;
         // the list of the jobs the QP codes: quant_check found a coefficient above its threshold, whose
         // level is then not zero; the others keep the prediction's SSD and empty statistics
         if (tid == 0) S.coded = 0;
