@@ -35,7 +35,8 @@
 // and 3.58 ms.  Four columns a task in the inverse row pass
 // and levels formed two to a word: 24.0, 0.71, 3.54.  One QP at a time again, with the job's buffers sharing
 // bytes, so that a tile holds half as many jobs more: 22.4, 0.59, 3.49.  The constants of a QP formed on the host
-// (a division and four table reads per QP, thread and tile): 21.8, 0.57, 3.46.
+// (a division and four table reads per QP, thread and tile) and 16 coefficients
+// a quantisation task: 21.4, 0.57, 3.46.
 #include "lattice_kernel.cuh"
 
 #include <mutex>

@@ -864,91 +864,114 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         // in even/odd order of v).  The
         // level (|c| q_value + 2^(q_bits-1)) >> q_bits is exact in 32 bits: |c| <= 2^15 and
         // q_value < 2^15; it is 0 below the level threshold and, with q_value 0, for a QP that codes
-        // nothing of the job.  A task is one coefficient row v of a job over RU columns (lanes take
-        // consecutive v): the statistics are summed in registers and reduced once per task.
+        // nothing of the job.  A task is RV coefficient rows (HV apart) of a job over RU columns, 16
+        // coefficients or 8, and lanes take consecutive v: the statistics are summed in registers and reduced
+        // once per task (with 8 coefficients a task, reductions and indexing were half of the instructions;
+        // above 1024 samples a tile holds so few jobs that 8 keep more threads busy).
         // The position weight of raster position p = v w + u is linear in p but for its lowest bit, and
         // w and the first column are even: weight = row part + constant of the column.
         {
-            constexpr int TPJ = KH_ * NUC, SEG = TPJ < 32 ? TPJ : 32;
+            constexpr int CT = W_ * H_ > 1024 ? 8 : 16, RV = CT / RU < KH_ ? CT / RU : KH_, HV = KH_ / RV;
+            constexpr int TPJ = HV * NUC, SEG = TPJ < 32 ? TPJ : 32;
             for (int base = wbase; base < J * TPJ; base += LAT_THREADS) {
                 const int i = base + lane;
                 const bool act = i < J * TPJ;
                 const int ii = act ? i : base;
-                const int v = ii & (KH_ - 1), uc = (ii >> LKH_) % NUC, j = ii / TPJ;
+                const int v = ii % HV, uc = ii / HV % NUC, j = ii / TPJ;
                 const u32 on = act ? (s_flag[j] >> q) & 1 : 0u;
                 if (!__any_sync(0xFFFFFFFFu, on)) continue;
-                const u32 wrow = (u32)(v * w + uc * RU) * 0x9E3779B1u + 0x7F4A7C15u;
                 const int qv = on ? q_value : 0;
-                u32 cp[RU / 2];
-                lat_row<RU / 2>(JC(j) + v * L.cs + uc * RU, cp);
                 // level of c: (|c| qv + 2^(q_bits - 1)) >> q_bits with c's sign, which is
                 // (c qv + 2^(q_bits - 1) - (c < 0)) >> q_bits; two to a word (|c| <= 2^15, qv < 2^15 and
                 // q_bits >= 15, so 16 bits hold one)
-                int lv[RU];
-                u32 lp[RU / 2], mask = 0;
+                int lv[RV][RU];
+                u32 lp[RV][RU / 2], mask[RV], any = 0;
 #pragma unroll
-                for (int r = 0; r < RU; r++) {
-                    const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
-                    lv[r] = (c * qv + ((int)qadd + (c >> 31))) >> q_bits;
-                }
+                for (int k = 0; k < RV; k++) {
+                    u32 cp[RU / 2];
+                    lat_row<RU / 2>(JC(j) + (v + k * HV) * L.cs + uc * RU, cp);
+                    mask[k] = 0;
 #pragma unroll
-                for (int k = 0; k < RU / 2; k++) {
-                    lp[k] = __byte_perm((u32)lv[2 * k], (u32)lv[2 * k + 1], 0x5410);
-                    mask += __vminu2(lp[k], 0x00010001u) << k;   // bit k: column 2k, bit 16 + k: column 2k + 1
+                    for (int r = 0; r < RU; r++) {
+                        const int c = r & 1 ? (int)cp[r >> 1] >> 16 : (int)(s16)(cp[r >> 1] & 0xFFFF);
+                        lv[k][r] = (c * qv + ((int)qadd + (c >> 31))) >> q_bits;
+                    }
+#pragma unroll
+                    for (int r = 0; r < RU / 2; r++) {
+                        lp[k][r] = __byte_perm((u32)lv[k][2 * r], (u32)lv[k][2 * r + 1], 0x5410);
+                        mask[k] += __vminu2(lp[k][r], 0x00010001u) << r;   // bit r: column 2r, bit 16 + r: column 2r + 1
+                    }
+                    any |= mask[k];
                 }
                 // rows and chunks of eight columns without a level are not stored: the inverse passes
                 // do not read them (a chunk with a level is stored whole)
-                if (!__any_sync(0xFFFFFFFFu, mask != 0)) continue;
-                s16 *dqt = JDQT(j) + uc * RU * L.ds + lat_eo(v, KH_);
-                u32 sa = 0;
+                if (!__any_sync(0xFFFFFFFFu, any != 0)) continue;
+                u32 sa = 0, hs = 0, count = 0, rows[RV];
+                int own_last = -1;
 #pragma unroll
-                for (int r = 0; r < RU; r += 2) {
-                    sa += (u32)abs(lv[r]) + (u32)abs(lv[r + 1]);
-                    const int d0 = (lv[r] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
-                    const int d1 = (lv[r + 1] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
-                    u32 d = lat_pack16(d0, d1);
-                    if (odd) d = __byte_perm((u32)(((int)(s16)(d & 0xFFFF) * 181 + 128) >> 8), (u32)((((int)d >> 16) * 181 + 128) >> 8), 0x5410);
-                    if (act) {
-                        dqt[r * L.ds] = (s16)(d & 0xFFFF);
-                        dqt[(r + 1) * L.ds] = (s16)(d >> 16);
+                for (int k = 0; k < RV; k++) {
+                    const int vk = v + k * HV;
+                    s16 *dqt = JDQT(j) + uc * RU * L.ds + lat_eo(vk, KH_);
+#pragma unroll
+                    for (int r = 0; r < RU; r += 2) {
+                        sa += (u32)abs(lv[k][r]) + (u32)abs(lv[k][r + 1]);
+                        const int d0 = (lv[k][r] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
+                        const int d1 = (lv[k][r + 1] * dq_scale + (1 << dq_shift >> 1)) >> dq_shift;
+                        u32 d = lat_pack16(d0, d1);
+                        if (odd) d = __byte_perm((u32)(((int)(s16)(d & 0xFFFF) * 181 + 128) >> 8), (u32)((((int)d >> 16) * 181 + 128) >> 8), 0x5410);
+                        if (act) {
+                            dqt[r * L.ds] = (s16)(d & 0xFFFF);
+                            dqt[(r + 1) * L.ds] = (s16)(d >> 16);
+                        }
                     }
-                }
-                // sum of level x weight, the weight of column r being wrow + K r + (r & 1): from the
-                // sums over the pairs k of s_k = lev[2k] + lev[2k+1], of k s_k, and of the odd columns
-                int at = 0, ks = 0, odds = 0;
+                    // sum of level x weight, the weight of column r being wrow + K r + (r & 1): from the
+                    // sums over the pairs p of s_p = lev[2p] + lev[2p+1], of p s_p, and of the odd columns
+                    int at = 0, ks = 0, odds = 0;
 #pragma unroll
-                for (int k = RU / 2 - 1; k >= 0; k--) {
-                    at = dp2a_lo(lp[k], 0x0101u, at);
-                    if (k > 0) ks += at;
-                    odds = dp2a_lo(lp[k], 0x0100u, odds);
+                    for (int r = RU / 2 - 1; r >= 0; r--) {
+                        at = dp2a_lo(lp[k][r], 0x0101u, at);
+                        if (r > 0) ks += at;
+                        odds = dp2a_lo(lp[k][r], 0x0100u, odds);
+                    }
+                    const u32 wrow = (u32)(vk * w + uc * RU) * 0x9E3779B1u + 0x7F4A7C15u;
+                    hs += (u32)at * wrow + (u32)ks * (2u * 0x9E3779B1u) + (u32)odds * (0x9E3779B1u + 1u);
+                    count += (u32)__popc(mask[k]);
+                    // along a row the scan index grows with the column
+                    const int he = 31 - __clz((int)(mask[k] & 0xFFFFu)), ho = 31 - __clz((int)(mask[k] >> 16));
+                    if (mask[k]) own_last = max(own_last, (int)s_scan[vk * KW_ + uc * RU + max(2 * he, 2 * ho + 1)]);
+                    rows[k] = CHUNKS ? __ballot_sync(0xFFFFFFFFu, mask[k] != 0) : 0;
                 }
-                u32 hs = (u32)at * wrow + (u32)ks * (2u * 0x9E3779B1u) + (u32)odds * (0x9E3779B1u + 1u);
-                // the count of levels rides above the sum of their magnitudes: of a segment's at most
-                // 32 x 8 levels the sum is below 2^23
-                const u32 both = lat_seg_sum<SEG>(sa | (u32)__popc(mask) << 23, lane);
-                const u32 nz = both >> 23;
+                // the count of levels rides above the sum of their magnitudes, which is below 2^23 for a
+                // segment's at most 512 levels (those are below 23053, and below 16303 where a segment has
+                // more than 256); a count of 512 wraps to 0
+                const u32 both = lat_seg_sum<SEG>(sa + (count << 23), lane);
                 sa = both & 0x7FFFFFu; hs = lat_seg_sum<SEG>(hs, lane);
-                // along a row the scan index grows with the column
-                const int he = 31 - __clz((int)(mask & 0xFFFFu)), ho = 31 - __clz((int)(mask >> 16));
-                const int own_last = mask ? (int)s_scan[v * KW_ + uc * RU + max(2 * he, 2 * ho + 1)] : -1;
+                const u32 nz = SEG * CT == 512 && both >> 23 == 0 && sa ? 512u : both >> 23;
                 const int last = lat_seg_max<SEG>(own_last, lane);
-                const u32 rows = __ballot_sync(0xFFFFFFFFu, mask != 0);
                 if (act && (lane & (SEG - 1)) == 0 && nz) {
-                    // which chunks of columns and of rows hold levels (bits 16.. and 20..)
                     atomicAdd(&S.sum[j], PACK ? both : sa);
                     atomicAdd(&S.hash[j], hs);
                     atomicMax(&S.last[j], last);
                     if (!PACK) atomicAdd(&S.nz[j], nz);
                     if (!CHUNKS) continue;
-                    u32 ch = 0;
-                    const u32 own = SEG == 32 ? rows : (rows >> lane) & ((1u << (SEG & 31)) - 1);
+                    // which chunks of columns and of rows hold levels (bits 16.. and 20..)
+                    constexpr u32 SEG_MASK = SEG == 32 ? 0xFFFFFFFFu : (1u << (SEG & 31)) - 1;
+                    u32 ch = KH_ <= 8 ? 1u << 20 : 0u, cols = 0;
 #pragma unroll
-                    for (int k = 0; k < SEG / KH_; k++)
-                        if ((own >> (k * KH_ & 31)) & (KH_ == 32 ? 0xFFFFFFFFu : (1u << (KH_ & 31)) - 1)) ch |= 1u << (16 + (uc + k) % NUC);
+                    for (int k = 0; k < RV; k++) {
+                        const u32 own = (rows[k] >> lane) & SEG_MASK;
+                        cols |= own;
+                        if (KH_ > 8 && HV < 8 && own) ch |= 1u << (20 + k * HV / 8);
+                        if (KH_ > 8 && HV >= 8) {
 #pragma unroll
-                    for (int k = 0; k < SEG / 8; k++)
-                        if ((own >> (k * 8)) & 0xFFu) ch |= 1u << (20 + (KH_ < 8 ? 0 : k % (KH_ / 8 ? KH_ / 8 : 1)));
-                    if (KH_ < 8) ch |= 1u << 20;
+                            for (int g = 0; g < SEG / 8; g++)
+                                if ((own >> (8 * g)) & 0xFFu) ch |= 1u << (20 + k * (HV / 8) + g % (HV >= 8 ? HV / 8 : 1));
+                        }
+                    }
+                    constexpr u32 HV_MASK = HV == 32 ? 0xFFFFFFFFu : (1u << (HV & 31)) - 1;
+#pragma unroll
+                    for (int g = 0; g < SEG / HV; g++)
+                        if ((cols >> (g * HV)) & HV_MASK) ch |= 1u << (16 + (uc + g) % NUC);
                     atomicOr(&S.nz[j], ch);
                 }
             }
