@@ -194,4 +194,13 @@ __host__ __device__ __forceinline__ void had_tile_shape(int w, int h, int *tw, i
     else { if (w == 4 || (w & 7)) { *tw = 4; *th = 8; } else { *tw = 8; *th = 16; } }
 }
 
+// four values clipped to 0..255 and packed, a in the lowest byte
+__device__ __forceinline__ u32 pack_sat_u8(int a, int b, int c, int d)
+{
+    u32 t;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(d), "r"(c), "r"(0));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(b), "r"(a), "r"(t));
+    return t;
+}
+
 }  // namespace uc

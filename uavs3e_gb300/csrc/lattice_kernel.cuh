@@ -305,15 +305,6 @@ __device__ __forceinline__ u32 lat_pack16(int lo, int hi)
     asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(d) : "r"(hi), "r"(lo));
     return d;
 }
-// four values clipped to 0..255 and packed, a in the lowest byte
-__device__ __forceinline__ u32 lat_pack8(int a, int b, int c, int d)
-{
-    u32 t;
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(d), "r"(c), "r"(0));
-    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(b), "r"(a), "r"(t));
-    return t;
-}
-
 // stores NW words of a row (aligned to its size)
 template <int NW>
 __device__ __forceinline__ void lat_store(void *p, const u32 (&v)[NW])
@@ -1071,7 +1062,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                     const auto pair = [](const pel *p) { return (u32)*reinterpret_cast<const u16 *>(p); };
                     const u32 pl = pair(pp + r * L.ps + x), pr = pair(pp + r * L.ps + W_ - 2 - x);
                     const u32 org = pair(po + r * L.ps + x) | pair(po + r * L.ps + W_ - 2 - x) << 16;
-                    const u32 rec = lat_pack8((int)(pl & 0xFF) + ((e0[r] + o0[r]) >> 12), (int)(pl >> 8) + ((e1[r] + o1[r]) >> 12),
+                    const u32 rec = pack_sat_u8((int)(pl & 0xFF) + ((e0[r] + o0[r]) >> 12), (int)(pl >> 8) + ((e1[r] + o1[r]) >> 12),
                                               (int)(pr & 0xFF) + ((e1[r] - o1[r]) >> 12), (int)(pr >> 8) + ((e0[r] - o0[r]) >> 12));
                     e = lat_sq4(org, rec, e);
                 }

@@ -6,7 +6,7 @@
 // Affine CUs: com_mc_cu_affine (:361-422) -- sub-block MVs from the control points, luma by the
 // 16-phase 8-tap filters, chroma by the 32-phase 4-tap filters, 1/16-sample positions.
 //
-// One warp per CU; lanes walk the CU's samples in raster order, so every store of the warp is
+// Lanes walk the samples of a CU in raster order, so every store of the lanes of a CU is
 // one contiguous run of the output buffer.
 #include "common.cuh"
 #include "affine.cuh"
@@ -18,6 +18,8 @@
 namespace uc {
 
 constexpr int MC_WARPS = 8;
+// CUs from which a warp takes four: four to each of the 64 warps of an SM, 152 SMs
+constexpr int MC_LONG_LIST = 4 * 64 * 152;
 
 struct McReq {
     s16 x, y; u8 w, h; s8 slot[2]; s16 mv[2][2]; u8 channel; u8 pad[3]; u32 out_offset;
@@ -35,43 +37,56 @@ struct McParams {
 };
 
 // 4-tap chroma filters at the 8 eighth-sample phases (com_tbl_mc_c_coeff, src/com_tables.c)
-__device__ __constant__ static const s8 kMcChroma[8][4] = {
+__device__ __constant__ alignas(4) static const s8 kMcChroma[8][4] = {
     { 0, 64, 0, 0 }, { -4, 62, 6, 0 }, { -6, 56, 15, -1 }, { -5, 47, 25, -3 },
     { -4, 36, 36, -4 }, { -3, 25, 47, -5 }, { -1, 15, 56, -6 }, { 0, 6, 62, -4 },
 };
 
-// one chroma prediction sample: src at the block's integer position (i, j) of the sample
-__device__ __forceinline__ int mc_chroma_sample(const pel *s, int ic, int dx, int dy)
+// Four chroma prediction samples of a row, as bytes, s at the first one's integer position: the two-pass
+// form (horizontal, then vertical sums, (sum + 2048) >> 12) for every phase.  The filter of phase 0 is a
+// factor 64, so this is s[0] at (0, 0) and the one-pass (sum + 32) >> 6 where one phase is 0, exactly, and
+// with a vertical phase of 0 one row is read.  A row's window is seven bytes: two words shifted out of the
+// two or three aligned ones that hold them (no word without a byte of the window is read).
+__device__ __forceinline__ u32 mc_chroma4(const pel *s, int ic, int dx, int dy)
 {
-    if (!dx && !dy) return s[0];
-    if (!dy) {
-        const int v = s[-1] * kMcChroma[dx][0] + s[0] * kMcChroma[dx][1] + s[1] * kMcChroma[dx][2] +
-                      s[2] * kMcChroma[dx][3];
-        return min(255, max(0, (v + 32) >> 6));
-    }
-    if (!dx) {
-        const int v = s[-ic] * kMcChroma[dy][0] + s[0] * kMcChroma[dy][1] + s[ic] * kMcChroma[dy][2] +
-                      s[2 * ic] * kMcChroma[dy][3];
-        return min(255, max(0, (v + 32) >> 6));
-    }
-    // two passes: horizontal into 16 bits (8-bit: no rounding), vertical (sum + 2048) >> 12
-    int v = 0;
+    const u32 ch = *reinterpret_cast<const u32 *>(kMcChroma[dx]);
+    int v[4] = { 2048, 2048, 2048, 2048 };
+    const pel *row = s - 1 + (dy ? -ic : 0);
+    for (int t = dy ? 0 : 1; t < (dy ? 4 : 2); t++, row += ic) {
+        const uintptr_t a = (uintptr_t)row;
+        const u32 sh = (u32)(a & 3) * 8;
+        const u32 *wp = (const u32 *)(a & ~(uintptr_t)3);
+        const u32 m = __ldg(wp + 1), lo = __funnelshift_r(__ldg(wp), m, sh);
+        const u32 hi = __funnelshift_r(m, __ldg(wp + (((a & 3) + 6) >> 2)), sh);
+        const int cv = kMcChroma[dy][t];
 #pragma unroll
-    for (int t = 0; t < 4; t++) {
-        const pel *r = s + (t - 1) * ic;
-        const int hs = r[-1] * kMcChroma[dx][0] + r[0] * kMcChroma[dx][1] + r[1] * kMcChroma[dx][2] +
-                       r[2] * kMcChroma[dx][3];
-        v += (int)(s16)hs * kMcChroma[dy][t];
+        for (int k = 0; k < 4; k++) {
+            int hs;
+            asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(hs) : "r"(__funnelshift_r(lo, hi, 8 * k)), "r"(ch), "r"(0));
+            v[k] += hs * cv;
+        }
     }
-    return min(255, max(0, (v + 2048) >> 12));
+    return pack_sat_u8(v[0] >> 12, v[1] >> 12, v[2] >> 12, v[3] >> 12);
 }
 
-__global__ void __launch_bounds__(32 * MC_WARPS) k_mc_cu(const McParams P)
+// eight bytes from any address
+__device__ __forceinline__ uint2 mc_load8(const pel *s)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * MC_WARPS + warp;
-    if (r >= P.n) return;
-    const McReq q = P.reqs[r];
+    const uintptr_t a = (uintptr_t)s;
+    const u32 *wp = (const u32 *)(a & ~(uintptr_t)3);
+    const u32 sh = (u32)(a & 3) * 8, m = __ldg(wp + 1);
+    return make_uint2(__funnelshift_r(__ldg(wp), m, sh), __funnelshift_r(m, __ldg(wp + 2), sh));
+}
+
+__device__ __forceinline__ void mc_store4(pel *d, u32 v, bool aligned)
+{
+    if (aligned) *(u32 *)d = v;
+    else { d[0] = (pel)v; d[1] = (pel)(v >> 8); d[2] = (pel)(v >> 16); d[3] = (pel)(v >> 24); }
+}
+
+// one CU by `lanes` lanes (a power of two), of which this is number `lane`
+__device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lane, int lanes)
+{
     const int w = q.w, h = q.h, wc = w >> 1, hc = h >> 1;
     const bool luma = q.channel != 2, chroma = q.channel != 1;
     const int nl = (q.slot[0] >= 0) + (q.slot[1] >= 0);
@@ -83,52 +98,78 @@ __global__ void __launch_bounds__(32 * MC_WARPS) k_mc_cu(const McParams P)
         return;
     pel *o = P.out + q.out_offset;
     if (luma) {
-        const pel *src[2];
-        int k = 0;
+        const pel *src[2] = { nullptr, nullptr };
+#pragma unroll
         for (int l = 0; l < 2; l++) {
             if (q.slot[l] < 0) continue;
             const int qx = (q.x << 2) + q.mv[l][0], qy = (q.y << 2) + q.mv[l][1];
             const int px = min(max(qx >> 2, -128 - 4), P.W + 4), py = min(max(qy >> 2, -128 - 4), P.H + 4);
-            src[k++] = P.planes[q.slot[l] * 16 + (qy & 3) * 4 + (qx & 3)] + (long long)py * P.i_ref + px;
+            src[l] = P.planes[q.slot[l] * 16 + (qy & 3) * 4 + (qx & 3)] + (long long)py * P.i_ref + px;
         }
-        // 4 samples a lane: word loads from the (any-alignment) source rows, byte-wise rounded
-        // average of the two lists (pel_avrg), word stores where the output is 4-byte aligned
-        const int lq = 31 - __clz(w >> 2);           // log2 of the words per row
+        const pel *s0 = src[0] ? src[0] : src[1], *s1 = src[0] ? src[1] : nullptr;
+        // byte-wise rounded average of the two lists (pel_avrg), word stores where the output is
+        // 4-byte aligned
+        const int lq = 31 - __clz(w >> 3);           // log2 of the 8-sample pieces per row
         const bool aligned = ((uintptr_t)o & 3) == 0;
-        for (int i = lane; i < (w * h) >> 2; i += 32) {
-            const int j = i >> lq, c = (i - (j << lq)) << 2;
-            u32 v = 0;
-            for (int t = 0; t < k; t++) {
-                const uintptr_t a = (uintptr_t)(src[t] + j * P.i_ref + c);
-                const u32 *wp = (const u32 *)(a & ~(uintptr_t)3);
-                const u32 sv = __funnelshift_r(__ldg(wp), __ldg(wp + 1), (u32)(a & 3) * 8);
-                v = t ? __vavgu4(v, sv) : sv;
+        for (int i = lane; i < (w * h) >> 3; i += lanes) {
+            const int j = i >> lq, c = (i - (j << lq)) << 3;
+            uint2 v = mc_load8(s0 + j * P.i_ref + c);
+            if (s1) {
+                const uint2 b = mc_load8(s1 + j * P.i_ref + c);
+                v = make_uint2(__vavgu4(v.x, b.x), __vavgu4(v.y, b.y));
             }
-            pel *d = o + (i << 2);
-            if (aligned) *(u32 *)d = v;
-            else { d[0] = (pel)v; d[1] = (pel)(v >> 8); d[2] = (pel)(v >> 16); d[3] = (pel)(v >> 24); }
+            mc_store4(o + (i << 3), v.x, aligned);
+            mc_store4(o + (i << 3) + 4, v.y, aligned);
         }
         o += w * h;
     }
     if (chroma) {
-        for (int pl = 0; pl < 2; pl++, o += wc * hc) {
-            const pel *src[2];
-            int dx[2], dy[2], k = 0;
-            for (int l = 0; l < 2; l++) {
-                if (q.slot[l] < 0) continue;
-                const int qx = (q.x << 2) + q.mv[l][0], qy = (q.y << 2) + q.mv[l][1];
-                const int cx = min(max(qx >> 3, -64 - 2), (P.W + 4) >> 1), cy = min(max(qy >> 3, -64 - 2), (P.H + 4) >> 1);
-                dx[k] = qx & 7; dy[k] = qy & 7;
-                src[k++] = P.chroma[q.slot[l] * 2 + pl] + (long long)cy * P.i_c + cx;
-            }
-            const int lwc = 31 - __clz(wc);
-            for (int i = lane; i < wc * hc; i += 32) {
-                const int j = i >> lwc, c = i - (j << lwc);
-                int v = mc_chroma_sample(src[0] + j * P.i_c + c, P.i_c, dx[0], dy[0]);
-                if (k == 2) v = (v + mc_chroma_sample(src[1] + j * P.i_c + c, P.i_c, dx[1], dy[1]) + 1) >> 1;
-                o[i] = (pel)v;
-            }
+        // both planes in one loop
+        const bool aligned = ((uintptr_t)o & 3) == 0;
+        const int lwc = 31 - __clz(wc >> 2), cnt = (wc * hc) >> 2;
+        int dx[2] = { 0, 0 }, dy[2] = { 0, 0 };
+        long long at[2] = { 0, 0 };
+#pragma unroll
+        for (int l = 0; l < 2; l++) {
+            const int qx = (q.x << 2) + q.mv[l][0], qy = (q.y << 2) + q.mv[l][1];
+            const int cx = min(max(qx >> 3, -64 - 2), (P.W + 4) >> 1), cy = min(max(qy >> 3, -64 - 2), (P.H + 4) >> 1);
+            dx[l] = qx & 7; dy[l] = qy & 7;
+            at[l] = (long long)cy * P.i_c + cx;
         }
+        for (int i = lane; i < 2 * cnt; i += lanes) {
+            const int pl = i >= cnt, t = i - pl * cnt, j = t >> lwc, c = (t - (j << lwc)) << 2;
+            u32 v = 0;
+            if (q.slot[0] >= 0) v = mc_chroma4(P.chroma[q.slot[0] * 2 + pl] + at[0] + j * P.i_c + c, P.i_c, dx[0], dy[0]);
+            if (q.slot[1] >= 0) {
+                const u32 b = mc_chroma4(P.chroma[q.slot[1] * 2 + pl] + at[1] + j * P.i_c + c, P.i_c, dx[1], dy[1]);
+                v = q.slot[0] >= 0 ? __vavgu4(v, b) : b;
+            }
+            mc_store4(o + (i << 2), v, aligned);
+        }
+    }
+}
+
+// Bound by instruction issue (the planes' rows come from L2 at any alignment), so a lane forms eight luma
+// samples or four chroma samples at a time.  An 8x8 CU is eight such pieces of luma and eight of chroma:
+// in a long list a warp takes four CUs, at once if all have at most 256 samples (eight lanes each), else
+// in turn.  In a list that one CU a warp does not fill the chip with, a warp takes one (MC_LONG_LIST).
+// The 170,000 CUs of a 1080p frame, two references: 238 us with a lane a luma word or chroma sample,
+// 182 us in pieces, one CU a warp, 152 us four a warp.
+__global__ void __launch_bounds__(32 * MC_WARPS) k_mc_cu(const McParams P, int per_warp)
+{
+    const int wid = blockIdx.x * MC_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (per_warp == 1) {
+        if (wid < P.n) { const McReq q = P.reqs[wid]; mc_cu(P, q, lane, 32); }
+        return;
+    }
+    const int r0 = wid * 4;
+    if (r0 >= P.n) return;
+    const int mine = r0 + (lane >> 3);
+    const bool big = mine < P.n && P.reqs[mine].w * P.reqs[mine].h > 256;
+    const bool split = __any_sync(0xFFFFFFFFu, big);
+    for (int k = 0; k < (split ? 4 : 1); k++) {
+        const int r = split ? r0 + k : mine;
+        if (r < P.n) { const McReq q = P.reqs[r]; mc_cu(P, q, split ? lane : lane & 7, split ? 32 : 8); }
     }
 }
 
@@ -319,7 +360,8 @@ int launch_mc_cu(int W, int H, const pel *const *planes, int n_slots, int i_ref,
     P.i_ref = i_ref; P.i_c = i_c; P.n_slots = n_slots; P.W = W; P.H = H;
     P.reqs = (const McReq *)reqs; P.n = n; P.out = out; P.out_bytes = out_bytes;
     prof_begin(PROF_MC, st);
-    k_mc_cu<<<(unsigned)((n + MC_WARPS - 1) / MC_WARPS), 32 * MC_WARPS, 0, st>>>(P);
+    const int per = n >= MC_LONG_LIST ? 4 : 1;
+    k_mc_cu<<<(unsigned)((n + MC_WARPS * per - 1) / (MC_WARPS * per)), 32 * MC_WARPS, 0, st>>>(P, per);
     UC_CHECK(cudaGetLastError());
     count_launch(1);
     prof_end(PROF_MC, st);
