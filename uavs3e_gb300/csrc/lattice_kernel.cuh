@@ -25,11 +25,6 @@ static const u8 hDqShift[80] = {
     9, 8, 8, 8, 8, 8, 8, 8, 7, 7, 7, 7, 7, 7, 7, 7, 6, 6, 6, 6, 6, 6, 6, 6, 5, 5, 5, 5, 5, 5, 5, 5,
 };
 
-// weight of raster position p in the level hash of a record: odd, spread over 32 bits, so the
-// hash sum_p level[p] * weight(p) (mod 2^32) changes with any single level, any sign and any
-// exchange of two different levels
-__host__ __device__ __forceinline__ constexpr u32 lat_pos_weight(u32 p) { return (p * 0x9E3779B1u + 0x7F4A7C15u) | 1u; }
-
 // sum of 4 (unsigned byte of a) x (signed byte of b) products + c
 __device__ __forceinline__ int dp4a_us(u32 a, u32 b, int c)
 {
@@ -219,8 +214,8 @@ struct LatShared {
     int tables;   // shape class whose matrices and scan table are in place (-1: none)
 };
 
-// lanes [k*seg, (k+1)*seg) of a warp hold one job's elements (seg = 16 or 32): the sum, max
-// or or over the lane's segment, with the warp-wide reduction instructions
+// lanes [k*seg, (k+1)*seg) of a warp hold one job's elements (seg = 16 or 32): the sum or
+// max over the lane's segment, with the warp-wide reduction instructions
 __device__ __forceinline__ u32 seg_sum(u32 v, int seg, int lane)
 {
     if (seg == 32) return __reduce_add_sync(0xFFFFFFFFu, v);
@@ -233,13 +228,6 @@ __device__ __forceinline__ int seg_max(int v, int seg, int lane)
     if (seg == 32) return __reduce_max_sync(0xFFFFFFFFu, v);
     const int lo = __reduce_max_sync(0xFFFFFFFFu, lane < 16 ? v : -1);
     const int hi = __reduce_max_sync(0xFFFFFFFFu, lane < 16 ? -1 : v);
-    return lane < 16 ? lo : hi;
-}
-__device__ __forceinline__ u32 seg_or(u32 v, int seg, int lane)
-{
-    if (seg == 32) return __reduce_or_sync(0xFFFFFFFFu, v);
-    const u32 lo = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? v : 0u);
-    const u32 hi = __reduce_or_sync(0xFFFFFFFFu, lane < 16 ? 0u : v);
     return lane < 16 ? lo : hi;
 }
 
@@ -859,8 +847,11 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         // coefficients or 8, and lanes take consecutive v: the statistics are summed in registers and reduced
         // once per task (with 8 coefficients a task, reductions and indexing were half of the instructions;
         // above 1024 samples a tile holds so few jobs that 8 keep more threads busy).
-        // The position weight of raster position p = v w + u is linear in p but for its lowest bit, and
-        // w and the first column are even: weight = row part + constant of the column.
+        // The level hash of a record is the sum of level x weight(p) mod 2^32 over raster positions
+        // p = v w + u, weight(p) = (K p + 0x7F4A7C15) | 1 with K = 0x9E3779B1: odd and spread over 32 bits, so
+        // the hash changes with any single level, any sign and any exchange of two different levels.  The
+        // weight is linear in p but for its lowest bit, and w and the first column are even: weight = row
+        // part + constant of the column.
         {
             constexpr int CT = W_ * H_ > 1024 ? 8 : 16, RV = CT / RU < KH_ ? CT / RU : KH_, HV = KH_ / RV;
             constexpr int TPJ = HV * NUC, SEG = TPJ < 32 ? TPJ : 32;
