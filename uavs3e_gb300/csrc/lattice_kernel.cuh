@@ -467,7 +467,8 @@ __device__ __forceinline__ u32 lat_pred4(const u32 *tab, const pel *s, const Ipr
     int v[4];
     const bool own = m == 1 || m == 2;                 // their values enter the IPF unclipped
     if (!own) {
-        const uint4 e4 = __ldg(reinterpret_cast<const uint4 *>(tab + (m * H + y) * W + x));
+        // (a list may hold an entry that is no mode: it reads mode 32's row, not past the table)
+        const uint4 e4 = __ldg(reinterpret_cast<const uint4 *>(tab + (min(m, 32) * H + y) * W + x));
         const u32 e[4] = { e4.x, e4.y, e4.z, e4.w };
 #pragma unroll
         for (int k = 0; k < 4; k++) {
