@@ -612,8 +612,9 @@ UAVS3E_CUDA_API int uavs3e_cuda_intra_lattice(const uint8_t *org, int i_org, con
                                               const int *qps, int n_qp, int is_intra_slice, uint32_t *satd,
                                               uavs3e_cuda_lat_q_t *q);
 /* The same over a subset of modes: d_modes holds n_modes mode indices (0..32) per CU
- * ([n_cus][n_modes], device); only those (CU, mode) records are written.  Used by the pruned
- * search, which evaluates a shortlist of modes per CU. */
+ * ([n_cus][n_modes], device); only those (CU, mode) records are written.  An entry above 32 (an
+ * empty slot of a candidate list, byte 255, or the IPCM index 33) writes no record.  Used by the
+ * pruned search, which evaluates a shortlist of modes per CU. */
 UAVS3E_CUDA_API int uavs3e_cuda_intra_lattice_modes_device(const uint8_t *d_org, int i_org, const uint8_t *d_rec,
                                                            int i_rec, int width, int height,
                                                            const uavs3e_cuda_cu_t *d_cus, int n_cus,

@@ -77,3 +77,46 @@ def test_lattice_satd_only(gpu, oracle, n_modes):
     at = (np.arange(n)[:, None] * 33 + modes).ravel()
     want[at] = satd_o.ravel()[at]
     assert np.array_equal(d_satd.cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("n_qp", [0, 1, 3])
+def test_lattice_list_entries_that_are_no_modes(gpu, oracle, n_qp):
+    # empty slots (255) and IPCM (33) of candidate lists write no record: every record of a listed mode is
+    # right, every other word of the buffers, and the words behind them, keep what they held
+    import torch
+    W, H, n_modes, guard, qps = 72, 64, 5, 2048, np.array([24, 41, 34][:n_qp], np.int32)
+    org, rec = _frames(W, H, 90 + n_qp, 6)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    satd_o, q_o = oracle_lattice(oracle, org, rec, cus, 1, list(qps) if n_qp else [32])
+    rng = np.random.default_rng(90 + n_qp)
+    modes = np.stack([rng.permutation(33)[:n_modes] for _ in range(n)]).astype(np.uint8)
+    drop = rng.random(modes.shape) < 0.3
+    drop[-1], drop[-2] = True, [True, False, True, True, False]        # the last CU has no mode at all
+    modes[drop] = rng.choice(np.array([33, 34, 128, 255], np.uint8), int(drop.sum()))
+    modes[-1, :2] = 255, 33
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8), modes)]
+    words = gpu.LAT_Q.itemsize // 4
+    d_satd = torch.full((n * 33 + guard,), -7, dtype=torch.int32, device="cuda")
+    d_q = torch.full(((n * 33 * n_qp + guard) * words,), -7, dtype=torch.int32, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_modes_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, d[3].data_ptr(), n_modes, 1,
+        qps.ctypes.data if n_qp else None, n_qp, 1, d_satd.data_ptr(), d_q.data_ptr() if n_qp else None,
+        torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    cu, slot = np.nonzero(~drop)
+    at = cu * 33 + modes[cu, slot]
+    want = np.full(n * 33 + guard, -7, np.int32)
+    want[at] = satd_o.ravel().astype(np.uint32).view(np.int32)[at]
+    assert np.array_equal(d_satd.cpu().numpy(), want)
+    if n_qp:
+        want_q = np.full((n * 33 + guard, n_qp * words), -7, np.int32)[:n * 33]
+        got = d_q.cpu().numpy()
+        assert (got[n * 33 * n_qp * words:] == -7).all()
+        got = got[:n * 33 * n_qp * words].reshape(n * 33, n_qp * words)
+        keep = np.zeros(n * 33, bool)
+        keep[at] = True
+        assert np.array_equal(got[~keep], want_q[~keep])
+        rec_g, rec_o = np.ascontiguousarray(got[keep]).view(gpu.LAT_Q), q_o.reshape(n * 33, n_qp)[keep]
+        for f in FIELDS:
+            assert np.array_equal(rec_g[f], rec_o[f]), f

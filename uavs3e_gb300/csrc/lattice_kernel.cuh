@@ -59,6 +59,7 @@ constexpr int LAT_MAX_G = 8;            // CUs per CTA
 constexpr int LAT_MAX_JOBS = 132;       // (CU, mode) jobs of a tile: 4 CUs of 33 modes
 constexpr int LAT_NB = 592;             // neighbour buffer per CU (INTRA_NEIB_SIZE + pad)
 constexpr int LAT_SHAPES = 25;          // log2 sides 2..6
+constexpr int LAT_NO_MODE = 33;         // a list entry that is no mode (above 32): a job without records
 
 // shared-memory layout of one shape's CTAs (host and device compute it the same way)
 struct LatLayout {
@@ -467,7 +468,7 @@ __device__ __forceinline__ u32 lat_pred4(const u32 *tab, const pel *s, const Ipr
     int v[4];
     const bool own = m == 1 || m == 2;                 // their values enter the IPF unclipped
     if (!own) {
-        // (a list may hold an entry that is no mode: it reads mode 32's row, not past the table)
+        // (LAT_NO_MODE reads mode 32's row, not past the table)
         const uint4 e4 = __ldg(reinterpret_cast<const uint4 *>(tab + (min(m, 32) * H + y) * W + x));
         const u32 e[4] = { e4.x, e4.y, e4.z, e4.w };
 #pragma unroll
@@ -634,7 +635,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     if (tid < Gv) S.cu[tid] = lat_perm(perm + cu0 + tid);
     for (int j = tid; j < J; j += LAT_THREADS) {
         const int g = JG(j), mi = m0 + (j - g * MCv);
-        s_mode[j] = P.modes ? P.modes[(size_t)lat_perm(perm + cu0 + g).id * P.n_modes + mi] : (u8)mi;
+        // (a record is stored at its mode: an entry above 32 would fall into other CUs' records)
+        s_mode[j] = (u8)(P.modes ? min((int)P.modes[(size_t)lat_perm(perm + cu0 + g).id * P.n_modes + mi], LAT_NO_MODE) : mi);
         s_satd[j] = 0; s_flag[j] = 0; S.ssd0[j] = 0;
     }
     LAT_STAGE(0);
@@ -818,7 +820,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     }
     __syncthreads(); LAT_STAGE(5);
     for (int j = tid; j < J; j += LAT_THREADS)
-        P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
+        if (s_mode[j] != LAT_NO_MODE) P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
 
     // levels and magnitudes of a block of at most 256 coefficients go into one word, the count from bit 23
     constexpr bool PACK = KW_ * KH_ <= 256, CHUNKS = KW_ > 8 || KH_ > 8;
@@ -1067,6 +1069,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         else inv_row(std::integral_constant<int, 4>{});
         __syncthreads(); LAT_STAGE(8);
         for (int j = tid; j < J; j += LAT_THREADS) {
+            if (s_mode[j] == LAT_NO_MODE) continue;
             LatQ o;
             o.ssd = (s_flag[j] >> q) & 1 ? S.ssd[j] : S.ssd0[j];
             o.coef_hash = S.hash[j];
