@@ -80,3 +80,125 @@ def test_coef_rate_chain_lengths_on_two_streams(gpu, oracle):
     torch.cuda.synchronize()
     for (lv, rq), (keep, out) in zip(sets, got):
         assert out.cpu().numpy().tobytes() == oracle.coef_rate(lv, rq).tobytes()
+
+
+def _rdoq_device(gpu, reqs, ests, coefs, stream=None, est_shift=0):
+    """the call on device copies; the estimates start est_shift bytes off a 256-byte boundary"""
+    import torch
+    e = np.ascontiguousarray(ests).view(np.uint8).reshape(-1)
+    d_e = torch.zeros(len(e) + 256, dtype=torch.uint8, device="cuda")
+    d_e[est_shift:est_shift + len(e)] = torch.from_numpy(e.copy()).cuda()
+    d_r = torch.from_numpy(np.ascontiguousarray(reqs).view(np.uint8).reshape(-1).copy()).cuda()
+    d_c = torch.from_numpy(coefs.copy()).cuda()
+    nz = torch.zeros(len(reqs), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    gpu.rdoq_device(d_r.data_ptr(), len(reqs), d_e.data_ptr() + est_shift, len(ests), d_c.data_ptr(), coefs.size,
+                    nz.data_ptr(), stream)
+    return d_c, nz, (d_e, d_r)
+
+
+def _check_rdoq(oracle, reqs, ests, coefs, d_c, nz):
+    want_c = coefs.copy()
+    want = oracle.rdoq(reqs, ests, want_c)
+    assert np.array_equal(nz.cpu().numpy(), want)
+    assert np.array_equal(d_c.cpu().numpy(), want_c)
+
+
+class _Graph:
+    """what a capture of `calls` on a stream gives, by the driver's own interface"""
+
+    def __init__(self, stream, calls):
+        import ctypes
+        self.c, self.L, self.execs = ctypes, ctypes.CDLL("libcuda.so.1"), []
+        self.handle = ctypes.c_void_p()
+        self.ok(self.L.cuStreamBeginCapture_v2(ctypes.c_void_p(stream), 0))
+        calls()
+        self.ok(self.L.cuStreamEndCapture(ctypes.c_void_p(stream), ctypes.byref(self.handle)))
+
+    def ok(self, rc):
+        assert rc == 0, f"CUDA driver error {rc}"
+
+    def instantiate(self, graph=None):
+        e = self.c.c_void_p()
+        self.ok(self.L.cuGraphInstantiateWithFlags(self.c.byref(e), graph or self.handle, self.c.c_ulonglong(0)))
+        self.execs.append(e)
+        return e
+
+    def launch(self, e, stream):
+        self.ok(self.L.cuGraphLaunch(e, self.c.c_void_p(stream)))
+
+    def parent(self):
+        """a graph with this one as its only, child, node"""
+        g, node = self.c.c_void_p(), self.c.c_void_p()
+        self.ok(self.L.cuGraphCreate(self.c.byref(g), 0))
+        self.ok(self.L.cuGraphAddChildGraphNode(self.c.byref(node), g, None, self.c.c_size_t(0), self.handle))
+        return g
+
+    def destroy(self, *graphs):
+        for e in self.execs:
+            self.ok(self.L.cuGraphExecDestroy(e))
+        for g in graphs:
+            self.ok(self.L.cuGraphDestroy(g))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", (3, 600))
+def test_captured_block_lists(gpu, oracle, n):
+    # one capture of both calls, replayed on new blocks by two executables of the graph and as a child of
+    # another graph, after the captured one itself is gone
+    import torch
+    rd = [cases.rdoq_inputs(oracle, dict(n=n, k=2), 4600 + n)]
+    for k in range(3):
+        r, e, c = rd[0]
+        rng = np.random.default_rng(k)
+        rd.append((r, e, np.clip(c.astype(int) * rng.choice([-1, 1], c.size) + rng.integers(-3, 4, c.size), -32768, 32767).astype(np.int16)))
+    levels, rreqs = cases.coef_rate_inputs(np.random.default_rng(700 + n), n)
+    d_c, nz, keep = _rdoq_device(gpu, *rd[0])                          # tables and pools exist from here on
+    d_e, d_r = keep
+    rate_keep, rate = _rate_device(gpu, levels, rreqs)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    st = s.cuda_stream
+
+    def calls():
+        gpu.rdoq_device(d_r.data_ptr(), n, d_e.data_ptr(), 2, d_c.data_ptr(), rd[0][2].size, nz.data_ptr(), st)
+        gpu.coef_rate_device(rate_keep[1].data_ptr(), n, rate_keep[0].data_ptr(), levels.size, rate.data_ptr(), st)
+
+    g = _Graph(st, calls)
+    want_rate = oracle.coef_rate(levels, rreqs).tobytes()
+    parent = g.parent()
+    runs = [g.instantiate(), g.instantiate(), g.instantiate(parent)]
+    g.ok(g.L.cuGraphDestroy(g.handle))
+    for (r, e, c), x in zip(rd[1:], runs):
+        d_c.copy_(torch.from_numpy(c))
+        nz.fill_(-5)
+        rate.zero_()
+        torch.cuda.synchronize()
+        g.launch(x, st)
+        # a call outside the graph while it runs
+        other, onz, okeep = _rdoq_device(gpu, *rd[0])
+        torch.cuda.synchronize()
+        _check_rdoq(oracle, r, e, c, d_c, nz)
+        _check_rdoq(oracle, *rd[0], other, onz)
+        assert rate.cpu().numpy().tobytes() == want_rate
+    g.destroy(parent)
+
+
+@pytest.mark.gpu
+def test_captured_workspaces_are_given_back(gpu, oracle):
+    import torch
+    reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=8, k=1), 4700)
+    coefs = np.concatenate([coefs, np.zeros((8 << 20) - coefs.size, np.int16)])     # 32 MB of workspace a call
+    d_c, nz, (d_e, d_r) = _rdoq_device(gpu, reqs, ests, coefs)
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    free = []
+    for k in range(48):
+        g = _Graph(s.cuda_stream, lambda: gpu.rdoq_device(d_r.data_ptr(), 8, d_e.data_ptr(), 1, d_c.data_ptr(), coefs.size,
+                                                          nz.data_ptr(), s.cuda_stream))
+        x = g.instantiate()
+        g.launch(x, s.cuda_stream)
+        torch.cuda.synchronize()
+        g.destroy(g.handle)
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[7] - free[-1] < 512 << 20, (free[7], free[-1])           # 40 calls' blocks would be 1.3 GB

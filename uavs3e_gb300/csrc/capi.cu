@@ -7,6 +7,7 @@
 
 #include <cudaTypedefs.h>
 #include <mutex>
+#include <new>
 #include <stdio.h>
 #include <string.h>
 #include <vector>
@@ -44,39 +45,131 @@ int ensure_init()
     return uavs3e_cuda_init(0);
 }
 
-// One memory pool per device for the calls' workspaces.  The device's default pool gives its memory
-// back at every synchronisation, so a call after one maps it anew (0.28 ms for 155 MB); this one
-// keeps up to WORK_POOL_KEEP bytes.  Allocations and frees follow the stream's order, so calls on
-// several streams or threads never share a block that is in use.
+// Workspaces of calls.  One memory pool per device: the device's default pool gives its memory back at
+// every synchronisation, so a call after one maps it anew (0.28 ms for 155 MB); this one keeps up to
+// WORK_POOL_KEEP bytes.  Allocations and frees follow the stream's order, so calls on several streams or
+// threads never share a block that is in use.
+//
+// A captured call's workspace is not a memory node: a graph with memory nodes can neither be a child of
+// another nor be instantiated twice.  It is a block of the same pool, allocated on the device's own stream
+// and held by a user object of the graph, so that it lives as long as the graph, its copies and their
+// executables do.  The object's destructor may not call CUDA: it hands the block to the `retired` list,
+// which the next call on the device gives back.
+namespace {
+struct WorkBlock { void *p; int dev; WorkBlock *next; };
+struct WorkPools {
+    std::mutex mu;
+    cudaMemPool_t pool[64] = {};
+    cudaStream_t own[64] = {};
+    std::mutex retired_mu;             // no CUDA call is made under it: the destructor takes it
+    WorkBlock *retired = nullptr;
+};
+// never destroyed: a graph may outlive the library's static objects
+WorkPools &work_pools()
+{
+    static WorkPools *w = new WorkPools;
+    return *w;
+}
+
+void CUDART_CB work_retire(void *block)
+{
+    WorkPools &W = work_pools();
+    WorkBlock *b = (WorkBlock *)block;
+    std::lock_guard<std::mutex> lk(W.retired_mu);
+    b->next = W.retired;
+    W.retired = b;
+}
+
+// calls that a capture under way on the thread would otherwise refuse (they touch no capturing stream)
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// the device's pool and stream, and the blocks of graphs that are gone given back
+int work_open(int dev, cudaMemPool_t *pool, cudaStream_t *own)
+{
+    WorkPools &W = work_pools();
+    std::lock_guard<std::mutex> lk(W.mu);
+    if (!W.pool[dev]) {
+        RelaxedCapture relaxed;
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        if (!W.own[dev]) UC_CHECK(cudaStreamCreateWithFlags(&W.own[dev], cudaStreamNonBlocking));
+        cudaMemPool_t p;
+        UC_CHECK(cudaMemPoolCreate(&p, &props));
+        uint64_t keep = WORK_POOL_KEEP;
+        UC_CHECK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+        W.pool[dev] = p;
+    }
+    *pool = W.pool[dev];
+    *own = W.own[dev];
+    WorkBlock *mine = nullptr;
+    {
+        std::lock_guard<std::mutex> lr(W.retired_mu);
+        for (WorkBlock **at = &W.retired; *at;) {
+            WorkBlock *b = *at;
+            if (b->dev != dev) { at = &b->next; continue; }
+            *at = b->next;
+            b->next = mine;
+            mine = b;
+        }
+    }
+    while (mine) {
+        WorkBlock *b = mine;
+        mine = b->next;
+        RelaxedCapture relaxed;
+        cudaFreeAsync(b->p, *own);
+        delete b;
+    }
+    return UC_OK;
+}
+}  // namespace
+
 int work_alloc(void **p, size_t bytes, cudaStream_t st)
 {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     int dev = 0;
     UC_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return set_status(UC_ERR_UNSUPPORTED, "workspace: device index");
     cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!pools[dev]) {
-            cudaMemPoolProps props;
-            memset(&props, 0, sizeof(props));
-            props.allocType = cudaMemAllocationTypePinned;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            UC_CHECK(cudaMemPoolCreate(&pool, &props));
-            uint64_t keep = WORK_POOL_KEEP;
-            UC_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-            pools[dev] = pool;
-        }
-        pool = pools[dev];
+    cudaStream_t own;
+    int rc = work_open(dev, &pool, &own);
+    if (rc) return rc;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    UC_CHECK(cudaStreamGetCaptureInfo(st, &cap, nullptr, &graph));
+    if (cap == cudaStreamCaptureStatusNone) {
+        UC_CHECK(cudaMallocFromPoolAsync(p, bytes, pool, st));
+        return UC_OK;
     }
-    UC_CHECK(cudaMallocFromPoolAsync(p, bytes, pool, st));
+    if (cap != cudaStreamCaptureStatusActive) return check_cuda(cudaErrorStreamCaptureInvalidated, "workspace: capture");
+    RelaxedCapture relaxed;
+    UC_CHECK(cudaMallocFromPoolAsync(p, bytes, pool, own));
+    cudaError_t e = cudaStreamSynchronize(own);         // any stream may use it from here on
+    WorkBlock *b = new (std::nothrow) WorkBlock{ *p, dev, nullptr };
+    cudaUserObject_t obj = nullptr;
+    if (e == cudaSuccess && !b) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = cudaUserObjectCreate(&obj, b, work_retire, 1, cudaUserObjectNoDestructorSync);
+    if (obj) {
+        e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) cudaUserObjectRelease(obj, 1);   // its destructor retires the block
+    } else {
+        delete b;
+        cudaFreeAsync(*p, own);
+    }
+    UC_CHECK(e);
     return UC_OK;
 }
 
 int work_free(void *p, cudaStream_t st)
 {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    UC_CHECK(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return UC_OK;      // the graph's
     UC_CHECK(cudaFreeAsync(p, st));
     return UC_OK;
 }
