@@ -104,6 +104,27 @@ def _check_rdoq(oracle, reqs, ests, coefs, d_c, nz):
     assert np.array_equal(d_c.cpu().numpy(), want_c)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("est_shift", (0, 4, 8))
+def test_rdoq_estimates_off_16_bytes(gpu, oracle, est_shift):
+    import torch
+    reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=70, k=3), 4400)
+    d_c, nz, keep = _rdoq_device(gpu, reqs, ests, coefs, est_shift=est_shift)
+    torch.cuda.synchronize()
+    _check_rdoq(oracle, reqs, ests, coefs, d_c, nz)
+
+
+@pytest.mark.gpu
+def test_rdoq_lists_on_two_streams(gpu, oracle):
+    import torch
+    sets = [cases.rdoq_inputs(oracle, dict(n=n, k=2), 4500 + n) for n in (200, 3, 90, 257)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [_rdoq_device(gpu, *s, stream=streams[k % 2].cuda_stream) for k, s in enumerate(sets)]
+    torch.cuda.synchronize()
+    for s, (d_c, nz, keep) in zip(sets, got):
+        _check_rdoq(oracle, *s, d_c, nz)
+
+
 class _Graph:
     """what a capture of `calls` on a stream gives, by the driver's own interface"""
 
