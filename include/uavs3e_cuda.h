@@ -542,12 +542,13 @@ typedef struct {
 /* The lattice of a call is one persistent launch walking a device queue of tiles (a tile =
  * several whole CUs of one shape, or one CU and a chunk of its modes), largest shapes first,
  * with no wait on the host between its launches: once the layouts are tuned, a call can be
- * captured into a CUDA graph.  Layout autotuning (on by default): the first call with QPs per
- * device and mode count times, for every shape with at least 512 CUs, the tile layouts given by
- * shared-memory budgets of 16..50 KB on the queue restricted to that shape and keeps the
- * fastest (that call waits for the GPU; make it before any capture); records are the same for
- * every layout.  budgets: per shape (log2 w - 2) * 5 + (log2 h - 2), in bytes, 0 = the default
- * 50 KB (not tuned). */
+ * captured into a CUDA graph.  Layout autotuning (on by default): the first call with one QP, and
+ * the first with more, per device and mode count times, for every shape with at least 512 CUs, the
+ * tile layouts given by shared-memory budgets of 16..50 KB on the queue restricted to that shape
+ * and keeps the fastest (that call waits for the GPU; a captured call does not tune and takes the
+ * default where nothing is tuned); records are the same for every layout.  budgets: per shape
+ * (log2 w - 2) * 5 + (log2 h - 2), in bytes, 0 = the default 50 KB (not tuned); those of calls with
+ * several QPs once such a call has tuned, else those of calls with one. */
 UAVS3E_CUDA_API void uavs3e_cuda_lattice_autotune(int on);
 UAVS3E_CUDA_API int uavs3e_cuda_lattice_budgets(int n_modes, int out[25]);
 

@@ -120,3 +120,45 @@ def test_lattice_list_entries_that_are_no_modes(gpu, oracle, n_qp):
         rec_g, rec_o = np.ascontiguousarray(got[keep]).view(gpu.LAT_Q), q_o.reshape(n * 33, n_qp)[keep]
         for f in FIELDS:
             assert np.array_equal(rec_g[f], rec_o[f]), f
+
+
+@pytest.mark.parametrize("n_modes,first", [(29, 1), (30, 2)])
+def test_lattice_layouts_are_tuned_per_kind(gpu, n_modes, first):
+    # calls of one QP and of several have different tile layouts: each kind tunes with its own first call
+    # (told by the launches it takes: 4 of a tuned call), and a captured call tunes nothing
+    import torch
+    W, H = 136, 104
+    org, rec = _frames(W, H, n_modes, 5)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    modes = np.stack([np.random.default_rng(k).permutation(33)[:n_modes] for k in range(n)]).astype(np.uint8)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8), modes)]
+    stream = torch.cuda.Stream()
+
+    def buffers():
+        return (torch.zeros(n * 33, dtype=torch.int32, device="cuda"),
+                torch.zeros(n * 33 * 2 * gpu.LAT_Q.itemsize, dtype=torch.uint8, device="cuda"))
+
+    def call(n_qp, out):
+        before = gpu.lib().uavs3e_cuda_launch_count()
+        qps = np.array([27, 36][:n_qp], np.int32)
+        gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_modes_device(
+            d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, d[3].data_ptr(), n_modes, 1, qps.ctypes.data,
+            n_qp, 1, out[0].data_ptr(), out[1].data_ptr(), stream.cuda_stream), "intra_lattice")
+        return gpu.lib().uavs3e_cuda_launch_count() - before
+
+    second = 3 - first
+    plain, cap = {k: buffers() for k in (1, 2)}, buffers()
+    torch.cuda.synchronize()
+    assert call(first, plain[first]) > 4 and call(first, plain[first]) == 4
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=stream):
+        assert call(second, cap) == 4
+    g.replay()
+    torch.cuda.synchronize()
+    assert call(second, plain[second]) > 4 and call(second, plain[second]) == 4
+    assert call(first, plain[first]) == 4
+    torch.cuda.synchronize()
+    assert any(gpu.lattice_budgets(n_modes))
+    assert torch.equal(cap[0], plain[second][0]) and torch.equal(cap[1], plain[second][1])

@@ -203,16 +203,18 @@ int lattice_tables(DevTables &t)
     return UC_OK;
 }
 
-// Autotuning of the tile layouts: per device and mode count, the first call with at least
-// LAT_TUNE_MIN_CUS CUs of a class times the queue restricted to that class for each distinct
-// layout the candidate budgets give (every run writes the same records) and keeps the fastest.
+// Autotuning of the tile layouts: per device, mode count and layout kind (one QP, or more: a job of one
+// QP has half the buffers, so a budget that suits one kind can be half a tile of the other), the first
+// call with QPs times, for each class of at least LAT_TUNE_MIN_CUS CUs, the queue restricted to that class
+// for each distinct layout the candidate budgets give (every run writes the same records) and keeps the
+// fastest.
 // All budgets are at most LAT_BUDGET, the launch's shared-memory size, so four CTAs share an SM.
 constexpr int LAT_TUNE_MIN_CUS = 512;
 static const int kLatBudgets[] = { 16 * 1024, 24 * 1024, 32 * 1024, 40 * 1024, LAT_BUDGET };
 struct LatTune {
     std::mutex mu;
-    int budget[34][LAT_SHAPES] = {};   // 0: the default LAT_BUDGET (not tuned)
-    bool done[34] = {};                // the tuning pass of this mode count has run
+    int budget[34][2][LAT_SHAPES] = {};   // [mode count][more than one QP]; 0: the default LAT_BUDGET (not tuned)
+    bool done[34][2] = {};             // the tuning pass of this mode count and kind has run
 };
 static LatTune g_tune[64];
 static bool g_tune_on = true;
@@ -342,25 +344,30 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
     P.images = tab->lat_images; P.ipred = tab->lat_ipred;
     P.counts = S.counters; P.cu_off = S.counters + 64; P.tile_off = S.counters + 96; P.perm = S.perm;
     P.next = S.counters + 127;
-    // the classes' layouts: tuned on the first call with QPs per device and mode count (that call
-    // waits for the CU counts and times the candidates of every class with enough CUs; later
-    // calls, and every SATD-only call, do not wait -- make the first call before any capture)
+    // the classes' layouts: tuned on the first call with QPs per device, mode count and layout kind (that
+    // call waits for the CU counts and times the candidates of every class with enough CUs; later
+    // calls, every SATD-only call and captured calls, which take the default where nothing is tuned,
+    // do not wait)
     int budgets[LAT_SHAPES];
     {
         LatTune &T = g_tune[dev];
         std::lock_guard<std::mutex> lk(T.mu);
-        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = n_qp > 0 && T.budget[n_modes][c] ? T.budget[n_modes][c] : LAT_BUDGET;
-        if (g_tune_on && !T.done[n_modes] && n_qp > 0) {
-            T.done[n_modes] = true;   // one pass: classes with too few CUs keep the default
+        const int kind = n_qp > 1;
+        int *tuned = T.budget[n_modes][kind];
+        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = n_qp > 0 && tuned[c] ? tuned[c] : LAT_BUDGET;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0) UC_CHECK(cudaStreamIsCapturing(st, &cap));
+        if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0 && cap == cudaStreamCaptureStatusNone) {
+            T.done[n_modes][kind] = true;   // one pass: classes with too few CUs keep the default
             int counts[32];
             UC_CHECK(cudaMemcpyAsync(counts, S.counters, 32 * sizeof(int), cudaMemcpyDeviceToHost, st));
             UC_CHECK(cudaStreamSynchronize(st));
             for (int c = 0; c < LAT_SHAPES; c++) {
-                if (T.budget[n_modes][c] || counts[c] < LAT_TUNE_MIN_CUS) continue;
+                if (tuned[c] || counts[c] < LAT_TUNE_MIN_CUS) continue;
                 int best = LAT_BUDGET;
                 int r = lat_tune_class(c, P, cus, n_cus, W, H, budgets, S, st, &launches, &best);
                 if (r) return r;
-                T.budget[n_modes][c] = budgets[c] = best;
+                tuned[c] = budgets[c] = best;
             }
         }
     }
@@ -419,7 +426,7 @@ UAVS3E_CUDA_API int uavs3e_cuda_lattice_budgets(int n_modes, int out[25])
     if (dev < 0 || dev >= 64) return set_status(UC_ERR_UNSUPPORTED, "lattice_budgets: device index");
     LatTune &T = g_tune[dev];
     std::lock_guard<std::mutex> lk(T.mu);
-    for (int c = 0; c < 25; c++) out[c] = T.budget[n_modes][c];
+    for (int c = 0; c < 25; c++) out[c] = T.budget[n_modes][T.done[n_modes][1]][c];
     return UC_OK;
 }
 
