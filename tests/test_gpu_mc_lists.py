@@ -31,3 +31,26 @@ def test_affine_output_alignment(gpu, oracle, shift):
     nbytes += shift
     want = oracle.mc_affine(p["w"], p["h"], luma[1], luma[2], chroma[1], chroma[2], reqs, nbytes)
     assert np.array_equal(want, _gpu_affine(gpu, p, luma, chroma, reqs, nbytes))
+
+
+@pytest.mark.parametrize("extra,big_at", [(-1, ()), (0, ()), (0, (0, 31, 32, 95, 1000)), (33, (70,)), (7, "last")])
+def test_mc_small_cus_in_long_lists(gpu, oracle, extra, big_at):
+    # CUs of at most 256 samples, grouped by 32 from the device's list length on: lists one short of it, at
+    # it and not a multiple of 32 past it, groups broken by one larger CU or by a request that is skipped
+    import torch
+    p = cases.MC_CASES[0]
+    n = 256 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    luma, chroma, reqs, _ = cases.mc_inputs(oracle, dict(p, n=6000), 79)
+    area = reqs["w"].astype(int) * reqs["h"]
+    small, big = reqs[(area <= 256) & (area > 0)], reqs[area > 256]
+    reqs = small[np.random.default_rng(n).integers(0, len(small), n)].copy()
+    for k in (n - 1,) if big_at == "last" else big_at:
+        reqs[k] = big[k % len(big)]
+    size = np.where(reqs["channel"] == 0, 3, np.where(reqs["channel"] == 1, 2, 1)) * reqs["w"].astype(int) * reqs["h"] // 2
+    reqs["out_offset"] = np.cumsum(size) - size
+    nbytes = int(size.sum())
+    keep = np.ones(n, bool)
+    if big_at:
+        reqs["x"][200], keep[200] = -8, False            # outside the domain: nothing written
+    want = oracle.mc_cu(p["w"], p["h"], luma[1], luma[2], chroma[1], chroma[2], reqs[keep], nbytes)
+    assert np.array_equal(want, _gpu_mc(gpu, p, luma, chroma, reqs, nbytes))

@@ -18,8 +18,10 @@
 namespace uc {
 
 constexpr int MC_WARPS = 8;
-// CUs from which a warp takes four: four to each of the 64 warps of an SM, 152 SMs
-constexpr int MC_LONG_LIST = 4 * 64 * 152;
+// CUs per SM from which k_mc_cu groups small CUs: lists of CUs of at most 256 samples take the same time
+// either way at 38,912 CUs on 152 SMs (25 us); 10,000 take 11 us ungrouped and 17 grouped, 100,000 take
+// 58 and 53
+constexpr int MC_GROUP_PER_SM = 256;
 
 struct McReq {
     s16 x, y; u8 w, h; s8 slot[2]; s16 mv[2][2]; u8 channel; u8 pad[3]; u32 out_offset;
@@ -46,12 +48,14 @@ __device__ __constant__ alignas(4) static const s8 kMcChroma[8][4] = {
 // form (horizontal, then vertical sums, (sum + 2048) >> 12) for every phase.  The filter of phase 0 is a
 // factor 64, so this is s[0] at (0, 0) and the one-pass (sum + 32) >> 6 where one phase is 0, exactly, and
 // with a vertical phase of 0 one row is read.  A row's window is seven bytes: two words shifted out of the
-// two or three aligned ones that hold them (no word without a byte of the window is read).
+// two or three aligned ones that hold them (no word without a byte of the window is read).  The rows'
+// loads are in flight together.
 __device__ __forceinline__ u32 mc_chroma4(const pel *s, int ic, const s8 (*filter)[4], int dx, int dy)
 {
     const u32 ch = *reinterpret_cast<const u32 *>(filter[dx]);
     int v[4] = { 2048, 2048, 2048, 2048 };
     const pel *row = s - 1 + (dy ? -ic : 0);
+#pragma unroll 4
     for (int t = dy ? 0 : 1; t < (dy ? 4 : 2); t++, row += ic) {
         const uintptr_t a = (uintptr_t)row;
         const u32 sh = (u32)(a & 3) * 8;
@@ -84,7 +88,8 @@ __device__ __forceinline__ void mc_store4(pel *d, u32 v, bool aligned)
     else { d[0] = (pel)v; d[1] = (pel)(v >> 8); d[2] = (pel)(v >> 16); d[3] = (pel)(v >> 24); }
 }
 
-// one CU by `lanes` lanes (a power of two), of which this is number `lane`
+// one CU by `lanes` lanes (a power of two), of which this is number `lane`, U luma pieces of a lane in flight
+template <int U>
 __device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lane, int lanes)
 {
     const int w = q.w, h = q.h, wc = w >> 1, hc = h >> 1;
@@ -111,15 +116,25 @@ __device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lan
         // 4-byte aligned
         const int lq = 31 - __clz(w >> 3);           // log2 of the 8-sample pieces per row
         const bool aligned = ((uintptr_t)o & 3) == 0;
-        for (int i = lane; i < (w * h) >> 3; i += lanes) {
-            const int j = i >> lq, c = (i - (j << lq)) << 3;
-            uint2 v = mc_load8(s0 + j * P.i_ref + c);
-            if (s1) {
-                const uint2 b = mc_load8(s1 + j * P.i_ref + c);
-                v = make_uint2(__vavgu4(v.x, b.x), __vavgu4(v.y, b.y));
+        const int n8 = (w * h) >> 3;
+#pragma unroll 1
+        for (int i0 = lane; i0 < n8; i0 += U * lanes) {
+            uint2 v[U], b[U];
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = i0 + k * lanes, j = i >> lq, c = (i - (j << lq)) << 3;
+                if (i >= n8) break;
+                v[k] = mc_load8(s0 + j * P.i_ref + c);
+                if (s1) b[k] = mc_load8(s1 + j * P.i_ref + c);
             }
-            mc_store4(o + (i << 3), v.x, aligned);
-            mc_store4(o + (i << 3) + 4, v.y, aligned);
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int i = i0 + k * lanes;
+                if (i >= n8) break;
+                if (s1) v[k] = make_uint2(__vavgu4(v[k].x, b[k].x), __vavgu4(v[k].y, b[k].y));
+                mc_store4(o + (i << 3), v[k].x, aligned);
+                mc_store4(o + (i << 3) + 4, v[k].y, aligned);
+            }
         }
         o += w * h;
     }
@@ -136,6 +151,7 @@ __device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lan
             dx[l] = qx & 7; dy[l] = qy & 7;
             at[l] = (long long)cy * P.i_c + cx;
         }
+#pragma unroll 1
         for (int i = lane; i < 2 * cnt; i += lanes) {
             const int pl = i >= cnt, t = i - pl * cnt, j = t >> lwc, c = (t - (j << lwc)) << 2;
             u32 v = 0;
@@ -149,28 +165,33 @@ __device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lan
     }
 }
 
-// Bound by instruction issue (the planes' rows come from L2 at any alignment), so a lane forms eight luma
-// samples or four chroma samples at a time.  An 8x8 CU is eight such pieces of luma and eight of chroma:
-// in a long list a warp takes four CUs, at once if all have at most 256 samples (eight lanes each), else
-// in turn.  In a list that one CU a warp does not fill the chip with, a warp takes one (MC_LONG_LIST).
-// The 170,000 CUs of a 1080p frame, two references: 238 us with a lane a luma word or chroma sample,
-// 182 us in pieces, one CU a warp, 152 us four a warp.
-__global__ void __launch_bounds__(32 * MC_WARPS) k_mc_cu(const McParams P, int per_warp)
+// Bound by the loads' latency and by instruction issue (the planes' rows come from L2 at any alignment), so a
+// lane forms eight luma samples or four chroma samples at a time, a warp to a CU, with four pieces of luma
+// or four rows of chroma in flight: 1,000 CUs of more than 256 samples take 21 us (31 one piece at a time).
+// An 8x8 CU is eight pieces of luma and eight of chroma, so half of a warp is idle: in a long list
+// (GROUP), where 32 CUs in a row have at most 256 samples each, one CTA takes all of them, four CUs a warp
+// with eight lanes each, and the three CTAs beside it end.  The 170,000 CUs of a 1080p frame, two
+// references, planes in the L1 and L2: 107 us, 130 without groups.  (A warp that took any four CUs, big ones
+// in turn, needed 161 us for that list and 138 for one of 60,000 CUs, largest first, that takes 39 now: its
+// last warps hold four 64x64 CUs each.)
+template <bool GROUP>
+__global__ void __launch_bounds__(32 * MC_WARPS) k_mc_cu(const McParams P)
 {
-    const int wid = blockIdx.x * MC_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (per_warp == 1) {
-        if (wid < P.n) { const McReq q = P.reqs[wid]; mc_cu(P, q, lane, 32); }
-        return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int r = blockIdx.x * MC_WARPS + warp, at = lane, lanes = 32;
+    if (GROUP) {
+        const int g0 = (int)(blockIdx.x & ~3u) * MC_WARPS, k = g0 + lane;
+        const bool small = k < P.n && P.reqs[k].w * P.reqs[k].h <= 256;
+        if (__all_sync(0xFFFFFFFFu, small)) {
+            if (blockIdx.x & 3) return;
+            r = g0 + warp * 4 + (lane >> 3);
+            at = lane & 7;
+            lanes = 8;
+        }
     }
-    const int r0 = wid * 4;
-    if (r0 >= P.n) return;
-    const int mine = r0 + (lane >> 3);
-    const bool big = mine < P.n && P.reqs[mine].w * P.reqs[mine].h > 256;
-    const bool split = __any_sync(0xFFFFFFFFu, big);
-    for (int k = 0; k < (split ? 4 : 1); k++) {
-        const int r = split ? r0 + k : mine;
-        if (r < P.n) { const McReq q = P.reqs[r]; mc_cu(P, q, split ? lane : lane & 7, split ? 32 : 8); }
-    }
+    if (r >= P.n) return;
+    const McReq q = P.reqs[r];
+    mc_cu<GROUP ? 2 : 4>(P, q, at, lanes);
 }
 
 // ------------------------------------------------------------------ affine CUs
@@ -260,7 +281,8 @@ __global__ void __launch_bounds__(32 * AFF_WARPS) k_mc_affine(const McParams P, 
     }
     o += w * h;
     // chroma: 4x4 blocks per 8x8 luma with the rounded mean of their four 4x4 MVs, a lane per row of four
-    // samples (a lane a sample: 174 us for the 20,400 affine CUs of a 1080p frame, now 114)
+    // samples (a lane a sample: 174 us for the 20,400 affine CUs of a 1080p frame, one row at a time 121, now
+    // 110)
     const int wc = w >> 1, hc = h >> 1;
     const bool aligned = ((uintptr_t)o & 3) == 0;
     for (int pl = 0; pl < 2; pl++, o += wc * hc)
@@ -336,9 +358,13 @@ int launch_mc_cu(int W, int H, const pel *const *planes, int n_slots, int i_ref,
     }
     P.i_ref = i_ref; P.i_c = i_c; P.n_slots = n_slots; P.W = W; P.H = H;
     P.reqs = (const McReq *)reqs; P.n = n; P.out = out; P.out_bytes = out_bytes;
+    int dev = 0, sms = 0;
+    UC_CHECK(cudaGetDevice(&dev));
+    UC_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     prof_begin(PROF_MC, st);
-    const int per = n >= MC_LONG_LIST ? 4 : 1;
-    k_mc_cu<<<(unsigned)((n + MC_WARPS * per - 1) / (MC_WARPS * per)), 32 * MC_WARPS, 0, st>>>(P, per);
+    const unsigned ctas = (unsigned)((n + MC_WARPS - 1) / MC_WARPS);
+    if (n >= MC_GROUP_PER_SM * sms) k_mc_cu<true><<<ctas, 32 * MC_WARPS, 0, st>>>(P);
+    else k_mc_cu<false><<<ctas, 32 * MC_WARPS, 0, st>>>(P);
     UC_CHECK(cudaGetLastError());
     count_launch(1);
     prof_end(PROF_MC, st);
