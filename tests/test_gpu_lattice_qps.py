@@ -162,3 +162,27 @@ def test_lattice_layouts_are_tuned_per_kind(gpu, n_modes, first):
     torch.cuda.synchronize()
     assert any(gpu.lattice_budgets(n_modes))
     assert torch.equal(cap[0], plain[second][0]) and torch.equal(cap[1], plain[second][1])
+
+
+@pytest.mark.parametrize("n_modes,W,H", [(1, 64, 64), (2, 136, 72), (3, 128, 128), (33, 64, 32)])
+def test_lattice_four_qps_of_few_jobs(gpu, oracle, n_modes, W, H):
+    # the lists of the jobs that each QP codes, from none of them to all, in tiles of few and of many jobs
+    import torch
+    qps = np.array([63, 37, 0, 51], np.int32)
+    org, rec = _frames(W, H, 70 + n_modes, 7)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    satd_o, q_o = oracle_lattice(oracle, org, rec, cus, 0, list(qps))
+    modes = np.stack([np.random.default_rng(k).permutation(33)[:n_modes] for k in range(n)]).astype(np.uint8)
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8), modes)]
+    d_satd = torch.zeros(n * 33, dtype=torch.int32, device="cuda")
+    d_q = torch.zeros(n * 33 * 4 * gpu.LAT_Q.itemsize, dtype=torch.uint8, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_modes_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, d[3].data_ptr(), n_modes, 0, qps.ctypes.data,
+        4, 1, d_satd.data_ptr(), d_q.data_ptr(), torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    at = (np.arange(n)[:, None] * 33 + modes).ravel()
+    assert np.array_equal(d_satd.cpu().numpy().view(np.uint32)[at], satd_o.ravel()[at])
+    got, want = d_q.cpu().numpy().view(gpu.LAT_Q).reshape(n * 33, 4)[at], q_o.reshape(n * 33, 4)[at]
+    for f in FIELDS:
+        assert np.array_equal(got[f], want[f]), f

@@ -204,12 +204,12 @@ struct LatShared {
     u8 mode[LAT_MAX_JOBS];
     u32 satd[LAT_MAX_JOBS], ssd0[LAT_MAX_JOBS];   // ssd0: of the prediction, for QPs that code nothing
     u32 flag[LAT_MAX_JOBS];   // bit q: QP q codes the job
-    // of the QP at hand: the statistics, the SSD and the list of the jobs it codes.  nz also has bits
-    // 16 + k / 20 + k: chunk k of eight columns / rows holds a level
+    // of the QP at hand: the statistics and the SSD.  nz also has bits 16 + k / 20 + k: chunk k of eight
+    // columns / rows holds a level
     u32 nz[LAT_MAX_JOBS], sum[LAT_MAX_JOBS], hash[LAT_MAX_JOBS], ssd[LAT_MAX_JOBS];
     int last[LAT_MAX_JOBS];
-    u8 list[LAT_MAX_JOBS];
-    int coded;      // jobs of the list
+    u8 list[LAT_MAX_QP][LAT_MAX_JOBS];   // the jobs that each QP codes
+    int coded[LAT_MAX_QP];               // and how many
     int tile_off[LAT_SHAPES + 1], cu_off[LAT_SHAPES], counts[LAT_SHAPES];   // of the queue (LatParams)
     int next[2], rank[2];           // the tile after this one and its launch rank, by the tile's parity
     int tables;   // shape class whose matrices and scan table are in place (-1: none)
@@ -638,6 +638,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         // (a record is stored at its mode: an entry above 32 would fall into other CUs' records)
         s_mode[j] = (u8)(P.modes ? min((int)P.modes[(size_t)lat_perm(perm + cu0 + g).id * P.n_modes + mi], LAT_NO_MODE) : mi);
         s_satd[j] = 0; s_flag[j] = 0; S.ssd0[j] = 0;
+        S.nz[j] = 0; S.sum[j] = 0; S.hash[j] = 0; S.last[j] = -1; S.ssd[j] = 0;
     }
     LAT_STAGE(0);
 
@@ -821,42 +822,43 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     __syncthreads(); LAT_STAGE(5);
     for (int j = tid; j < J; j += LAT_THREADS)
         if (s_mode[j] != LAT_NO_MODE) P.satd_out[(size_t)S.cu[JG(j)].id * 33 + s_mode[j]] = s_satd[j];
-
+    if (P.n_qp == 0) return;
+    // the list of the jobs that each QP codes, a warp per QP: quant_check found a coefficient above its
+    // threshold, whose level is then not zero; the others keep the prediction's SSD and empty statistics.
+    // The first reader, the inverse column pass, comes behind the barrier of the first quantisation.
+    // (Built at the start of each QP's turn, behind a barrier of its own, the lists made calls of few modes
+    // slower than no lists at all: 104 us and 96 for one mode at four QPs of 256x256.)
+    if ((tid >> 5) < P.n_qp) {
+        const int q = tid >> 5;
+        int n = 0;
+        for (int base = 0; base < J; base += 32) {
+            const int j = base + lane;
+            const bool own = j < J && ((s_flag[j] >> q) & 1);
+            const u32 m = __ballot_sync(0xFFFFFFFFu, own);
+            if (own) S.list[q][n + __popc(m & ((1u << lane) - 1))] = (u8)j;
+            n += __popc(m);
+        }
+        if (lane == 0) S.coded[q] = n;
+    }
     // levels and magnitudes of a block of at most 256 coefficients go into one word, the count from bit 23
     constexpr bool PACK = KW_ * KH_ <= 256, CHUNKS = KW_ > 8 || KH_ > 8;
     for (int q = 0; q < P.n_qp; q++) {
         const int q_value = P.qp[lN - 4][q].q_value, dq_scale = P.qp[lN - 4][q].dq_scale, dq_shift = P.qp[lN - 4][q].dq_shift;
-        // the list of the jobs the QP codes: quant_check found a coefficient above its threshold, whose
-        // level is then not zero; the others keep the prediction's SSD and empty statistics
-        if (tid == 0) S.coded = 0;
-        for (int j = tid; j < J; j += LAT_THREADS) {
-            S.nz[j] = 0; S.sum[j] = 0; S.hash[j] = 0; S.last[j] = -1; S.ssd[j] = 0;
-        }
-        __syncthreads();
-        for (int base = wbase; base < J; base += LAT_THREADS) {
-            const int j = base + lane;
-            const bool own = j < J && ((s_flag[j] >> q) & 1);
-            const u32 m = __ballot_sync(0xFFFFFFFFu, own);
-            int at = 0;
-            if (lane == 0 && m) at = atomicAdd(&S.coded, __popc(m));
-            at = __shfl_sync(0xFFFFFFFFu, at, 0);
-            if (own) S.list[at + __popc(m & ((1u << lane) - 1))] = (u8)j;
-        }
         // first-pass levels, statistics, dequantisation (stored transposed, DQ^T[u][v], each row
         // in even/odd order of v).  The
         // level (|c| q_value + 2^(q_bits-1)) >> q_bits is exact in 32 bits: |c| <= 2^15 and
         // q_value < 2^15; it is 0 below the level threshold and, with q_value 0, for a QP that codes
-        // nothing of the job.  A task is RV coefficient rows (HV apart) of a job over RU columns, 16
-        // coefficients or 8, and lanes take consecutive v: the statistics are summed in registers and reduced
-        // once per task (with 8 coefficients a task, reductions and indexing were half of the instructions;
-        // above 1024 samples a tile holds so few jobs that 8 keep more threads busy).
+        // nothing of the job.  A task is RV coefficient rows (HV apart) of a job over RU columns, 8
+        // coefficients, and lanes take consecutive v: the statistics are summed in registers and reduced
+        // once per task.  (16 a task: 20.57 ms for a 1080p frame at four QPs where 8 take 20.86, but 96 us
+        // for one mode at four QPs of 256x256 where 8 take 87: tiles of few jobs leave most threads idle.)
         // The level hash of a record is the sum of level x weight(p) mod 2^32 over raster positions
         // p = v w + u, weight(p) = (K p + 0x7F4A7C15) | 1 with K = 0x9E3779B1: odd and spread over 32 bits, so
         // the hash changes with any single level, any sign and any exchange of two different levels.  The
         // weight is linear in p but for its lowest bit, and w and the first column are even: weight = row
         // part + constant of the column.
         {
-            constexpr int CT = W_ * H_ > 1024 ? 8 : 16, RV = CT / RU < KH_ ? CT / RU : KH_, HV = KH_ / RV;
+            constexpr int RV = 8 / RU, HV = KH_ / RV;
             constexpr int TPJ = HV * NUC, SEG = TPJ < 32 ? TPJ : 32;
             for (int base = wbase; base < J * TPJ; base += LAT_THREADS) {
                 const int i = base + lane;
@@ -927,11 +929,10 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                     rows[k] = CHUNKS ? __ballot_sync(0xFFFFFFFFu, mask[k] != 0) : 0;
                 }
                 // the count of levels rides above the sum of their magnitudes, which is below 2^23 for a
-                // segment's at most 512 levels (those are below 23053, and below 16303 where a segment has
-                // more than 256); a count of 512 wraps to 0
+                // segment's at most 256 levels (those are below 23053)
                 const u32 both = lat_seg_sum<SEG>(sa + (count << 23), lane);
                 sa = both & 0x7FFFFFu; hs = lat_seg_sum<SEG>(hs, lane);
-                const u32 nz = SEG * CT == 512 && both >> 23 == 0 && sa ? 512u : both >> 23;
+                const u32 nz = both >> 23;
                 const int last = lat_seg_max<SEG>(own_last, lane);
                 if (act && (lane & (SEG - 1)) == 0 && nz) {
                     atomicAdd(&S.sum[j], PACK ? both : sa);
@@ -963,7 +964,8 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         }
         __syncthreads(); LAT_STAGE(6);
         // the inverse passes run over the coded jobs only
-        const int JC_ = S.coded;
+        const int JC_ = S.coded[q];
+        const u8 *list = S.list[q];
         // inverse column pass T2[y][u] = clip16((sum_v Fh[v][y] DQ[v][u] + 16) >> 5); a task forms
         // rows y and H-1-y from the even-v and odd-v sums over CU columns u.  Chunks of columns past the
         // last level's are left out, empty ones before it are zeros.  Tiles with few
@@ -972,7 +974,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
             constexpr int CU = decltype(cu_tag)::value, NCU = KW_ / CU;
             for (int i = tid; i < JC_ * NCU * (H_ / 2); i += LAT_THREADS) {
                 const int y = i & (H_ / 2 - 1), uc = (i >> (LH - 1)) % NCU, k = i / ((H_ / 2) * NCU);
-                const int j = S.list[k];
+                const int j = list[k];
                 const u32 ch = S.nz[j] >> 16;
                 const int col = uc * CU >> 3;
                 if (KW_ > 8 && !((ch & 15) >> col)) continue;
@@ -1019,7 +1021,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
                 const bool act = i < JC_ * TPJ;
                 const int ii = act ? i : base;
                 const int x = (ii & (W_ / 4 - 1)) * 2, yc = (ii >> (LW - 2)) % NCY, k = ii / TPJ;
-                const int j = S.list[k];
+                const int j = list[k];
                 const s16 *t2 = JT2(j) + yc * CY * L.t2s;
                 const u32 *f = fwt + x * L.fwt_ws;
                 // e0, o0: column x (and W-1-x); e1, o1: column x+1 (and W-2-x)
@@ -1069,14 +1071,14 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
         else inv_row(std::integral_constant<int, 4>{});
         __syncthreads(); LAT_STAGE(8);
         for (int j = tid; j < J; j += LAT_THREADS) {
-            if (s_mode[j] == LAT_NO_MODE) continue;
             LatQ o;
             o.ssd = (s_flag[j] >> q) & 1 ? S.ssd[j] : S.ssd0[j];
             o.coef_hash = S.hash[j];
             o.num_nz = (u16)(PACK ? S.sum[j] >> 23 : S.nz[j] & 0xFFFFu);
             o.last_nz = (s16)S.last[j];
             o.sum_abs = PACK ? S.sum[j] & 0x7FFFFFu : S.sum[j];
-            P.q_out[((size_t)S.cu[JG(j)].id * 33 + s_mode[j]) * P.n_qp + q] = o;
+            if (s_mode[j] != LAT_NO_MODE) P.q_out[((size_t)S.cu[JG(j)].id * 33 + s_mode[j]) * P.n_qp + q] = o;
+            if (q + 1 < P.n_qp) { S.nz[j] = 0; S.sum[j] = 0; S.hash[j] = 0; S.last[j] = -1; S.ssd[j] = 0; }
         }
         __syncthreads(); LAT_STAGE(9);
     }
