@@ -164,6 +164,24 @@ def test_lattice_layouts_are_tuned_per_kind(gpu, n_modes, first):
     assert torch.equal(cap[0], plain[second][0]) and torch.equal(cap[1], plain[second][1])
 
 
+@pytest.mark.parametrize("W,H", [(16, 8), (256, 128), (256, 136)])
+def test_lattice_satd_only_call_sizes(gpu, oracle, W, H):
+    # the tile layout of a SATD-only call follows from its size: the smallest, and both sides of the line
+    # (on 152 SMs)
+    import torch
+    org, rec = _frames(W, H, W + H, 6)
+    cus = gpu.lattice_cus(W, H)
+    n = len(cus)
+    satd_o, _ = oracle_lattice(oracle, org, rec, cus, 1, [32])
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8))]
+    d_satd = torch.full((n * 33,), -1, dtype=torch.int32, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, 1, None, 0, 1, d_satd.data_ptr(), None,
+        torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    assert np.array_equal(d_satd.cpu().numpy().view(np.uint32), satd_o.ravel())
+
+
 @pytest.mark.parametrize("n_modes,W,H", [(1, 64, 64), (2, 136, 72), (3, 128, 128), (33, 64, 32)])
 def test_lattice_four_qps_of_few_jobs(gpu, oracle, n_modes, W, H):
     # the lists of the jobs that each QP codes, from none of them to all, in tiles of few and of many jobs

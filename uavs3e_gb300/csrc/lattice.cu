@@ -219,6 +219,12 @@ struct LatTune {
 static LatTune g_tune[64];
 static bool g_tune_on = true;
 
+// SATD-only calls are not tuned.  A large one takes the default budget; one of fewer than
+// LAT_SATD_SMALL_JOBS (CU, mode) jobs per resident CTA takes LAT_SATD_SMALL, whose shorter tiles keep all
+// CTAs busy to the end: 33 modes of 64x64 41 us (67 with the default), of 256x128 (403 jobs a CTA) 96 (99),
+// of 256x192 (605) 127 (123); 5 modes of 192x128 44 (67), of 512x384 (367) 106 (107).
+constexpr int LAT_SATD_SMALL = 20 * 1024, LAT_SATD_SMALL_JOBS = 410;
+
 // per device: the CU permutation and the queue's counters
 struct LatScratch {
     LatPerm *perm = nullptr;
@@ -354,7 +360,9 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
         std::lock_guard<std::mutex> lk(T.mu);
         const int kind = n_qp > 1;
         int *tuned = T.budget[n_modes][kind];
-        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = n_qp > 0 && tuned[c] ? tuned[c] : LAT_BUDGET;
+        const bool small = n_qp == 0 && (long long)n_cus * n_modes < (long long)LAT_SATD_SMALL_JOBS * S.sms * S.occ;
+        for (int c = 0; c < LAT_SHAPES; c++)
+            budgets[c] = small ? LAT_SATD_SMALL : n_qp > 0 && tuned[c] ? tuned[c] : LAT_BUDGET;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0) UC_CHECK(cudaStreamIsCapturing(st, &cap));
         if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0 && cap == cudaStreamCaptureStatusNone) {
