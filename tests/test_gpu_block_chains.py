@@ -105,10 +105,10 @@ def _check_rdoq(oracle, reqs, ests, coefs, d_c, nz):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("est_shift", (0, 4, 8))
-def test_rdoq_estimates_off_16_bytes(gpu, oracle, est_shift):
+@pytest.mark.parametrize("est_shift,n", ((0, 70), (4, 70), (4, 900), (8, 70), (8, 900)))
+def test_rdoq_estimates_off_16_bytes(gpu, oracle, est_shift, n):
     import torch
-    reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=70, k=3), 4400)
+    reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=n, k=3), 4400 + n)
     d_c, nz, keep = _rdoq_device(gpu, reqs, ests, coefs, est_shift=est_shift)
     torch.cuda.synchronize()
     _check_rdoq(oracle, reqs, ests, coefs, d_c, nz)
@@ -117,7 +117,7 @@ def test_rdoq_estimates_off_16_bytes(gpu, oracle, est_shift):
 @pytest.mark.gpu
 def test_rdoq_lists_on_two_streams(gpu, oracle):
     import torch
-    sets = [cases.rdoq_inputs(oracle, dict(n=n, k=2), 4500 + n) for n in (200, 3, 90, 257)]
+    sets = [cases.rdoq_inputs(oracle, dict(n=n, k=2), 4500 + n) for n in (900, 3, 90, 801)]
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
     got = [_rdoq_device(gpu, *s, stream=streams[k % 2].cuda_stream) for k, s in enumerate(sets)]
     torch.cuda.synchronize()
@@ -163,7 +163,7 @@ class _Graph:
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", (3, 600))
+@pytest.mark.parametrize("n", (3, 1000))
 def test_captured_block_lists(gpu, oracle, n):
     # one capture of both calls, replayed on new blocks by two executables of the graph and as a child of
     # another graph, after the captured one itself is gone
@@ -223,3 +223,47 @@ def test_captured_workspaces_are_given_back(gpu, oracle):
         g.destroy(g.handle)
         free.append(torch.cuda.mem_get_info()[0])
     assert free[7] - free[-1] < 512 << 20, (free[7], free[-1])           # 40 calls' blocks would be 1.3 GB
+
+
+def _sms():
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extra", (-1, 0, 1, 33))
+@pytest.mark.parametrize("by", (0, 3))
+def test_rdoq_list_lengths(gpu, oracle, extra, by):
+    # around the length from which blocks are grouped by their chains (5 per SM); some outside the domain
+    n = 5 * _sms() + extra
+    reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=n, k=3), 4800 + extra)
+    reqs, coefs = _shift(reqs, coefs, by)
+    bad = np.arange(n) % 97 == 5
+    want_c, got_c = coefs.copy(), coefs.copy()
+    want = np.full(n, -1, np.int32)
+    want[~bad] = oracle.rdoq(reqs[~bad], ests, want_c)
+    reqs["qp"][bad] = 80
+    assert np.array_equal(gpu.rdoq(reqs, ests, got_c), want)
+    assert np.array_equal(got_c, want_c)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("extra", (-1, 0, 1, 33))
+def test_coef_rate_list_lengths(gpu, oracle, extra):
+    # around the length from which blocks are grouped by their chains (6 per SM); each block from two coder
+    # states, some requests outside the domain
+    n = 6 * _sms() + extra
+    levels, reqs = cases.coef_rate_inputs(np.random.default_rng(800 + extra), (n + 1) // 2)
+    other = reqs.copy()
+    other["range"] = 256 + (reqs["range"] + 100) % 256
+    reqs = np.concatenate([reqs, other])[:n]
+    reqs["range"][::89] = 512
+    reqs["num_sig"][7::101] = 4096
+    bad = np.arange(n) % 89 == 0
+    bad[7::101] = True
+    want = np.zeros(n, dtype=gpu.COEF_RATE_OUT)
+    want[~bad] = oracle.coef_rate(levels, reqs[~bad])
+    want["bits"][bad] = 0xFFFFFFFF                       # and the state as it was
+    for f in ("range", "run", "run_rdoq", "level", "last1", "last2"):
+        want[f][bad] = reqs[f][bad]
+    assert gpu.coef_rate(levels, reqs).tobytes() == want.tobytes()

@@ -6,13 +6,14 @@
 // (range and the channel's run, run_rdoq, level, last1, last2 models).  Results: the bits
 // counted, the range and the models after the block, bit-exact with the reference.
 //
-// Two launches with a grouping between them: a warp per block lists its levels in scan order
-// (k_cr_list), the blocks are ordered by the bins they will code (blocksort.cuh), and a lane per
-// block codes its chain (k_cr_code).  The chains bound the call: one lane's bins follow one another.
-// 60,000 blocks of the 23 shapes (5.6 M levels, 31 M bins, up to 5,300 bins a block) take 54 us to list
-// and 0.55 ms to code; one launch in which a warp listed 32 blocks in turn and then coded them side by
-// side, symbol after symbol, took 2.37 ms with 4 of 32 lanes active on average.  The model update is
-// the rule the reference tabulates in tbl_plps / tbl_plps_ext (src/entropy.c:41), computed.
+// Two launches with a grouping between them; a short list takes one (CR_SHORT_PER_SM).  A warp per block
+// lists its levels in scan order (k_cr_list), the blocks are ordered by the bins they will code
+// (blocksort.cuh), and a lane per block codes its chain (k_cr_code).  The chains bound the call: one lane's
+// bins follow one another.  60,000 blocks of the 23 shapes (5.6 M levels, 31 M bins, up to 5,300 bins a
+// block) take 67 us to list and 0.55 ms to code; one launch in which a warp listed 32 blocks in turn and
+// then coded them side by side, symbol after symbol, took 2.37 ms with 4 of 32 lanes active on average.
+// The model update is the rule the reference tabulates in tbl_plps / tbl_plps_ext (src/entropy.c:41),
+// computed.
 #include "blocksort.cuh"
 #include "common.cuh"
 #include "tables.h"
@@ -84,6 +85,11 @@ __device__ __forceinline__ u16 cr_code_of(u32 mdl, u32 bin)
 // bits of the exp-Golomb escape of v >= -1 (order 0): sum of 2^k steps down to below 0
 __device__ __forceinline__ u32 cr_egk(int v) { return 2u * (31u - (u32)__clz(v + 2)) + 1u; }
 
+// blocks per SM below which a list takes one launch, a CTA per block (k_cr_short), instead of listing,
+// grouping and chains: as long as two waves of CTAs hold it.  On 152 SMs, one 4x4 block takes 10.5 us and
+// 22, 768 blocks of at most 64 samples 56 and 71, of 1024 samples and more 339 and 585; at 2,048 99 and 71,
+// 545 and 538.
+constexpr int CR_SHORT_PER_SM = 6;
 constexpr int CR_LIST_WARPS = 8;     // blocks per CTA of the listing
 constexpr int CR_LIST_UNROLL = 4;    // 32-position windows whose loads are in flight together
 constexpr u32 CR_BAD = 0xFFFFFFFFu;  // a request outside the domain, or fewer levels than num_sig
@@ -98,13 +104,11 @@ __device__ __forceinline__ u32 cr_entry(int run, int sym, int pos, int n)
 
 // Listing, a warp per block: checks the request and writes, in scan order, an entry for each of the
 // block's first num_sig non-zero levels to list[] at the block's own level offset (a ballot and a
-// prefix count per 32 positions); sums the bits the coder state has no part in (signs and escapes)
-// and the bins the block will code, which are its chain length for the grouping.
-__global__ void __launch_bounds__(32 * CR_LIST_WARPS) k_cr_list(const CrParams P, u32 *list_all, BlockOrder O)
+// prefix count per 32 positions); sums the bits the coder state has no part in (signs and escapes), or
+// CR_BAD, and the bins the block will code (0 for a bad request).
+struct CrListed { u32 fixed, len; };
+__device__ __forceinline__ CrListed cr_list(const CrParams &P, int r, u32 *list_all, int lane)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * CR_LIST_WARPS + warp;
-    if (r >= P.n) return;
     const u32 word = lane < 30 ? reinterpret_cast<const u32 *>(P.reqs + r)[lane] : 0u;
     const u32 offset = __shfl_sync(0xffffffffu, word, 0), dims = __shfl_sync(0xffffffffu, word, 1);
     const u32 sr = __shfl_sync(0xffffffffu, word, 2);
@@ -158,9 +162,19 @@ __global__ void __launch_bounds__(32 * CR_LIST_WARPS) k_cr_list(const CrParams P
         fixed = __reduce_add_sync(0xffffffffu, fixed);
         ok = cnt >= num_sig;
     }
+    return { ok ? fixed : CR_BAD, ok ? len : 0u };
+}
+
+// the listing of a grouped list: a block's bins are its chain length
+__global__ void __launch_bounds__(32 * CR_LIST_WARPS) k_cr_list(const CrParams P, u32 *list_all, BlockOrder O)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = blockIdx.x * CR_LIST_WARPS + warp;
+    if (r >= P.n) return;
+    const CrListed l = cr_list(P, r, list_all, lane);
     if (lane == 0) {
-        O.key[r] = bs_count(O.counts, ok ? len : 0u);
-        P.fixed[r] = ok ? fixed : CR_BAD;
+        O.key[r] = bs_count(O.counts, l.len);
+        P.fixed[r] = l.fixed;
     }
 }
 
@@ -259,15 +273,85 @@ __device__ __forceinline__ void cr_lasts(CrShared &S, CrWalk &W, u16 (*codes)[32
     }
 }
 
+// cr_next of every model and bin by `threads` threads, of which this is number t
+__device__ __forceinline__ void cr_fill(CrTable &T, int t, int threads)
+{
+    for (int k = t; k < 2 * 8192; k += threads) T.next[k] = (u16)cr_next((u32)k >> 1, (k & 1) == ((k >> 1) & 1));
+}
+
+// the chains of 32 listed blocks by the CTA's five warps, lane l working on block i (where `mine`), whose
+// listing gave `fixed`; every thread of the CTA calls it, with the model table in place
+__device__ __forceinline__ void cr_chains(const CrParams &P, CrShared &S, const u32 *list_all, int lane, int role, bool mine,
+                                          int i, u32 fixed)
+{
+    // a role's models: words [w0, w1) of the request's 27 and the same words of the result
+    const int w0 = role == 0 ? 0 : role == 1 ? 12 : role == 2 ? 6 : 18, w1 = role == 3 ? 27 : role == 4 ? 18 : w0 + 6;
+    const u32 *qw = reinterpret_cast<const u32 *>(P.reqs + i);
+    u32 *ow = reinterpret_cast<u32 *>(P.out + i);
+    const u32 sr = qw[2];
+    CrWalk W;
+    W.k = 0;
+    W.num_sig = fixed == CR_BAD ? 0u : sr & 0xffff;    // a bad request codes no level: its state stays
+    W.list.open(list_all + qw[0], role < 4 ? W.num_sig : 0u, smem_addr(&S.ring[role & 3][0][lane]));
+    W.t0 = 10;
+    for (int k = w0; k < w1; k++) {
+        const u32 x = qw[3 + k];
+        S.mdl[2 * k][lane] = (u16)x;
+        S.mdl[2 * k + 1][lane] = (u16)(x >> 16);
+    }
+    u32 range = sr >> 16, bits = fixed;
+    bool fill = true;
+    for (int s = 0;; s++) {
+        const int b = s & 1;
+        u16 (*codes)[32] = S.codes[b];
+        if (fill) {
+            if (role == 0) {
+                const int nc = cr_models<0>(S, W, codes, lane);
+                // up to a multiple of four codes: an MPS with LPS range 0 changes nothing
+#pragma unroll
+                for (int j = 0; j < 3; j++) codes[nc + j][lane] = 256;
+                S.n_codes[b][lane] = nc;
+                const int more = __any_sync(0xffffffffu, W.k < W.num_sig);
+                if (lane == 0) S.more[b] = more;
+            } else if (role == 1) {
+                cr_models<1>(S, W, codes, lane);
+            } else if (role == 2) {
+                cr_models<2>(S, W, codes, lane);
+            } else if (role == 3) {
+                cr_lasts(S, W, codes, lane);
+            }
+        }
+        if (role == 4 && s > 0) {
+            codes = S.codes[b ^ 1];
+            const int nc = S.n_codes[b ^ 1][lane];
+            for (int j = 0; j < nc; j += 4) {
+                u32 c[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) c[q] = codes[j + q][lane];
+#pragma unroll
+                for (int q = 0; q < 4; q++) cr_code(range, bits, c[q] & 255, c[q] >> 8);
+            }
+        }
+        __syncthreads();
+        if (!fill) break;
+        fill = S.more[b] != 0;
+    }
+    W.list.close();
+    if (mine) {
+        for (int k = w0; k < w1; k++) ow[2 + k] = (u32)S.mdl[2 * k][lane] | (u32)S.mdl[2 * k + 1][lane] << 16;
+        if (role == 4) {
+            ow[0] = bits;                              // CR_BAD = ~0 for a bad request
+            ow[1] = range;
+        }
+    }
+}
+
 __global__ void __launch_bounds__(32 * CR_ROLES) k_cr_code(const CrParams P, const u32 *list_all, const BlockOrder O)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     CrShared &S = *reinterpret_cast<CrShared *>(smem_raw);
     const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < 2 * 8192; k += 32 * CR_ROLES)
-        S.T.next[k] = (u16)cr_next((u32)k >> 1, (k & 1) == ((k >> 1) & 1));
-    // a role's models: words [w0, w1) of the request's 27 and the same words of the result
-    const int w0 = role == 0 ? 0 : role == 1 ? 12 : role == 2 ? 6 : 18, w1 = role == 3 ? 27 : role == 4 ? 18 : w0 + 6;
+    cr_fill(S.T, threadIdx.x, 32 * CR_ROLES);
     // groups of 32 chains from the work counter, the longest chains first
     for (;;) {
         if (threadIdx.x == 0) S.group = (int)atomicAdd(O.counts + BS_WORK, 1u);
@@ -276,65 +360,25 @@ __global__ void __launch_bounds__(32 * CR_ROLES) k_cr_code(const CrParams P, con
         const int at = S.group * 32 + lane;
         const bool mine = at < P.n;
         const int i = mine ? O.perm[at] : 0;
-        const u32 *qw = reinterpret_cast<const u32 *>(P.reqs + i);
-        u32 *ow = reinterpret_cast<u32 *>(P.out + i);
-        const u32 fixed = mine ? P.fixed[i] : CR_BAD, sr = qw[2];
-        CrWalk W;
-        W.k = 0;
-        W.num_sig = fixed == CR_BAD ? 0u : sr & 0xffff;    // a bad request codes no level: its state stays
-        W.list.open(list_all + qw[0], role < 4 ? W.num_sig : 0u, smem_addr(&S.ring[role & 3][0][lane]));
-        W.t0 = 10;
-        for (int k = w0; k < w1; k++) {
-            const u32 x = qw[3 + k];
-            S.mdl[2 * k][lane] = (u16)x;
-            S.mdl[2 * k + 1][lane] = (u16)(x >> 16);
-        }
-        u32 range = sr >> 16, bits = fixed;
-        bool fill = true;
-        for (int s = 0;; s++) {
-            const int b = s & 1;
-            u16 (*codes)[32] = S.codes[b];
-            if (fill) {
-                if (role == 0) {
-                    const int nc = cr_models<0>(S, W, codes, lane);
-                    // up to a multiple of four codes: an MPS with LPS range 0 changes nothing
-#pragma unroll
-                    for (int j = 0; j < 3; j++) codes[nc + j][lane] = 256;
-                    S.n_codes[b][lane] = nc;
-                    const int more = __any_sync(0xffffffffu, W.k < W.num_sig);
-                    if (lane == 0) S.more[b] = more;
-                } else if (role == 1) {
-                    cr_models<1>(S, W, codes, lane);
-                } else if (role == 2) {
-                    cr_models<2>(S, W, codes, lane);
-                } else if (role == 3) {
-                    cr_lasts(S, W, codes, lane);
-                }
-            }
-            if (role == 4 && s > 0) {
-                codes = S.codes[b ^ 1];
-                const int nc = S.n_codes[b ^ 1][lane];
-                for (int j = 0; j < nc; j += 4) {
-                    u32 c[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) c[q] = codes[j + q][lane];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) cr_code(range, bits, c[q] & 255, c[q] >> 8);
-                }
-            }
-            __syncthreads();
-            if (!fill) break;
-            fill = S.more[b] != 0;
-        }
-        W.list.close();
-        if (mine) {
-            for (int k = w0; k < w1; k++) ow[2 + k] = (u32)S.mdl[2 * k][lane] | (u32)S.mdl[2 * k + 1][lane] << 16;
-            if (role == 4) {
-                ow[0] = bits;                          // CR_BAD = ~0 for a bad request
-                ow[1] = range;
-            }
-        }
+        cr_chains(P, S, list_all, lane, role, mine, i, mine ? P.fixed[i] : CR_BAD);
     }
+}
+
+// A short list, in one launch: a CTA per block, whose first warp lists it while the others fill the model
+// table; lane 0 of each warp then works on its chain.
+__global__ void __launch_bounds__(32 * CR_ROLES) k_cr_short(const CrParams P, u32 *list_all)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    CrShared &S = *reinterpret_cast<CrShared *>(smem_raw);
+    const int lane = threadIdx.x & 31, role = threadIdx.x >> 5;
+    if (role == 0) {
+        const CrListed l = cr_list(P, blockIdx.x, list_all, lane);
+        if (lane == 0) S.group = (int)l.fixed;
+    } else {
+        cr_fill(S.T, threadIdx.x - 32, 32 * (CR_ROLES - 1));
+    }
+    __syncthreads();
+    cr_chains(P, S, list_all, lane, role, lane == 0, blockIdx.x, lane == 0 ? (u32)S.group : CR_BAD);
 }
 
 int launch_coef_rate(const void *reqs, int n, const s16 *levels, unsigned long long n_levels, void *out,
@@ -351,21 +395,24 @@ int launch_coef_rate(const void *reqs, int n, const s16 *levels, unsigned long l
     P.reqs = (const CrReq *)reqs; P.n = n; P.levels = levels; P.n_levels = n_levels; P.out = (CrOut *)out;
     for (int a = 0; a < 7; a++)
         for (int b = 0; b < 7; b++) P.scan[a][b] = tab->scan[a][b];
+    int sms = 0;
+    UC_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool brief = n < CR_SHORT_PER_SM * sms;
     // one word per level (the lists, at the levels' offsets), the grouping's arrays, a word per block
     const size_t b_list = ((size_t)n_levels * sizeof(u32) + 255) & ~(size_t)255, b_order = bs_bytes((size_t)n);
     char *ws = nullptr;
-    int rc = work_alloc((void **)&ws, b_list + b_order + (size_t)n * sizeof(u32), st);
+    int rc = work_alloc((void **)&ws, b_list + (brief ? 256 : b_order + (size_t)n * sizeof(u32)), st);
     if (rc) return rc;
     u32 *list = (u32 *)ws;
     const BlockOrder O = bs_place(ws + b_list, (size_t)n);
     P.fixed = (u32 *)(ws + b_list + b_order);
-    // persistent CTAs: each fills its model table once
-    int sms = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_cr_code, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CrShared));
-    if (e == cudaSuccess) e = cudaMemsetAsync(O.counts, 0, BS_CLEAR, st);
-    if (e == cudaSuccess) {
+    cudaError_t e = cudaFuncSetAttribute(brief ? (const void *)k_cr_short : (const void *)k_cr_code,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CrShared));
+    if (e == cudaSuccess && brief) {
+        k_cr_short<<<(unsigned)n, 32 * CR_ROLES, sizeof(CrShared), st>>>(P, list);
+        e = cudaGetLastError();
+    } else if (e == cudaSuccess && (e = cudaMemsetAsync(O.counts, 0, BS_CLEAR, st)) == cudaSuccess) {
+        // persistent CTAs: each fills its model table once
         k_cr_list<<<(unsigned)((n + CR_LIST_WARPS - 1) / CR_LIST_WARPS), 32 * CR_LIST_WARPS, 0, st>>>(P, list, O);
         k_bs_scatter<<<(unsigned)((n + BS_BUCKETS - 1) / BS_BUCKETS), BS_BUCKETS, 0, st>>>(O.key, O.counts, n, O.perm);
         k_cr_code<<<(unsigned)std::min((n + 31) / 32, sms * CR_CTAS), 32 * CR_ROLES, sizeof(CrShared), st>>>(P, list, O);
@@ -374,7 +421,7 @@ int launch_coef_rate(const void *reqs, int n, const s16 *levels, unsigned long l
     rc = work_free(ws, st);
     UC_CHECK(e);
     if (rc) return rc;
-    count_launch(3);
+    count_launch(brief ? 1 : 3);
     return UC_OK;
 }
 

@@ -3,12 +3,12 @@
 // the encoder derived from its entropy-coder state (rdoq_init_cu_est_bits, :139-156) -- the
 // levels and the count of coded coefficients bit-exact with the reference's call.
 //
-// Two launches with a grouping between them.  k_rdoq_list, a warp per block: zeroes the coefficients
-// past 32 columns / rows, runs quant_check, and lists in scan order the positions whose first-pass
-// level (quant_rdoq) is not zero.  The decision pass is a chain (each coded level selects the
-// contexts of the next), so k_rdoq_chain walks one block per lane over its listed positions, the
-// blocks ordered by their position counts (blocksort.cuh): a run of z zero levels adds
-// est_run[last_b_zero][0] + (z - 1) est_run[1][0] bits at once, as the reference's per-position
+// Two launches with a grouping between them; a short list takes one (RQ_SHORT_PER_SM).  k_rdoq_list, a
+// warp per block: zeroes the coefficients past 32 columns / rows, runs quant_check, and lists in scan
+// order the positions whose first-pass level (quant_rdoq) is not zero.  The decision pass is a chain
+// (each coded level selects the contexts of the next), so k_rdoq_chain walks one block per lane over its
+// listed positions, the blocks ordered by their position counts (blocksort.cuh): a run of z zero levels
+// adds est_run[last_b_zero][0] + (z - 1) est_run[1][0] bits at once, as the reference's per-position
 // loop accumulates them.  The listing is bound by memory latency (60 us for 60,000 blocks of the 23
 // shapes, 39 M coefficients), the chains by the dependent instructions of the longest block (0.30 ms
 // for 860 positions, about 190 instructions each).  One launch in which a warp listed its 32 blocks one
@@ -26,6 +26,11 @@
 
 namespace uc {
 
+// blocks per SM below which a list takes one launch, a warp per block (k_rdoq_short), instead of listing,
+// grouping and chains.  On 152 SMs, blocks of 1024 samples and more take the same time either way at
+// 760 (258 us and 265; 217 and 265 at 512, 349 and 267 at 2,048), mixed shapes at 1,024 (259 and 265);
+// one 4x4 block takes 12 us and 22.
+constexpr int RQ_SHORT_PER_SM = 5;
 constexpr int RQ_WARPS = 2;          // blocks per CTA of the listing: they differ in size, few wait for one another
 
 struct RdoqReq {
@@ -66,12 +71,11 @@ constexpr int RQ_UNROLL = 4;         // 32-position windows whose shared loads a
 
 // Listing, a warp per block: zeroes the coefficients past 32 columns / rows, runs quant_check and, for
 // a block that is coded, lists in scan order the positions whose first-pass level (quant_rdoq) is
-// not zero (a ballot and a prefix count per 32 positions), clears the block (the chain writes its
-// levels) and counts it into the grouping by its positions.  The block is read from memory once, by
-// 16-byte vectors where it starts on a 16-byte boundary.
+// not zero (a ballot and a prefix count per 32 positions) and clears the block (the chain writes its
+// levels).  Returns the positions listed.  The block is read from memory once, by 16-byte vectors where it
+// starts on a 16-byte boundary.
 template <bool VEC>
-__device__ __forceinline__ void rq_list_block(const RdoqParams &P, const RdoqReq &q, int r, s16 *st, int lane,
-                                              const BlockOrder &O)
+__device__ __forceinline__ int rq_list_block(const RdoqParams &P, const RdoqReq &q, s16 *st, int lane)
 {
     const int lw = q.log2w, lh = q.log2h, w = 1 << lw, h = 1 << lh;
     s16 *coef = P.coefs + q.coef_offset;
@@ -119,10 +123,7 @@ __device__ __forceinline__ void rq_list_block(const RdoqParams &P, const RdoqReq
         }
         for (int p = max_used + lane; p < max_num; p += 32) coef[p] = 0;
     }
-    if (!__any_sync(0xffffffffu, above)) {
-        if (lane == 0) { P.num_nz[r] = 0; O.key[r] = bs_count(O.counts, 0); }
-        return;
-    }
+    if (!__any_sync(0xffffffffu, above)) return 0;
     __syncwarp();
     // scan order; the positions whose first-pass level (quant_rdoq) is not zero -- exactly those
     // with |c| >= thr -- are listed in order as (position << 16 | coefficient).  The zig-zag visits
@@ -152,9 +153,21 @@ __device__ __forceinline__ void rq_list_block(const RdoqParams &P, const RdoqReq
         for (int v = lane; v < max_used / 8; v += 32) reinterpret_cast<uint4 *>(coef)[v] = make_uint4(0, 0, 0, 0);
     else
         for (int p = lane; p < max_used; p += 32) coef[p] = 0;
-    if (lane == 0) { P.num_nz[r] = cnt; O.key[r] = bs_count(O.counts, cnt); }
+    return cnt;
 }
 
+// the positions listed of a block, -1 for one outside the supported domain (left untouched)
+__device__ __forceinline__ int rq_list(const RdoqParams &P, const RdoqReq &q, s16 *st, int lane)
+{
+    const int lw = q.log2w, lh = q.log2h;
+    if (lw < 2 || lw > 6 || lh < 2 || lh > 6 || q.qp > 79 || q.ch_type > 2 || q.est >= P.n_est ||
+        (unsigned long long)q.coef_offset + (1ull << (lw + lh)) > P.n_coefs)
+        return -1;
+    return (((uintptr_t)(P.coefs + q.coef_offset)) & 15) == 0 ? rq_list_block<true>(P, q, st, lane)
+                                                              : rq_list_block<false>(P, q, st, lane);
+}
+
+// the listing of a grouped list: each block is counted into the grouping by its positions
 __global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq_list(const RdoqParams P, BlockOrder O)
 {
     __shared__ __align__(16) s16 s_stage[RQ_WARPS][RQ_STAGE];
@@ -162,15 +175,8 @@ __global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq_list(const RdoqParams P,
     const int r = blockIdx.x * RQ_WARPS + warp;
     if (r >= P.n) return;
     const RdoqReq q = P.reqs[r];
-    const int lw = q.log2w, lh = q.log2h;
-    // blocks outside the supported domain are left untouched, with num_nz = -1
-    if (lw < 2 || lw > 6 || lh < 2 || lh > 6 || q.qp > 79 || q.ch_type > 2 || q.est >= P.n_est ||
-        (unsigned long long)q.coef_offset + (1ull << (lw + lh)) > P.n_coefs) {
-        if (lane == 0) { P.num_nz[r] = -1; O.key[r] = bs_count(O.counts, 0); }
-        return;
-    }
-    if ((((uintptr_t)(P.coefs + q.coef_offset)) & 15) == 0) rq_list_block<true>(P, q, r, s_stage[warp], lane, O);
-    else rq_list_block<false>(P, q, r, s_stage[warp], lane, O);
+    const int cnt = rq_list(P, q, s_stage[warp], lane);
+    if (lane == 0) { P.num_nz[r] = cnt; O.key[r] = bs_count(O.counts, (u32)max(cnt, 0)); }
 }
 
 // N pairs of estimates: 8 or 16 bytes at once where the estimate sets start on 16 bytes (a set is a
@@ -190,17 +196,10 @@ __device__ __forceinline__ void rq_pairs(const s32 (*p)[2], int2 (&v)[N])
     }
 }
 
-// Decision chains, a block per lane, 32 blocks with about as many listed positions per warp in the
-// order of the grouping.  num_nz[r] holds the positions listed (0 or -1: the block is done).
+// the decision chain of a block, by one lane, over its cnt > 0 listed positions; returns num_nz
 template <bool VEC>
-__global__ void __launch_bounds__(32) k_rdoq_chain(const RdoqParams P, const int *perm)
+__device__ __forceinline__ int rq_chain(const RdoqParams &P, const RdoqReq &q, int cnt)
 {
-    const int at = blockIdx.x * 32 + threadIdx.x;
-    if (at >= P.n) return;
-    const int r = perm[at];
-    const int cnt = P.num_nz[r];
-    if (cnt <= 0) return;
-    const RdoqReq q = P.reqs[r];
     const int lw = q.log2w, lh = q.log2h, ch = q.ch_type, max_num = 1 << (lw + lh);
     const int odd = (lw + lh) & 1, log2_size = (lw + lh) >> 1;
     const int q_bits = 14 + (15 - 8 - log2_size);
@@ -282,7 +281,35 @@ __global__ void __launch_bounds__(32) k_rdoq_chain(const RdoqParams P, const int
     if (num_nz)
         for (int k = k_end + 1; k <= k_last; k++)  // levels after the chosen last position, back to zero
             coef[scan[list[k] >> 16]] = 0;
-    P.num_nz[r] = num_nz;
+    return num_nz;
+}
+
+// Decision chains, a block per lane, 32 blocks with about as many listed positions per warp in the
+// order of the grouping.  num_nz[r] holds the positions listed (0 or -1: the block is done).
+template <bool VEC>
+__global__ void __launch_bounds__(32) k_rdoq_chain(const RdoqParams P, const int *perm)
+{
+    const int at = blockIdx.x * 32 + threadIdx.x;
+    if (at >= P.n) return;
+    const int r = perm[at];
+    const int cnt = P.num_nz[r];
+    if (cnt <= 0) return;
+    const RdoqReq q = P.reqs[r];
+    P.num_nz[r] = rq_chain<VEC>(P, q, cnt);
+}
+
+// A short list, in one launch: a warp lists a block and its first lane walks the chain.
+template <bool VEC>
+__global__ void __launch_bounds__(32 * RQ_WARPS) k_rdoq_short(const RdoqParams P)
+{
+    __shared__ __align__(16) s16 s_stage[RQ_WARPS][RQ_STAGE];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = blockIdx.x * RQ_WARPS + warp;
+    if (r >= P.n) return;
+    const RdoqReq q = P.reqs[r];
+    const int cnt = rq_list(P, q, s_stage[warp], lane);
+    __syncwarp();                                      // the list and the cleared block
+    if (lane == 0) P.num_nz[r] = cnt > 0 ? rq_chain<VEC>(P, q, cnt) : cnt;
 }
 
 // rdoq_init_err_scale (src/quant.c:69-83) for 8-bit: 2^(15 - tr_shift) / q_value in 20-bit fixed
@@ -326,27 +353,35 @@ int launch_rdoq(const void *reqs, int n, const void *ests, int n_est, s16 *coefs
         for (int b = 0; b < 7; b++) { P.scan[a][b] = tab->scan[a][b]; P.scanpos[a][b] = tab->scanpos[a][b]; }
     static const RqErrScale kErr;
     memcpy(P.err_scale, kErr.v, sizeof(P.err_scale));
+    int sms = 0;
+    UC_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const bool brief = n < RQ_SHORT_PER_SM * sms, vec = ((uintptr_t)ests & 15) == 0;
     // one word per coefficient (the position lists, at the coefficients' offsets) and the grouping's
     // arrays
     const size_t b_list = ((size_t)n_coefs * sizeof(u32) + 255) & ~(size_t)255;
     char *ws = nullptr;
-    int rc = work_alloc((void **)&ws, b_list + bs_bytes((size_t)n), st);
+    int rc = work_alloc((void **)&ws, b_list + (brief ? 256 : bs_bytes((size_t)n)), st);
     if (rc) return rc;
     P.scratch = (u32 *)ws;
-    const BlockOrder O = bs_place(ws + b_list, (size_t)n);
     prof_begin(PROF_RDOQ, st);
-    cudaError_t e = cudaMemsetAsync(O.counts, 0, BS_CLEAR, st);
-    if (e == cudaSuccess) {
+    cudaError_t e = cudaSuccess;
+    if (brief) {
+        const unsigned ctas = (unsigned)((n + RQ_WARPS - 1) / RQ_WARPS);
+        if (vec) k_rdoq_short<true><<<ctas, 32 * RQ_WARPS, 0, st>>>(P);
+        else k_rdoq_short<false><<<ctas, 32 * RQ_WARPS, 0, st>>>(P);
+        e = cudaGetLastError();
+    } else if ((e = cudaMemsetAsync(bs_place(ws + b_list, (size_t)n).counts, 0, BS_CLEAR, st)) == cudaSuccess) {
+        const BlockOrder O = bs_place(ws + b_list, (size_t)n);
         k_rdoq_list<<<(unsigned)((n + RQ_WARPS - 1) / RQ_WARPS), 32 * RQ_WARPS, 0, st>>>(P, O);
         k_bs_scatter<<<(unsigned)((n + BS_BUCKETS - 1) / BS_BUCKETS), BS_BUCKETS, 0, st>>>(O.key, O.counts, n, O.perm);
-        if (((uintptr_t)ests & 15) == 0) k_rdoq_chain<true><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(P, O.perm);
+        if (vec) k_rdoq_chain<true><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(P, O.perm);
         else k_rdoq_chain<false><<<(unsigned)((n + 31) / 32), 32, 0, st>>>(P, O.perm);
         e = cudaGetLastError();
     }
     rc = work_free(ws, st);
     UC_CHECK(e);
     if (rc) return rc;
-    count_launch(3);
+    count_launch(brief ? 1 : 3);
     prof_end(PROF_RDOQ, st);
     return UC_OK;
 }
