@@ -273,11 +273,12 @@ __global__ void __launch_bounds__(32, 32) k_me_tz(const TzParams P)
     o.mv[0] = q.mv[0]; o.mv[1] = q.mv[1];
     o.mv_ipel[0] = q.mv_ipel[0]; o.mv_ipel[1] = q.mv_ipel[1];
     const int x = q.x, y = q.y, w = q.w, h = q.h, mvr = q.mvr, bi = q.bi;
-    // the predictor as 32-bit values the compiler cannot narrow again: with q.mvp[1] >> mvr left to it,
-    // the shift of the record's upper halfword came out as 0 in some builds of this kernel (depending on
-    // the code around it) and the MV bits were counted from a predictor of 0
-    int mvpx = q.mvp[0], mvpy = q.mvp[1];
-    asm volatile("" : "+r"(mvpx), "+r"(mvpy));
+    // The predictor by two 16-bit loads of its own.  As q.mvp[1], the upper halfword of a loaded word, it was 0
+    // in every use of one version of this kernel, while a second read of the record gave the right value:
+    // with ptxas 13.0 at -O2 and -O3, not at -O1 and -O0, whatever nvcc's own level; a register made opaque
+    // where the value is used was 0 too.
+    const volatile s16 *mvp = P.reqs[r].mvp;
+    const int mvpx = mvp[0], mvpy = mvp[1];
     // calls outside the supported domain (block inside the picture, sides 4..64 powers of two,
     // known slots, resolution 0..4) come back with cost UINT64_MAX and their MVs unchanged
     const bool pow2 = (w & (w - 1)) == 0 && (h & (h - 1)) == 0;
