@@ -1,5 +1,6 @@
-"""QP counts and mode lists of the intra lattice against the oracle: the QPs of a tile run in pairs, a
-job that a QP codes nothing of keeps the prediction's SSD, and a tile holds a bounded number of jobs."""
+"""QP counts and mode lists of the intra lattice against the oracle: the QPs of a tile run one after the
+other, a job that a QP codes nothing of keeps the prediction's SSD, and a tile holds a bounded number of
+jobs."""
 import numpy as np
 import pytest
 

@@ -76,7 +76,7 @@ __device__ __forceinline__ int ame_bits(const s32 *mv, const s32 *mvp, int num_r
 // to 1/16 and clipped to 18 bits, and is filtered from the integer plane (com_mc_blk_luma, hp).
 // A lane takes two columns of a band of 4 rows, or 8 where the sub-blocks are 8x8 and that leaves every
 // lane a task, four rows of both at a time (aff_luma_pair).  One copy of the filter for both sizes: with
-// unrolled variants the step kernel waited for instructions a third of its time.
+// unrolled variants the kernel waited for instructions a third of its time.
 __device__ __noinline__ void ame_pred(const AffMeParams &P, const pel *plane, int x, int y, int w, int h, int lw,
                                       const s32 *mv, int sub, pel *dst, int lane)
 {

@@ -134,14 +134,10 @@ __device__ __forceinline__ int ang_sample(const pel *s, int mode, int w, int h, 
     return f4tap(s[idx], s[idx - 1], s[idx - 2], s[idx - 3], off);
 }
 
-// final prediction sample of com_intra_pred(ipm, ipf) at (i, j); with CW, CH > 0 the block is
-// known at compile time to be CW x CH at 8 bits (B's size fields are then not read)
-template <int CW = 0, int CH = 0>
+// final prediction sample of com_intra_pred(ipm, ipf) at (i, j)
 __device__ __forceinline__ int ipred_sample(const pel *s, const IpredBlock &B, int ipm, int ipf, int i, int j)
 {
-    constexpr bool K = CW > 0 && CH > 0;
-    const int w = K ? CW : B.w, h = K ? CH : B.h, mx = K ? 255 : (1 << B.bd) - 1;
-    const int blw = K ? ilog2d(CW) : B.lw, blh = K ? ilog2d(CH) : B.lh;
+    const int w = B.w, h = B.h, mx = (1 << B.bd) - 1, blw = B.lw, blh = B.lh;
     int v;
     bool s16path = false;
     if (ipm == 1) {                                         // plane

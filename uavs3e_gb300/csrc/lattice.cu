@@ -24,19 +24,11 @@
 // column pass and both inverse passes are dp2a products of s16 pairs with s8 matrix rows.
 //
 // The stages are bound by instruction issue and by the waits at their barriers, not by memory (a 1080p
-// frame at four QPs moves 1.06 GB, 0.16 ms of its time).  Prediction by table, four samples a task, the
-// inverse stages over the coded jobs only, QPs in pairs and the Hadamard rows packed two to a register
-// took a 1080p frame at four QPs from 28.7 to 27.5 ms, 416x240 at one QP with the IPF from 0.83 to 0.81,
-// and SATD of all modes + records of 5 at four QPs on 1272x716 from 6.57 to 5.81.  A SATD-only tile holds
-// predictions alone, so a CU's samples are fetched for several times as many modes, and a tile begins
-// with two dependent global loads (its CU's position, then the samples) instead of six: 27.3, 0.79 and
-// 3.75 ms.  Products over chunks of eight entries in rolled loops (a third of the code, and the inverse
-// passes stop at the last chunk that holds a level), rows stored whole and saturating packs: 24.9, 0.71
-// and 3.58 ms.  Four columns a task in the inverse row pass
-// and levels formed two to a word: 24.0, 0.71, 3.54.  One QP at a time again, with the job's buffers sharing
-// bytes, so that a tile holds half as many jobs more: 22.4, 0.59, 3.49.  The constants of a QP formed on the host
-// (a division and four table reads per QP, thread and tile) and 16 coefficients
-// a quantisation task: 21.4, 0.57, 3.46.
+// frame at four QPs moves 1.06 GB, 0.16 ms of its time).  The cost of a CU falls with every further job a
+// tile holds, as its samples, neighbours and barriers are shared, so a job's buffers share bytes; the code of
+// the 25 classes is fetched as the queue moves on, so loops over chunks stay rolled.  A 1080p frame at four
+// QPs takes 20.7 ms, 416x240 at one QP with the IPF 0.56, SATD of all modes + records of 5 at four QPs on
+// 1272x716 3.34 (28.7, 0.83 and 6.57 with a branch per mode and unrolled products).
 #include "lattice_kernel.cuh"
 
 #include <mutex>

@@ -63,10 +63,10 @@ constexpr int LAT_NO_MODE = 33;         // a list entry that is no mode (above 3
 
 // shared-memory layout of one shape's CTAs (host and device compute it the same way)
 struct LatLayout {
-    int w, h, lw, lh, kw, kh, lkw, lkh;
+    int w, h, lw, lh, kw, kh, lkw;
     int ps;            // prediction / org row stride (bytes): 16-byte aligned rows
     int ts;            // forward row-pass output row stride (s16): 16-byte aligned rows
-    int cs;            // coefficient row stride (s16): kw + 2
+    int cs;            // coefficient row stride (s16): 16-byte aligned rows
     int ds;            // transposed dequantised row stride (s16): 16-byte aligned rows
     int t2s;           // inverse column-pass output row stride (s16): 16-byte aligned rows
     int fw_ws, fh_ws, fht_ws, fwt_ws;   // table row strides in words
@@ -92,7 +92,7 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
 {
     L.lw = lw; L.lh = lh; L.w = 1 << lw; L.h = 1 << lh;
     L.kw = L.w < 32 ? L.w : 32; L.kh = L.h < 32 ? L.h : 32;
-    L.lkw = lw < 5 ? lw : 5; L.lkh = lh < 5 ? lh : 5;
+    L.lkw = lw < 5 ? lw : 5;
     // rows that are read whole by every lane of a warp (broadcast) start on 16 bytes; the
     // strides also keep the rows 8 lanes read at once on distinct banks
     L.ps = L.w <= 8 ? 16 : L.w <= 32 ? 48 : 80;
@@ -124,7 +124,7 @@ __host__ __device__ inline void lat_layout(int lw, int lh, int nm, int n_qp, int
     const int b_t = lat_up16(L.kw * L.ts * 2), b_t2 = lat_up16(L.h * L.t2s * 2);
     // T is dead once C is formed, and C once the levels of the last QP are: T2 takes T's place, and with one
     // QP DQT^T takes T's and T2 C's.  (Two QPs at a time, sharing the reads of C, took 24 % more bytes a
-    // job: 23.9 ms where one at a time takes 23.15, of a 1080p frame at four QPs.)
+    // job and was slower.)
     const int b_c = lat_up16(L.kh * L.cs * 2), b_dqt = lat_up16(L.kw * L.ds * 2);
     if (n_qp > 1) {
         L.j_t = L.j_t2 = j; j += b_t2 > b_t ? b_t2 : b_t;
@@ -601,7 +601,7 @@ __device__ __forceinline__ void lat_tile(const LatParams &P, const LatPerm *perm
     const int J = Gv * MCv;
     if (Gv <= 0 || MCv <= 0) return;
     // j / MCv as a multiply: with m = ceil(2^16 / MCv), (j m) >> 16 = j / MCv for every
-    // j * MCv < 2^16 (here j < 8 * 33 and MCv <= 33)
+    // j * MCv < 2^16 (here j < LAT_MAX_JOBS and MCv <= 33)
     const u32 mc_magic = (65536u + (u32)MCv - 1u) / (u32)MCv;
 
     const u32 *fw = (const u32 *)(sm + L.o_fw), *fh = (const u32 *)(sm + L.o_fh);
