@@ -267,3 +267,34 @@ def test_coef_rate_list_lengths(gpu, oracle, extra):
     for f in ("range", "run", "run_rdoq", "level", "last1", "last2"):
         want[f][bad] = reqs[f][bad]
     assert gpu.coef_rate(levels, reqs).tobytes() == want.tobytes()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("call", ("rdoq", "rate"))
+def test_large_workspace_is_kept_between_calls(gpu, oracle, call):
+    # a workspace of 384 MB (a word per coefficient, of which only a few blocks are named) stays with the
+    # library when the device is waited for: given back, it would be mapped anew by every call of a frame loop
+    import torch
+    n = 96 << 20
+    data = torch.zeros(n, dtype=torch.int16, device="cuda")
+    if call == "rdoq":
+        reqs, ests, coefs = cases.rdoq_inputs(oracle, dict(n=9, k=2), 77)
+        d = [torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).copy()).cuda() for a in (reqs, ests)]
+        out = torch.zeros(len(reqs), dtype=torch.int32, device="cuda")
+    else:
+        coefs, reqs = cases.coef_rate_inputs(np.random.default_rng(77), 9)
+        d = [torch.from_numpy(np.ascontiguousarray(reqs).view(np.uint8).copy()).cuda()]
+        out = torch.zeros(len(reqs) * gpu.COEF_RATE_OUT.itemsize, dtype=torch.uint8, device="cuda")
+    data[:coefs.size] = torch.from_numpy(coefs).cuda()
+    torch.cuda.synchronize()
+    if call == "rdoq":
+        gpu.rdoq_device(d[0].data_ptr(), len(reqs), d[1].data_ptr(), len(ests), data.data_ptr(), n, out.data_ptr())
+    else:
+        gpu.coef_rate_device(d[0].data_ptr(), len(reqs), data.data_ptr(), n, out.data_ptr())
+    held = torch.cuda.mem_get_info()[0]
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] - held < 32 << 20
+    if call == "rdoq":
+        assert np.array_equal(out.cpu().numpy(), oracle.rdoq(reqs, ests, coefs.copy()))
+    else:
+        assert out.cpu().numpy().tobytes() == oracle.coef_rate(coefs, reqs).tobytes()

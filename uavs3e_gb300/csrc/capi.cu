@@ -47,8 +47,11 @@ int ensure_init()
 
 // Workspaces of calls.  One memory pool per device: the device's default pool gives its memory back at
 // every synchronisation, so a call after one maps it anew (0.28 ms for 155 MB); this one keeps up to
-// WORK_POOL_KEEP bytes.  Allocations and frees follow the stream's order, so calls on several streams or
-// threads never share a block that is in use.
+// 1 / WORK_POOL_SHARE of the device's memory (9.3 GB of 298: the workspace of 2.3 G coefficients), and no more
+// than calls have used at a time.  Where 256 MB were kept, RDOQ of 100,000 / 200,000 32x32 blocks took 555 / 1,480
+// us, most of it for the mapping; now 123 / 206, and 395 / 705 with a buffer of its own per device before there was
+// a pool.  Allocations and frees follow the stream's order, so calls on several streams or threads never share a
+// block that is in use.
 //
 // A captured call's workspace is not a memory node: a graph with memory nodes can neither be a child of
 // another nor be instantiated twice.  It is a block of the same pool, allocated on the device's own stream
@@ -100,9 +103,11 @@ int work_open(int dev, cudaMemPool_t *pool, cudaStream_t *own)
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         if (!W.own[dev]) UC_CHECK(cudaStreamCreateWithFlags(&W.own[dev], cudaStreamNonBlocking));
+        size_t avail = 0, total = 0;
+        UC_CHECK(cudaMemGetInfo(&avail, &total));
+        uint64_t keep = total / WORK_POOL_SHARE;
         cudaMemPool_t p;
         UC_CHECK(cudaMemPoolCreate(&p, &props));
-        uint64_t keep = WORK_POOL_KEEP;
         UC_CHECK(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
         W.pool[dev] = p;
     }

@@ -36,10 +36,10 @@ struct MeResult {
 // optional per-kernel timing with CUDA events on the launching stream
 enum ProfKernel { PROF_PAD = 0, PROF_SUBPEL = 1, PROF_ME_INT = 2, PROF_ME_SUB = 3, PROF_LATTICE = 4, PROF_LOKA = 5, PROF_TZ = 6, PROF_MC = 7, PROF_RDOQ = 8, PROF_AFFME = 9, PROF_SHIFT = 10, PROF_N = 12 };
 int ensure_init();   // selects the library's device (initialising device 0 on first use)
-// stream-ordered workspace of one call from the library's pool on the current device (it keeps at
-// most WORK_POOL_KEEP bytes between calls).  Both may run while the stream is being captured: the
+// stream-ordered workspace of one call from the library's pool on the current device (it keeps at most
+// 1 / WORK_POOL_SHARE of the device's memory between calls).  Both may run while the stream is being captured: the
 // workspace then belongs to the graph and no node of it allocates or frees
-constexpr size_t WORK_POOL_KEEP = (size_t)256 << 20;
+constexpr size_t WORK_POOL_SHARE = 32;
 int work_alloc(void **p, size_t bytes, cudaStream_t st);
 int work_free(void *p, cudaStream_t st);
 int me_frame_once(); // one-time per-device setup of the frame search (me.cu)
