@@ -1,4 +1,4 @@
-"""CU motion compensation of lists around the length from which a warp takes four CUs, mixed and sorted by
+"""CU motion compensation of lists around the length from which small CUs are grouped, mixed and sorted by
 size, at aligned and unaligned output offsets, against the oracle."""
 import numpy as np
 import pytest
@@ -18,6 +18,21 @@ def test_mc_list_lengths(gpu, oracle, n, sort, shift):
     nbytes += shift
     if sort:
         reqs = reqs[np.argsort(reqs["w"].astype(int) * reqs["h"], kind="stable")]
+    want = oracle.mc_cu(p["w"], p["h"], luma[1], luma[2], chroma[1], chroma[2], reqs, nbytes)
+    assert np.array_equal(want, _gpu_mc(gpu, p, luma, chroma, reqs, nbytes))
+
+
+@pytest.mark.parametrize("channel", [0, 1])
+@pytest.mark.parametrize("shift", [1, 2, 3])
+def test_mc_unaligned_luma(gpu, oracle, shift, channel):
+    # every size with its luma off the 4-byte grid, one and two lists
+    p = cases.MC_CASES[0]
+    luma, chroma, reqs, _ = cases.mc_inputs(oracle, dict(p, n=400), 80 + shift)
+    reqs["channel"] = channel
+    size = reqs["w"].astype(int) * reqs["h"] * (2 if channel else 3) // 2
+    reqs["out_offset"] = np.cumsum(size) - size + shift
+    nbytes = int(size.sum()) + shift
+    assert len({(r["w"], r["h"]) for r in reqs}) >= 10 and (reqs["slot"] >= 0).all(1).any()
     want = oracle.mc_cu(p["w"], p["h"], luma[1], luma[2], chroma[1], chroma[2], reqs, nbytes)
     assert np.array_equal(want, _gpu_mc(gpu, p, luma, chroma, reqs, nbytes))
 

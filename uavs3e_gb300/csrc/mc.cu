@@ -73,7 +73,13 @@ __device__ __forceinline__ u32 mc_chroma4(const pel *s, int ic, const s8 (*filte
     return pack_sat_u8(v[0] >> 12, v[1] >> 12, v[2] >> 12, v[3] >> 12);
 }
 
-// eight bytes from any address
+// four and eight bytes from any address
+__device__ __forceinline__ u32 mc_load4(const pel *s)
+{
+    const uintptr_t a = (uintptr_t)s;
+    const u32 *wp = (const u32 *)(a & ~(uintptr_t)3);
+    return __funnelshift_r(__ldg(wp), __ldg(wp + 1), (u32)(a & 3) * 8);
+}
 __device__ __forceinline__ uint2 mc_load8(const pel *s)
 {
     const uintptr_t a = (uintptr_t)s;
@@ -112,28 +118,49 @@ __device__ __forceinline__ void mc_cu(const McParams &P, const McReq &q, int lan
             src[l] = P.planes[q.slot[l] * 16 + (qy & 3) * 4 + (qx & 3)] + (long long)py * P.i_ref + px;
         }
         const pel *s0 = src[0] ? src[0] : src[1], *s1 = src[0] ? src[1] : nullptr;
-        // byte-wise rounded average of the two lists (pel_avrg), word stores where the output is
-        // 4-byte aligned
-        const int lq = 31 - __clz(w >> 3);           // log2 of the 8-sample pieces per row
-        const bool aligned = ((uintptr_t)o & 3) == 0;
-        const int n8 = (w * h) >> 3;
+        // byte-wise rounded average of the two lists (pel_avrg), word stores where the output is 4-byte
+        // aligned; elsewhere a lane forms four samples, so that the byte stores of a warp lie on half as many
+        // lines (8,000 64x64 CUs, luma alone: 49 us with eight, 42 with four)
+        if (((uintptr_t)o & 3) == 0) {
+            const int lq = 31 - __clz(w >> 3);       // log2 of the 8-sample pieces per row
+            const int n8 = (w * h) >> 3;
 #pragma unroll 1
-        for (int i0 = lane; i0 < n8; i0 += U * lanes) {
-            uint2 v[U], b[U];
+            for (int i0 = lane; i0 < n8; i0 += U * lanes) {
+                uint2 v[U], b[U];
 #pragma unroll
-            for (int k = 0; k < U; k++) {
-                const int i = i0 + k * lanes, j = i >> lq, c = (i - (j << lq)) << 3;
-                if (i >= n8) break;
-                v[k] = mc_load8(s0 + j * P.i_ref + c);
-                if (s1) b[k] = mc_load8(s1 + j * P.i_ref + c);
+                for (int k = 0; k < U; k++) {
+                    const int i = i0 + k * lanes, j = i >> lq, c = (i - (j << lq)) << 3;
+                    if (i >= n8) break;
+                    v[k] = mc_load8(s0 + j * P.i_ref + c);
+                    if (s1) b[k] = mc_load8(s1 + j * P.i_ref + c);
+                }
+#pragma unroll
+                for (int k = 0; k < U; k++) {
+                    const int i = i0 + k * lanes;
+                    if (i >= n8) break;
+                    if (s1) v[k] = make_uint2(__vavgu4(v[k].x, b[k].x), __vavgu4(v[k].y, b[k].y));
+                    mc_store4(o + (i << 3), v[k].x, true);
+                    mc_store4(o + (i << 3) + 4, v[k].y, true);
+                }
             }
+        } else {
+            const int lq = 31 - __clz(w >> 2), n4 = (w * h) >> 2;
+#pragma unroll 1
+            for (int i0 = lane; i0 < n4; i0 += U * lanes) {
+                u32 v[U], b[U];
 #pragma unroll
-            for (int k = 0; k < U; k++) {
-                const int i = i0 + k * lanes;
-                if (i >= n8) break;
-                if (s1) v[k] = make_uint2(__vavgu4(v[k].x, b[k].x), __vavgu4(v[k].y, b[k].y));
-                mc_store4(o + (i << 3), v[k].x, aligned);
-                mc_store4(o + (i << 3) + 4, v[k].y, aligned);
+                for (int k = 0; k < U; k++) {
+                    const int i = i0 + k * lanes, j = i >> lq, c = (i - (j << lq)) << 2;
+                    if (i >= n4) break;
+                    v[k] = mc_load4(s0 + j * P.i_ref + c);
+                    if (s1) b[k] = mc_load4(s1 + j * P.i_ref + c);
+                }
+#pragma unroll
+                for (int k = 0; k < U; k++) {
+                    const int i = i0 + k * lanes;
+                    if (i >= n4) break;
+                    mc_store4(o + (i << 2), s1 ? __vavgu4(v[k], b[k]) : v[k], false);
+                }
             }
         }
         o += w * h;
