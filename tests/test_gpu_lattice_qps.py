@@ -205,3 +205,29 @@ def test_lattice_four_qps_of_few_jobs(gpu, oracle, n_modes, W, H):
     got, want = d_q.cpu().numpy().view(gpu.LAT_Q).reshape(n * 33, 4)[at], q_o.reshape(n * 33, 4)[at]
     for f in FIELDS:
         assert np.array_equal(got[f], want[f]), f
+
+
+@pytest.mark.parametrize("n_qp,jobs_per_cta,extra", [(4, 2, -1), (4, 2, 1), (1, 2, -1), (0, 6, -1), (0, 6, 1)])
+def test_lattice_of_few_cus(gpu, oracle, n_qp, jobs_per_cta, extra):
+    # CUs of any shape in lists on both sides of the lengths where the tile layouts change (four CTAs an SM)
+    import torch
+    W, H, qps = 192, 128, np.array([27, 45, 33, 38][:n_qp], np.int32)
+    n = jobs_per_cta * 4 * torch.cuda.get_device_properties(0).multi_processor_count // 33 + extra
+    org, rec = _frames(W, H, 50 + n_qp, 6)
+    cus = gpu.lattice_cus(W, H)
+    big = cus[(cus["w"].astype(int) * cus["h"] >= 1024)]
+    rng = np.random.default_rng(n)
+    cus = np.concatenate([big[rng.permutation(len(big))[:n // 3]], cus[rng.permutation(len(cus))[:n - n // 3]]])
+    satd_o, q_o = oracle_lattice(oracle, org, rec, cus, 1, list(qps) if n_qp else [32])
+    d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (org, rec, cus.view(np.uint8))]
+    d_satd = torch.zeros(n * 33, dtype=torch.int32, device="cuda")
+    d_q = torch.zeros(max(1, n * 33 * n_qp * gpu.LAT_Q.itemsize), dtype=torch.uint8, device="cuda")
+    gpu.check(gpu.lib().uavs3e_cuda_intra_lattice_device(
+        d[0].data_ptr(), W, d[1].data_ptr(), W, W, H, d[2].data_ptr(), n, 1, qps.ctypes.data if n_qp else None, n_qp, 1,
+        d_satd.data_ptr(), d_q.data_ptr() if n_qp else None, torch.cuda.current_stream().cuda_stream), "intra_lattice")
+    torch.cuda.synchronize()
+    assert np.array_equal(d_satd.cpu().numpy().view(np.uint32), satd_o.ravel())
+    if n_qp:
+        got = d_q.cpu().numpy().view(gpu.LAT_Q).ravel()
+        for f in FIELDS:
+            assert np.array_equal(got[f], q_o.ravel()[f]), f

@@ -211,11 +211,24 @@ struct LatTune {
 static LatTune g_tune[64];
 static bool g_tune_on = true;
 
-// SATD-only calls are not tuned.  A large one takes the default budget; one of fewer than
-// LAT_SATD_SMALL_JOBS (CU, mode) jobs per resident CTA takes LAT_SATD_SMALL, whose shorter tiles keep all
-// CTAs busy to the end: 33 modes of 64x64 41 us (67 with the default), of 256x128 (403 jobs a CTA) 96 (99),
-// of 256x192 (605) 127 (123); 5 modes of 192x128 44 (67), of 512x384 (367) 106 (107).
+// Calls with few (CU, mode) jobs per resident CTA take smaller tiles than the tuned or default ones, so that all
+// CTAs are busy to the end: lat_small gives their budget, 0 for a call large enough (SATD-only calls are not tuned
+// and take the default then).  On 608 CTAs, us with the tiles below and above each line:
+//   SATD only, 12 / 20 KB: 33 modes of 8 32x64 CUs (0.4 jobs a CTA) 38 / 47, of 100 32x4 (5) 38 / 44; the lattice
+//     of 64x64 with 5 modes (8) 47 / 50; 33 modes of 300 32x32 (16) 63 / 66, of 300 16x64 (16) 80 / 65
+//   SATD only, 20 / 50 KB: 33 modes of 64x64 41 / 67, of 256x128 (403) 96 / 99, of 256x192 (605) 127 / 123; 5 modes
+//     of 192x128 44 / 67, of 512x384 (367) 106 / 107
+//   four QPs, 24 / 50 KB: 33 modes of one 64x32 52 / 76, one mode of 100 32x16 (0.2) 47 / 63, 33 modes of 30 32x64
+//     (1.6) 79 / 69, of 16x16 (2.7) 49 / 57, 5 modes of 300 16x64 (2.5) 72 / 60
+constexpr int LAT_SATD_TINY = 12 * 1024, LAT_SATD_TINY_JOBS = 6;
 constexpr int LAT_SATD_SMALL = 20 * 1024, LAT_SATD_SMALL_JOBS = 410;
+constexpr int LAT_QP_SMALL = 24 * 1024, LAT_QP_SMALL_JOBS = 2;
+
+static int lat_small(long long jobs, long long ctas, int n_qp)
+{
+    if (n_qp > 0) return jobs < LAT_QP_SMALL_JOBS * ctas ? LAT_QP_SMALL : 0;
+    return jobs < LAT_SATD_TINY_JOBS * ctas ? LAT_SATD_TINY : jobs < LAT_SATD_SMALL_JOBS * ctas ? LAT_SATD_SMALL : 0;
+}
 
 // per device: the CU permutation and the queue's counters
 struct LatScratch {
@@ -352,9 +365,8 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
         std::lock_guard<std::mutex> lk(T.mu);
         const int kind = n_qp > 1;
         int *tuned = T.budget[n_modes][kind];
-        const bool small = n_qp == 0 && (long long)n_cus * n_modes < (long long)LAT_SATD_SMALL_JOBS * S.sms * S.occ;
-        for (int c = 0; c < LAT_SHAPES; c++)
-            budgets[c] = small ? LAT_SATD_SMALL : n_qp > 0 && tuned[c] ? tuned[c] : LAT_BUDGET;
+        const int small = lat_small((long long)n_cus * n_modes, (long long)S.sms * S.occ, n_qp);
+        for (int c = 0; c < LAT_SHAPES; c++) budgets[c] = small ? small : n_qp > 0 && tuned[c] ? tuned[c] : LAT_BUDGET;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0) UC_CHECK(cudaStreamIsCapturing(st, &cap));
         if (g_tune_on && !T.done[n_modes][kind] && n_qp > 0 && cap == cudaStreamCaptureStatusNone) {
@@ -367,7 +379,8 @@ int launch_intra_lattice(const pel *org, int i_org, const pel *rec, int i_rec, i
                 int best = LAT_BUDGET;
                 int r = lat_tune_class(c, P, cus, n_cus, W, H, budgets, S, st, &launches, &best);
                 if (r) return r;
-                tuned[c] = budgets[c] = best;
+                tuned[c] = best;
+                if (!small) budgets[c] = best;
             }
         }
     }
