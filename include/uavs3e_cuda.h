@@ -548,7 +548,8 @@ typedef struct {
  * and keeps the fastest (that call waits for the GPU; a captured call does not tune and takes the
  * default where nothing is tuned); records are the same for every layout.  budgets: per shape
  * (log2 w - 2) * 5 + (log2 h - 2), in bytes, 0 = the default 50 KB (not tuned); those of calls with
- * several QPs once such a call has tuned, else those of calls with one. */
+ * several QPs once such a call has tuned, else those of calls with one.  Calls of few CUs take
+ * smaller tiles than these. */
 UAVS3E_CUDA_API void uavs3e_cuda_lattice_autotune(int on);
 UAVS3E_CUDA_API int uavs3e_cuda_lattice_budgets(int n_modes, int out[25]);
 
